@@ -1481,35 +1481,6 @@ __global__ void __launch_bounds__(32 * WTile<M>::WPC)
     }
 }
 
-// ---------------------------------------------- direct DST (any n, dense sine matrix) ----
-// out_k = sqrt(2/(n+1)) sum_m in_m sin(pi (k+1)(m+1)/(n+1)); `mat` holds the n*n sines.
-constexpr int kDenseThreads = 128;
-template <bool STRIDED>
-__global__ void __launch_bounds__(kDenseThreads)
-    k_dst1_dense(const double2 *__restrict__ in, double2 *__restrict__ out, int n, long nlines, long in_ld,
-                 long out_ld, long plane_stride, const double *__restrict__ mat) {
-    extern __shared__ __align__(128) unsigned char smem_dense[];
-    double2   *x = reinterpret_cast<double2 *>(smem_dense);
-    const long line = blockIdx.x;
-    const long pbase = STRIDED ? (long)blockIdx.y * plane_stride : 0;
-    for (int m = threadIdx.x; m < n; m += blockDim.x)
-        x[m] = STRIDED ? in[pbase + line + (long)m * in_ld] : in[line * in_ld + m];
-    __syncthreads();
-    const double coef = sqrt(2.0 / (n + 1));
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const double *row = mat + (long)k * n;
-        double        sr = 0.0, si = 0.0;
-        for (int m = 0; m < n; m++) {
-            const double s = __ldg(row + m);
-            sr = fma(s, x[m].x, sr);
-            si = fma(s, x[m].y, si);
-        }
-        const double2 r = make_double2(coef * sr, coef * si);
-        if (STRIDED) out[pbase + line + (long)k * out_ld] = r;
-        else out[line * out_ld + k] = r;
-    }
-}
-
 // ------------------------------------------------------------------ tables --------
 __global__ void k_make_tables(int m, double2 *tw, double *sn) {
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < m; t += gridDim.x * blockDim.x) {
@@ -1517,16 +1488,6 @@ __global__ void k_make_tables(int m, double2 *tw, double *sn) {
         sincospi(2.0 * (double)t / (double)m, &s, &c); // exp(-2 pi i t/m) = c - i s
         tw[t] = make_double2(c, -s);
         sn[t] = sinpi((double)t / (double)m);
-    }
-}
-
-__global__ void k_make_dense(int n, double *mat) {
-    const long tot = (long)n * n;
-    for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < tot; q += (long)gridDim.x * blockDim.x) {
-        const long k = q / n, m = q % n;
-        // (k+1)(m+1) reduced mod 2(n+1) keeps the argument of sinpi in [0, 2)
-        const long   num = ((k + 1) * (m + 1)) % (2L * (n + 1));
-        mat[q] = sinpi((double)num / (double)(n + 1));
     }
 }
 
@@ -1562,22 +1523,6 @@ int prepare_dst(Ctx *c, int n) {
         return dense_for(c, n, &mat);
     }
     return HH_OK; // lengths the transforms refuse fail at solve time
-}
-
-int dense_for(Ctx *c, int n, const double **mat) {
-    std::lock_guard<std::mutex> g(c->mu);
-    auto it = c->dense.find(n);
-    if (it == c->dense.end()) {
-        double *d = nullptr;
-        HH_CUDA(cudaMalloc(&d, sizeof(double) * (size_t)n * (size_t)n));
-        k_make_dense<<<256, 256, 0, c->stream>>>(n, d);
-        HH_CUDA(cudaGetLastError());
-        c->launches++;
-        c->dense[n] = d;
-        it = c->dense.find(n);
-    }
-    *mat = it->second;
-    return HH_OK;
 }
 
 // -------------------------------------------------------------------- launch ------
@@ -1715,17 +1660,7 @@ template <bool IS, bool OS, bool LP = false, bool UPD = false> static int launch
         set_error("DST length %d: transposing modes need n+1 a power of two", n);
         return HH_ERR_UNSUPPORTED;
     }
-    const double *mat;
-    HH_TRY(dense_for(c, n, &mat));
-    const size_t shm = sizeof(double2) * (size_t)n;
-    if (shm > 48 * 1024)
-        HH_CUDA(cudaFuncSetAttribute(k_dst1_dense<IS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-    dim3 grid((unsigned)a.nlines, (unsigned)a.planes);
-    k_dst1_dense<IS><<<grid, kDenseThreads, shm, c->stream>>>(a.in, a.out, n, a.nlines, a.in_ld, a.out_ld,
-                                                              a.in_plane, mat);
-    HH_CUDA(cudaGetLastError());
-    c->launches++;
-    return HH_OK;
+    return launch_dst_dense(c, n, IS, a.nlines, a.planes, a.in, a.in_ld, a.in_plane, a.out, a.out_ld, a.out_plane);
 }
 
 bool rows_update_supported(int n, int rows_kernel) {

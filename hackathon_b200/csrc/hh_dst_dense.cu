@@ -1,0 +1,321 @@
+// DST-I of any length as two half-size FP64 tensor-core products (sm_100a).
+//
+// Serves the lengths whose n + 1 is not a power of two in 64 .. 8192, which the FFT kernels of
+// hh_dst.cu cannot take (the reference's own sizes among them: N = 100, 125, 500), in place of the
+// reference's length-(2n+2) real FFTs (2D_Program/solver_functions/DST.c:6-44,
+// 3D_Program/solver_functions/DST.c:148-204).
+//
+// With M = n + 1 the sine matrix splits by the mirror symmetry sin(pi (M-j) k / M) =
+// -(-1)^k sin(pi j k / M):
+//     S_k (k odd)  = sum_{j <= ceil(n/2)} sin(pi j k / M) a_j,   a_j = x_j + x_{M-j} (x_j alone at j = M/2)
+//     S_k (k even) = sum_{j <= floor(n/2)} sin(pi j k / M) d_j,  d_j = x_j - x_{M-j}
+// so a line of n complex values costs 2 n^2 real operations instead of 4 n^2, in sums half as long.
+//
+// A CTA takes NL lines, forms a and d of all of them in shared memory (so the transform may run in
+// place), and its warps walk units (8 odd and 8 even outputs) x (NTW tiles of 4 complex lines =
+// 8 real columns): mma.m8n8k4 in FP64 with the sine fragments as A and the lines as B.  The
+// sines come from a table laid out fragment by fragment, the odd and the even matrix side by side,
+// so that a lane reads both of its values with one 16-byte load, four steps ahead, and no shared
+// memory is spent on them: every CTA reads the table once (4 n^2 bytes, from L1/L2).  The C
+// fragment's two values are the real and imaginary part of one output, and the lane that holds output
+// 2i of a line also holds output 2i + 1, so stores go out as 32-byte pairs.
+//
+// Bound by the FP64 tensor rate from n ~ 200 on (37 TF measured; 4800 rows of n = 300 take 46 us, 23 us
+// of it at that rate), below that by the load and store phases.  Against one dot product per thread
+// with uncoalesced sines before: 8000 rows of n = 500 5083 -> 166 us, 40000 rows of n = 100 585 -> 52
+// us, columns 643 -> 48 us.
+#include "hh_internal.cuh"
+
+#include <algorithm>
+
+namespace hh {
+
+namespace {
+
+constexpr int kMmaThreads = 256, kMmaWarps = kMmaThreads / 32;
+constexpr int kMmaSmemMax = 227 * 1024;
+// the longest line that fits four to a CTA in both layouts (2 * 1200 * 6 * 16 bytes at n = 2400)
+constexpr int kMmaMaxN = 2400;
+
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+// geometry shared by host and device: h1 odd outputs (and values a_j), k4 steps of four j
+__host__ __device__ inline int half_up(int n) { return (n + 1) / 2; }
+__host__ __device__ inline int k4_steps(int n) { return (half_up(n) + 3) / 4; }
+__host__ __device__ inline int out_tiles(int n) { return (half_up(n) + 7) / 8; }
+// shared-memory pitches in complex values: a B fragment is 4 values of j by 8 real columns, read
+// by half warps of 4 x 4; rows (line-major): pitch = 4 mod 8 puts the two lines of a half warp on
+// different 64-byte halves of the banks; columns (j-major): pitch = 2 or 6 mod 8 puts its four j on
+// four different 32-byte quarters
+__host__ __device__ inline int rows_pitch(int n) { return 4 * k4_steps(n) + (k4_steps(n) % 2 ? 0 : 4); }
+__host__ __device__ inline int cols_pitch(int nl) { return nl + 2; } // nl is a multiple of 4
+
+inline size_t mma_smem(bool cols, int n, int nl) {
+    return 2 * sizeof(double2) * (cols ? (size_t)4 * k4_steps(n) * cols_pitch(nl) : (size_t)nl * rows_pitch(n));
+}
+
+// COLS: line c of a plane is column c (element j at c + j ld); otherwise row c (element j at c ld + j)
+template <bool COLS, int NTW>
+__global__ void __launch_bounds__(kMmaThreads, 3)
+    k_dst1_mma(const double2 *in, double2 *out, int n, long nlines, long in_ld, long out_ld, long in_plane,
+               long out_plane, int groups, const double2 *__restrict__ tab) {
+    extern __shared__ __align__(16) double2 mma_sm[];
+    const int  h1 = half_up(n), p = n / 2, ks = k4_steps(n), nl = 4 * NTW * groups;
+    const int  pitch = COLS ? cols_pitch(nl) : rows_pitch(n);
+    double2   *sa = mma_sm, *sd = mma_sm + (COLS ? 4 * ks : nl) * pitch;
+    const int  lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long l0 = (long)blockIdx.x * nl;
+    const int  live = (int)min((long)nl, nlines - l0);
+    const double2 zero = make_double2(0.0, 0.0);
+    in += (long)blockIdx.y * in_plane + (COLS ? l0 : l0 * in_ld);
+    out += (long)blockIdx.y * out_plane + (COLS ? l0 : l0 * out_ld);
+
+    // ---- a_j and d_j of every line; zeros past the halves and for lines past the end
+    auto put = [&](int at, int j, double2 x, double2 m) {
+        const bool mid = 2 * j + 1 == n;
+        sa[at] = mid ? x : cadd(x, m);
+        sd[at] = mid ? zero : csub(x, m);
+    };
+    if constexpr (COLS) {
+        for (int e0 = threadIdx.x; e0 < 4 * ks * nl; e0 += 4 * kMmaThreads) {
+            double2 x[4], m[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int j = (e0 + q * kMmaThreads) / nl, c = e0 + q * kMmaThreads - j * nl;
+                x[q] = m[q] = zero;
+                if (j < h1 && c < live) {
+                    x[q] = in[c + (long)j * in_ld];
+                    m[q] = in[c + (long)(n - 1 - j) * in_ld];
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int j = (e0 + q * kMmaThreads) / nl, c = e0 + q * kMmaThreads - j * nl;
+                if (j < 4 * ks) put(j * pitch + c, j, x[q], m[q]);
+            }
+        }
+    } else {
+        for (int c = warp; c < nl; c += kMmaWarps)
+            for (int j0 = lane; j0 < 4 * ks; j0 += 128) {
+                double2 x[4], m[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int j = j0 + 32 * q;
+                    x[q] = m[q] = zero;
+                    if (j < h1 && c < live) {
+                        x[q] = in[c * in_ld + j];
+                        m[q] = in[c * in_ld + (n - 1 - j)];
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    if (j0 + 32 * q < 4 * ks) put(c * pitch + j0 + 32 * q, j0 + 32 * q, x[q], m[q]);
+            }
+    }
+    __syncthreads();
+
+    const int    kk = lane & 3, nn = lane >> 2; // the lane's j within a step and real column within a tile
+    const int    units = out_tiles(n) * groups;
+    const double coef = sqrt(2.0 / (n + 1));
+    // strides in doubles: from one step of four j to the next, and from one tile of four lines to the next
+    const int kstep = COLS ? 8 * pitch : 8, nstep = COLS ? 8 : 8 * pitch;
+    const int b0 = 2 * (COLS ? kk * pitch + (nn >> 1) : (nn >> 1) * pitch + kk) + (nn & 1);
+    constexpr int PF = 2; // table steps in flight
+    for (int u = warp; u < units; u += kMmaWarps) {
+        const int      tile = u / groups, c0 = (u - tile * groups) * 4 * NTW;
+        const double2 *q = tab + ((long)tile * ks) * 32 + lane;
+        const double  *ba = reinterpret_cast<const double *>(sa) + b0 + (c0 / 4) * nstep;
+        const double  *bd = reinterpret_cast<const double *>(sd) + b0 + (c0 / 4) * nstep;
+        double ao[NTW][2], ae[NTW][2];
+#pragma unroll
+        for (int t = 0; t < NTW; t++) ao[t][0] = ao[t][1] = ae[t][0] = ae[t][1] = 0.0;
+        double2 cur[PF];
+#pragma unroll
+        for (int i = 0; i < PF; i++)
+            if (i < ks) cur[i] = __ldg(q + i * 32);
+        for (int k = 0; k < ks; k += PF) {
+            double2 nxt[PF];
+#pragma unroll
+            for (int i = 0; i < PF; i++)
+                if (k + PF + i < ks) nxt[i] = __ldg(q + (k + PF + i) * 32);
+#pragma unroll
+            for (int i = 0; i < PF; i++) {
+                if (k + i < ks) {
+#pragma unroll
+                    for (int t = 0; t < NTW; t++) {
+                        dmma(ao[t], cur[i].x, ba[(k + i) * kstep + t * nstep]);
+                        dmma(ae[t], cur[i].y, bd[(k + i) * kstep + t * nstep]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < PF; i++) cur[i] = nxt[i];
+        }
+        // output 2i (S_{2i+1}) and 2i + 1 (S_{2i+2}) of line c0 + 4 t + kk
+        const int i = 8 * tile + nn;
+#pragma unroll
+        for (int t = 0; t < NTW; t++) {
+            const int c = c0 + 4 * t + kk;
+            if (c < live) {
+                double2   *o = out + (COLS ? c + (long)(2 * i) * out_ld : c * out_ld + 2 * i);
+                const long step = COLS ? out_ld : 1;
+                if (i < h1) o[0] = make_double2(coef * ao[t][0], coef * ao[t][1]);
+                if (i < p) o[step] = make_double2(coef * ae[t][0], coef * ae[t][1]);
+            }
+        }
+    }
+}
+
+// the fragment table: (odd, even) sines of output row 8 tile + lane / 4 and value 4 k + lane % 4
+__global__ void k_make_mma(int n, double2 *tab) {
+    const int  h1 = half_up(n), p = n / 2, ks = k4_steps(n);
+    const long tot = (long)out_tiles(n) * ks * 32;
+    for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < tot; e += (long)gridDim.x * blockDim.x) {
+        const int  lane = (int)(e & 31);
+        const long s = e >> 5;
+        const long i = 8 * (s / ks) + (lane >> 2), j = 4 * (s % ks) + (lane & 3) + 1;
+        const long m2 = 2L * (n + 1); // arguments reduced mod 2 (n + 1) keep sinpi's in [0, 2)
+        double2    v = make_double2(0.0, 0.0);
+        if (i < h1 && j <= h1) v.x = sinpi((double)((2 * i + 1) * j % m2) / (double)(n + 1));
+        if (i < p && j <= p) v.y = sinpi((double)((2 * i + 2) * j % m2) / (double)(n + 1));
+        tab[e] = v;
+    }
+}
+
+// the full n x n sine matrix of the lengths past kMmaMaxN
+__global__ void k_make_dense(int n, double *mat) {
+    const long tot = (long)n * n;
+    for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < tot; q += (long)gridDim.x * blockDim.x) {
+        const long k = q / n, m = q % n;
+        // (k+1)(m+1) reduced mod 2(n+1) keeps the argument of sinpi in [0, 2)
+        const long num = ((k + 1) * (m + 1)) % (2L * (n + 1));
+        mat[q] = sinpi((double)num / (double)(n + 1));
+    }
+}
+
+// One line per CTA against the full matrix, for the lines too long for k_dst1_mma.  The matrix is
+// symmetric: thread k walks column k, so that a warp reads neighbouring values.
+constexpr int kDenseThreads = 128;
+template <bool STRIDED>
+__global__ void __launch_bounds__(kDenseThreads)
+    k_dst1_dense(const double2 *__restrict__ in, double2 *__restrict__ out, int n, long in_ld, long out_ld,
+                 long in_plane, long out_plane, const double *__restrict__ mat) {
+    extern __shared__ __align__(128) unsigned char smem_dense[];
+    double2   *x = reinterpret_cast<double2 *>(smem_dense);
+    const long line = blockIdx.x;
+    in += (long)blockIdx.y * in_plane;
+    out += (long)blockIdx.y * out_plane;
+    for (int m = threadIdx.x; m < n; m += blockDim.x) x[m] = STRIDED ? in[line + (long)m * in_ld] : in[line * in_ld + m];
+    __syncthreads();
+    const double coef = sqrt(2.0 / (n + 1));
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        double sr = 0.0, si = 0.0;
+        for (int m = 0; m < n; m++) {
+            const double s = __ldg(mat + (long)m * n + k);
+            sr = fma(s, x[m].x, sr);
+            si = fma(s, x[m].y, si);
+        }
+        const double2 r = make_double2(coef * sr, coef * si);
+        if (STRIDED) out[line + (long)k * out_ld] = r;
+        else out[line * out_ld + k] = r;
+    }
+}
+
+// Lines per CTA: 4 ntw lines per warp unit, `groups` units side by side.
+//  * groups: the least that gives all eight warps a unit (n < 64 has fewer than eight output tiles).
+//  * ntw: the widest of 4, 3, 2 whose lines leave room for three CTAs on an SM (n = 100: 52 us at 4
+//    against 54 at 3 and 56 at 2 for 40000 rows; n = 300: 46 us at 3 against 50 at 2; n = 500: 166 us
+//    at 2 against 196 at 1, two CTAs per SM with 3: 179), then 2 with two CTAs (n = 700: 228 us, 241 at
+//    1), then 1 (n = 1000: 655 us, 771 at 2).  Columns take the width (up to 5) that
+//    leaves the fewest idle columns in a plane's last tile (100 columns: 48 us at 5, 52 at 4).
+//  * fewer lines per CTA where the launch would leave SMs without one.
+void dense_shape(bool cols, int n, long nlines, long planes, int *ntw, int *groups) {
+    const int units = out_tiles(n);
+    int       g = units >= kMmaWarps ? 1 : std::min(4, kMmaWarps / units), w = 0;
+    auto per_sm = [&](int v) { return kMmaSmemMax / (long)(mma_smem(cols, n, 4 * v * g) + 1024); };
+    auto padded = [&](int v) { return (nlines + 4L * v * g - 1) / (4L * v * g) * (4L * v * g); };
+    for (int v = cols ? 5 : 4; v >= 2; v--)
+        if (per_sm(v) >= 3 && (w == 0 || (cols && padded(v) < padded(w)))) w = v;
+    if (w == 0) w = per_sm(2) >= 2 ? 2 : 1;
+    auto ctas = [&]() { return padded(w) / (4L * w * g) * planes; };
+    while (w > 1 && ctas() < 148) w--;
+    while (g > 1 && ctas() < 148) g--;
+    *ntw = w;
+    *groups = g;
+}
+
+template <bool COLS, int NTW>
+int launch_mma(Ctx *c, int n, long nlines, long planes, const double2 *in, long in_ld, long in_plane, double2 *out,
+               long out_ld, long out_plane, int groups, const double2 *tab) {
+    const int    nl = 4 * NTW * groups;
+    const size_t shm = mma_smem(COLS, n, nl);
+    HH_CUDA(cudaFuncSetAttribute(k_dst1_mma<COLS, NTW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+    dim3 grid((unsigned)((nlines + nl - 1) / nl), (unsigned)planes);
+    k_dst1_mma<COLS, NTW><<<grid, kMmaThreads, shm, c->stream>>>(in, out, n, nlines, in_ld, out_ld, in_plane, out_plane,
+                                                                 groups, tab);
+    HH_CUDA(cudaGetLastError());
+    c->launches++;
+    return HH_OK;
+}
+
+} // namespace
+
+int dense_for(Ctx *c, int n, const double **mat) {
+    std::lock_guard<std::mutex> g(c->mu);
+    auto it = c->dense.find(n);
+    if (it == c->dense.end()) {
+        double *d = nullptr;
+        if (n <= kMmaMaxN) {
+            HH_CUDA(cudaMalloc(&d, sizeof(double2) * 32 * (size_t)out_tiles(n) * k4_steps(n)));
+            k_make_mma<<<256, 256, 0, c->stream>>>(n, reinterpret_cast<double2 *>(d));
+        } else {
+            HH_CUDA(cudaMalloc(&d, sizeof(double) * (size_t)n * (size_t)n));
+            k_make_dense<<<256, 256, 0, c->stream>>>(n, d);
+        }
+        HH_CUDA(cudaGetLastError());
+        c->launches++;
+        c->dense[n] = d;
+        it = c->dense.find(n);
+    }
+    *mat = it->second;
+    return HH_OK;
+}
+
+int launch_dst_dense(Ctx *c, int n, bool cols, long nlines, long planes, const double2 *in, long in_ld, long in_plane,
+                     double2 *out, long out_ld, long out_plane) {
+    const double *mat;
+    HH_TRY(dense_for(c, n, &mat));
+    if (n > kMmaMaxN) {
+        const size_t shm = sizeof(double2) * (size_t)n;
+        auto         kern = cols ? k_dst1_dense<true> : k_dst1_dense<false>;
+        HH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+        dim3 grid((unsigned)nlines, (unsigned)planes);
+        kern<<<grid, kDenseThreads, shm, c->stream>>>(in, out, n, in_ld, out_ld, in_plane, out_plane, mat);
+        HH_CUDA(cudaGetLastError());
+        c->launches++;
+        return HH_OK;
+    }
+    const double2 *tab = reinterpret_cast<const double2 *>(mat);
+    int ntw = 1, groups = 1;
+    dense_shape(cols, n, nlines, planes, &ntw, &groups);
+#define HH_MMA(W)                                                                                                            \
+    case W:                                                                                                                  \
+        return cols ? launch_mma<true, W>(c, n, nlines, planes, in, in_ld, in_plane, out, out_ld, out_plane, groups, tab)    \
+                    : launch_mma<false, W>(c, n, nlines, planes, in, in_ld, in_plane, out, out_ld, out_plane, groups, tab);
+    switch (ntw) {
+        HH_MMA(1)
+        HH_MMA(2)
+        HH_MMA(3)
+        HH_MMA(4)
+        HH_MMA(5)
+    }
+#undef HH_MMA
+    set_error("DST length %d: no tile shape", n);
+    return HH_ERR_UNSUPPORTED;
+}
+
+} // namespace hh

@@ -68,7 +68,7 @@ struct Ctx {
     //   sn[M]  : sin(pi t / M),      t = 0..M-1                 (double)
     std::map<int, double2 *> tw;
     std::map<int, double *>  sn;
-    std::map<int, double *>  dense; // n*n sine matrices for the direct DST (n+1 not a power of two)
+    std::map<int, double *>  dense; // sine tables of the direct DST (n+1 not a power of two), hh_dst_dense.cu
     std::mutex               mu;
     std::vector<Plan *>      plans;
     long long                launches = 0;       // kernels launched through this context
@@ -102,7 +102,12 @@ struct Ctx {
 };
 
 int tables_for(Ctx *c, int m, const double2 **tw, const double **sn);
+// lengths without an FFT kernel (hh_dst_dense.cu): the sine table of length n (once per context),
+// and the transform of nlines rows (element j at line ld + j) or columns (line + j ld) of each plane;
+// in may equal out
 int dense_for(Ctx *c, int n, const double **mat);
+int launch_dst_dense(Ctx *c, int n, bool cols, long nlines, long planes, const double2 *in, long in_ld, long in_plane,
+                     double2 *out, long out_ld, long out_plane);
 // builds (once per context) the tables that DSTs of length n use
 int prepare_dst(Ctx *c, int n);
 

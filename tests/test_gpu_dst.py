@@ -159,3 +159,35 @@ def test_dst_cols_pitched(ctx, oracle, n):
         assert np.array_equal(got[:, ncols:], blk[:, ncols:])
     for p in range(planes - 1):
         assert np.array_equal(o[p * pstride + n * ld:(p + 1) * pstride], buf[p * pstride + n * ld:(p + 1) * pstride])
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 6, 8, 9, 15, 16, 17, 30, 31, 49, 64, 99, 125, 128, 300, 401, 701, 999])
+@pytest.mark.parametrize("rows,ncols,planes", [(3, 1, 2), (150, 31, 3), (20011, 125, 5)])
+def test_dst_any_length_tensor_core_tiles(ctx, n, rows, ncols, planes):
+    """Lengths without an FFT kernel (two half-size tensor-core products): odd and even lengths around
+    the tile sizes (8 outputs, 4 values, 4 lines), few and many lines (every lines-per-block choice), rows
+    and columns, in place and pitched, against numpy's FFT of the odd extension.  Sums of at most n / 2
+    products of values of order 1 stay within n eps of the exact value: 1e-13 at these lengths."""
+    if rows > 1000:
+        rows, planes = max(64, min(rows, 2_000_000 // n)), max(1, min(planes, 400_000 // (n * ncols)))
+    rng = np.random.default_rng(n + rows)
+
+    def want(x):
+        z = np.zeros(x.shape[:-1] + (1,))
+        y = np.fft.fft(np.concatenate([z, x, z, -x[..., ::-1]], axis=-1), axis=-1)[..., 1:n + 1]
+        return y * 0.5j * np.sqrt(2.0 / (n + 1))
+
+    x = rng.standard_normal((rows, n + 3)) + 1j * rng.standard_normal((rows, n + 3))
+    t = _dev(x)
+    ctx.dst1_rows(n, rows, t, t, in_ld=n + 3, out_ld=n + 3)
+    ctx.synchronize()
+    o = _host(t)
+    assert rel_err(o[:, :n], want(x[:, :n])) < 1e-13
+    assert np.array_equal(o[:, n:], x[:, n:])
+    x = rng.standard_normal((planes, n, ncols + 1)) + 1j * rng.standard_normal((planes, n, ncols + 1))
+    t = _dev(x)
+    ctx.dst1_cols(n, ncols, planes, t, ncols + 1, n * (ncols + 1), t)
+    ctx.synchronize()
+    o = _host(t)
+    assert rel_err(o[..., :ncols], want(x[..., :ncols].transpose(0, 2, 1)).transpose(0, 2, 1)) < 1e-13
+    assert np.array_equal(o[..., ncols], x[..., ncols])
