@@ -15,6 +15,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -26,9 +27,10 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall"] + ARCH
 CC_FLAGS = ["-O2", "-fPIC", "-std=gnu11", "-Wall"]
 
-CU_SOURCES = ["hh_api.cu", "hh_dst.cu", "hh_dst_dense.cu", "hh_tridiag.cu", "hh_server.cu", "hh_refine.cu", "hh_rhs.cu"]
+CU_SOURCES = ["hh_api.cu", "hh_dst.cu", "hh_dst_dense.cu", "hh_tridiag.cu", "hh_line_sym_real.cu",
+              "hh_line_sym_cplx.cu", "hh_server.cu", "hh_refine.cu", "hh_rhs.cu"]
 C_SOURCES = ["hh_coef.c"]
-HEADERS = ["hh_internal.cuh", "hh_tma.cuh"]
+HEADERS = ["hh_internal.cuh", "hh_tma.cuh", "hh_line.cuh", "hh_line_sym.cuh"]
 
 
 def _nvcc() -> str:
@@ -66,14 +68,16 @@ def build(verbose: bool = False, ptxas_info: bool = False) -> dict:
     os.makedirs(OBJ, exist_ok=True)
     nvcc, cc = _nvcc(), _cc()
     hdrs = [os.path.join(CSRC, h) for h in HEADERS] + [os.path.join(INCLUDE, "hh.h")]
-    objs = []
+    objs, jobs = [], []
     for src in CU_SOURCES:
         s = os.path.join(CSRC, src)
         o = os.path.join(OBJ, src + ".o")
         if _newer(o, [s] + hdrs) or ptxas_info:
             extra = ["-Xptxas", "-v"] if ptxas_info else []
-            _run([nvcc, *NVCC_FLAGS, *extra, "-I", INCLUDE, "-c", s, "-o", o], verbose or ptxas_info)
+            jobs.append([nvcc, *NVCC_FLAGS, *extra, "-I", INCLUDE, "-c", s, "-o", o])
         objs.append(o)
+    with ThreadPoolExecutor(max_workers=max(1, min(len(jobs), os.cpu_count() or 1))) as pool:
+        list(pool.map(lambda cmd: _run(cmd, verbose or ptxas_info), jobs))
     for src in C_SOURCES:
         s = os.path.join(CSRC, src)
         o = os.path.join(OBJ, src + ".o")

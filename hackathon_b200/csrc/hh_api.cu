@@ -395,6 +395,9 @@ static int plan_factor(hh_plan *pl, const std::vector<double2> &sub, const std::
         const double2 a = sub[(size_t)k * p.rows], b = sup[(size_t)k * p.rows];
         p.sym = a.x == b.x && a.y == b.y;
     }
+    p.real_coef = p.sym; // k2 (the source operator's k^2) is real then as well: k^2 h^2 is in every diagonal
+    for (int k = 0; k < 4 && p.real_coef; k++)
+        p.real_coef = sub[(size_t)k * p.rows].y == 0.0 && dia[(size_t)k * p.rows].y == 0.0;
     p.pf_ok = p.sym;
     for (int q = 0; q < p.lines && p.pf_ok; q++) {
         auto line_value = [&](const std::vector<double2> &tb) {

@@ -132,6 +132,7 @@ struct Plan {
     int      rows_kernel = 0;    // rows DST (n + 1 = 64 .. 1024): 0 default, 1 CTA ring, 2 per-warp buffers;
                                  // (n + 1 = 2048): 0, 1 two warps per line, 2 the Stockham kernel
     bool     sym = false;        // const_rows and sub == super on every line (constant k)
+    bool     real_coef = false;  // sym, and every coefficient of the lines real (k^2 real)
     bool     pf_ok = false;      // order-6 partial fractions well conditioned on every line
     double2 *subt = nullptr, *diagt = nullptr; // sub/diagonal row tables (4 * rows each)
     // super-diagonal(row, line) = rowc[0][row] mu[0][line] + rowc[1][row] mu[1][line] + rowc[2][row] mu[2][line] + rowc[3][row]

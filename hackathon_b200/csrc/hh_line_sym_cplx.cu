@@ -1,0 +1,10 @@
+// The symmetric line solve for complex line coefficients.
+#include "hh_line_sym.cuh"
+
+namespace hh {
+
+int launch_sym_cplx(Plan *p, const double2 *in, double2 *out, int batch, int src_order, const SymMulti *multi) {
+    return launch_sym_order<double2>(p, in, out, batch, src_order, multi);
+}
+
+} // namespace hh

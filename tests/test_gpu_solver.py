@@ -377,3 +377,32 @@ def test_rows_2047_two_warp_and_stockham_kernels_agree(ctx):
     assert torch.equal(outs[0], outs[1])
     assert ((outs[2] - outs[0]).abs().max() / outs[0].abs().max()).item() < 1e-12
     plan.close()
+
+
+@pytest.mark.parametrize("dim,n,order,k", [(2, 100, 6, 7j), (2, 255, 4, 12j), (3, 33, 6, 5j), (2, 64, 2, 3j),
+                                           (2, 130, 6, 20.0), (2, 130, 6, 20.0 + 1e-3j)])
+def test_real_and_complex_line_coefficients(ctx, oracle, dim, n, order, k):
+    """Plans whose k^2 is real (real or imaginary k) run the real-coefficient line solve, others the
+    complex one: every symmetric variant against the oracle, and solved beside a complex plan (where one
+    launch takes the complex kernel for both) the same bits."""
+    torch = pytest.importorskip("torch")
+    if dim == 2:
+        f = _source(n, n + order)
+        ref = oracle.pipeline_2d(n, order, k, f)
+        src = f[1:-1, 1:-1]
+    else:
+        f = W.source_3d(n, W.sine_modes(n, 8, n // 2, dim=3))
+        ref = oracle.pipeline_3d(n, order, k, f)
+        src = f[1:-1, 1:-1, 1:-1]
+    src = np.ascontiguousarray(src)
+    plan, other = hh.Plan.helmholtz(ctx, dim, n, order, k), hh.Plan.helmholtz(ctx, dim, n, order, 3.0 + 2.0j)
+    for v in range(2, 7):
+        plan.variant = other.variant = v
+        u = plan.solve_source_host(src)
+        assert rel_err(u, ref["sol"]) < TOL
+        both = torch.from_numpy(np.stack([src, src])).cuda()
+        hh.solve_source_multi([plan, other], [1, 1], both, both)
+        ctx.synchronize()
+        assert np.array_equal(both[0].cpu().numpy(), u)
+    plan.close()
+    other.close()
