@@ -142,6 +142,7 @@ struct SymParams {
     int     dim;
     double  linf, uinf;
     const double *pl, *pu; // Pade factors (rows >= 9 equal linf, uinf)
+    double        cz[16];  // (-linf)^(k+1): how an entering value of the forward Pade sweep reaches row k
 };
 
 // TMA-tile input of the symmetric line solve: one right-hand side of the CTA's CW lines arrives
@@ -183,6 +184,14 @@ __device__ __forceinline__ void sym_chunk(const double2 *__restrict__ in, double
     static_assert(!SEQ || (CW * NR <= 128 && NT >= 256), "cross-warp thread ranges");
     const int     t = threadIdx.x;
     const double2 zero = make_double2(0.0, 0.0);
+    // Order 6 with 16-row segments: the Pade sweeps forget their entering value within a segment (its
+    // factor shrinks by 0.101 a row, 1.2e-16 over 16 rows, less than the rounding of a row's own value), so a
+    // segment takes its entering value from the neighbouring segment alone, without a scan, and the
+    // forward sweep is completed as z_k + (-l)^(k+1) z_in, off the recurrence.  Segments past the first
+    // start beyond row 9, where the factors are the limit; the first has no entering value.  (Line solve with
+    // the scans -> without: 3D 255^3 x 4 506 -> 438 us, 127^3 x 16 207 -> 187 us, 2D 1023^2 x 64 552 -> 545 us,
+    // 2047^2 x 16 699 -> 672 us; errors against 64-bit solutions unchanged.)
+    constexpr bool WIN = SRC == 6 && KS >= 16;
     // Orders 0-4 keep the forward multipliers L_k and the reciprocal pivots ui_k in registers.
     // Order 6, where the two solves' rows fill the registers, keeps one value per row instead:
     // tau_k = s ui_k (= L_{k+1}), in the ui array or (16-row segments) in shared memory, one
@@ -309,8 +318,8 @@ __device__ __forceinline__ void sym_chunk(const double2 *__restrict__ in, double
 #pragma unroll
             for (int r = 0; r < NR; r++) {
                 yh[r] = zfms(v[r][k], l, yh[r]);
-                if constexpr (SRC == 6)
-                    zh[r] = zaxpy(g[r][k], -PL(k), zh[r]);
+                if constexpr (SRC == 6) zh[r] = zaxpy(g[r][k], -PL(k), zh[r]);
+                if constexpr (WIN) g[r][k] = zh[r];
             }
         }
         double2 Bfe[NR], bfe[NR];
@@ -320,7 +329,10 @@ __device__ __forceinline__ void sym_chunk(const double2 *__restrict__ in, double
             Bfe[r] = shfl_up2(Bf, CW);
             bfe[r] = zero;
             if (sl == SPW - 1) sm.BwF[r][w][c] = Bf;
-            if constexpr (SRC == 6) {
+            if constexpr (WIN) {
+                bfe[r] = shfl_up2(zh[r], CW);
+                if (sl == SPW - 1) sm.bwF[r][w][c] = zh[r];
+            } else if constexpr (SRC == 6) {
                 const double2 bf = sym_warp_scan<CW, true>(zh[r], ttF + t, NT, sl);
                 bfe[r] = shfl_up2(bf, CW);
                 if (sl == SPW - 1) sm.bwF[r][w][c] = bf;
@@ -357,7 +369,7 @@ __device__ __forceinline__ void sym_chunk(const double2 *__restrict__ in, double
                     sm.EF[r][x][cc] = E;
                     E = zfma(sm.BwF[r][x][cc], sm.AwF[x][cc], E);
                 }
-            } else if (t >= 128 && t < 128 + CW * NR) {
+            } else if (!WIN && t >= 128 && t < 128 + CW * NR) {
                 const int r = (t - 128) / CW, cc = (t - 128) % CW;
                 double2   E = zero;
 #pragma unroll
@@ -380,20 +392,21 @@ __device__ __forceinline__ void sym_chunk(const double2 *__restrict__ in, double
 #pragma unroll
                         for (int r = 0; r < NR; r++) {
                             EF[r] = zfma(sm.BwF[r][x][c], a, EF[r]);
-                            if constexpr (SRC == 6) eF[r] = zaxpy(sm.bwF[r][x][c], lds_keep(&sm.awF[x][c]), eF[r]);
+                            if constexpr (SRC == 6 && !WIN) eF[r] = zaxpy(sm.bwF[r][x][c], lds_keep(&sm.awF[x][c]), eF[r]);
                         }
                     }
                 }
             }
             const MT      AeF = lds_keep(tabF + LOG * NT + t);
             double        aeF = 0.0;
-            if constexpr (SRC == 6) aeF = lds_keep(ttF + LOG * NT + t);
+            if constexpr (SRC == 6 && !WIN) aeF = lds_keep(ttF + LOG * NT + t);
             double2 y[NR], z[NR];
 #pragma unroll
             for (int r = 0; r < NR; r++) {
                 y[r] = zfma(Bfe[r], AeF, SEQ ? sm.EF[r][w][c] : EF[r]);
                 z[r] = zero;
-                if constexpr (SRC == 6) z[r] = zaxpy(bfe[r], aeF, SEQ ? sm.eF[r][w][c] : eF[r]);
+                if constexpr (WIN) z[r] = sl > 0 ? bfe[r] : (w > 0 ? sm.bwF[r][w > 0 ? w - 1 : 0][c] : zero);
+                else if constexpr (SRC == 6) z[r] = zaxpy(bfe[r], aeF, SEQ ? sm.eF[r][w][c] : eF[r]);
             }
             // the rows keep ui_k y_k, so that the back substitution is x_k = ui_k y_k - tau_k x_{k+1}
             MT       tp = PCS ? PC(0) : tau_in;
@@ -414,7 +427,9 @@ __device__ __forceinline__ void sym_chunk(const double2 *__restrict__ in, double
                 for (int r = 0; r < NR; r++) {
                     y[r] = zfms(v[r][k], l, y[r]);
                     v[r][k] = cmul(u, y[r]);
-                    if constexpr (SRC == 6) {
+                    if constexpr (WIN) {
+                        g[r][k] = zaxpy(g[r][k], sp.cz[k], z[r]);
+                    } else if constexpr (SRC == 6) {
                         z[r] = zaxpy(g[r][k], -PL(k), z[r]);
                         g[r][k] = z[r];
                     }
@@ -441,7 +456,10 @@ __device__ __forceinline__ void sym_chunk(const double2 *__restrict__ in, double
             Bbe[r] = shfl_down2(Bb, CW);
             bbe[r] = zero;
             if (sl == 0) sm.BwB[r][w][c] = Bb;
-            if constexpr (SRC == 6) {
+            if constexpr (WIN) {
+                bbe[r] = shfl_down2(wh[r], CW);
+                if (sl == 0) sm.bwB[r][w][c] = wh[r];
+            } else if constexpr (SRC == 6) {
                 const double2 bb = sym_warp_scan<CW, false>(wh[r], ttB + t, NT, sl);
                 bbe[r] = shfl_down2(bb, CW);
                 if (sl == 0) sm.bwB[r][w][c] = bb;
@@ -460,7 +478,7 @@ __device__ __forceinline__ void sym_chunk(const double2 *__restrict__ in, double
                     sm.EB[r][x][cc] = E;
                     E = zfma(sm.BwB[r][x][cc], sm.AwB[x][cc], E);
                 }
-            } else if (t >= 128 && t < 128 + CW * NR) {
+            } else if (!WIN && t >= 128 && t < 128 + CW * NR) {
                 const int r = (t - 128) / CW, cc = (t - 128) % CW;
                 double2   E = zero;
 #pragma unroll
@@ -483,21 +501,22 @@ __device__ __forceinline__ void sym_chunk(const double2 *__restrict__ in, double
 #pragma unroll
                         for (int r = 0; r < NR; r++) {
                             EB[r] = zfma(sm.BwB[r][xw][c], a, EB[r]);
-                            if constexpr (SRC == 6) eB[r] = zaxpy(sm.bwB[r][xw][c], lds_keep(&sm.awB[xw][c]), eB[r]);
+                            if constexpr (SRC == 6 && !WIN) eB[r] = zaxpy(sm.bwB[r][xw][c], lds_keep(&sm.awB[xw][c]), eB[r]);
                         }
                     }
                 }
             }
             const MT      AeB = lds_keep(tabB + LOG * NT + t);
             double        aeB = 0.0;
-            if constexpr (SRC == 6) aeB = lds_keep(ttB + LOG * NT + t);
+            if constexpr (SRC == 6 && !WIN) aeB = lds_keep(ttB + LOG * NT + t);
             double2 x[NR], ww[NR];
             const MT cTv = PCS ? PC(3) : cT;
 #pragma unroll
             for (int r = 0; r < NR; r++) {
                 x[r] = zfma(Bbe[r], AeB, SEQ ? sm.EB[r][w][c] : EB[r]);
                 ww[r] = zero;
-                if constexpr (SRC == 6) ww[r] = zaxpy(bbe[r], aeB, SEQ ? sm.eB[r][w][c] : eB[r]);
+                if constexpr (WIN) ww[r] = sl < SPW - 1 ? bbe[r] : (w < NW - 1 ? sm.bwB[r][w < NW - 1 ? w + 1 : w][c] : zero);
+                else if constexpr (SRC == 6) ww[r] = zaxpy(bbe[r], aeB, SEQ ? sm.eB[r][w][c] : eB[r]);
             }
 #pragma unroll
             for (int k = KS - 1; k >= 0; k--) {
@@ -736,18 +755,20 @@ __global__ void __launch_bounds__(NT, MINB)
             sm.pl[t] = t < 9 ? sp.pl[t] : (t == 9 ? sp.linf : 0.0);
             sm.pu[t] = t < 9 ? sp.pu[t] : (t == 9 ? sp.uinf : 0.0);
         }
-        __syncthreads();
-        double af = 1.0, ab = 1.0;
+        if constexpr (KS < 16) { // (16-row segments need no Pade scan)
+            __syncthreads();
+            double af = 1.0, ab = 1.0;
 #pragma unroll
-        for (int k = 0; k < KS; k++) {
-            const int r = r0 + k;
-            af *= -(r < 9 ? sm.pl[r] : (r < rows ? sp.linf : 0.0));
-            ab *= -(r < 9 ? sm.pu[r] : (r < rows ? sp.uinf : 0.0));
+            for (int k = 0; k < KS; k++) {
+                const int r = r0 + k;
+                af *= -(r < 9 ? sm.pl[r] : (r < rows ? sp.linf : 0.0));
+                ab *= -(r < 9 ? sm.pu[r] : (r < rows ? sp.uinf : 0.0));
+            }
+            const double totF = sym_scan_table<CW, true>(af, ttF + t, NT, sl, 1.0);
+            const double totB = sym_scan_table<CW, false>(ab, ttB + t, NT, sl, 1.0);
+            if (sl == SPW - 1) sm.awF[w][c] = totF;
+            if (sl == 0) sm.awB[w][c] = totB;
         }
-        const double totF = sym_scan_table<CW, true>(af, ttF + t, NT, sl, 1.0);
-        const double totB = sym_scan_table<CW, false>(ab, ttB + t, NT, sl, 1.0);
-        if (sl == SPW - 1) sm.awF[w][c] = totF;
-        if (sl == 0) sm.awB[w][c] = totB;
     }
     __syncthreads();
 
@@ -811,6 +832,8 @@ static int launch_sym_t(Plan *p, const double2 *in, double2 *out, int batch, con
     sp.uinf = p->pade_uinf;
     sp.pl = p->pade_l;
     sp.pu = p->pade_u;
+    double cz = 1.0;
+    for (int k = 0; k < 16; k++) sp.cz[k] = cz *= -p->pade_linf;
     const int io_elems = TIO ? sym_tile_elems(p->rows, CW) * SymTileBufs<SRC, MT>::value : NR * (KS + 2) * NT;
     const int shm = 128 + (int)(sizeof(double2) * io_elems +
                                 sizeof(MT) * (2 * (LOG + 1) * NT + (SymUIS<SRC, KS, MT>::value ? KS * NT : 0) +
