@@ -6,19 +6,26 @@
 // The Helmholtz plans apply the constant-k operator in the mode basis inside the line solve
 // (hh_tridiag.cu); this file is the general form, used where k varies along the line direction
 // or the boundary data is not zero.  Its pieces:
-//  * Pade derivatives: each line of the extended grid along one axis gets its compact
-//    right-hand side (12 (f_- - 2 f_0 + f_+) / h^2 for [1 10 1], 3 (f_+ - f_-) / h for [1 4 1]),
-//    the boundary values subtracted at its two ends, and the Thomas recurrence of
-//    tridiag(1, diag, 1) with the reference's factors (L_j = 1/U_{j-1}, U_j = diag - L_j,
-//    division by U_j) -- one thread per line, sequential along it;
+//  * Pade derivatives (k_pade): T^-1 v along one axis, T = tridiag(1, d, 1), v the compact right-hand side
+//    (12 (f_- - 2 f_0 + f_+) / h^2 for d = 10, 3 (f_+ - f_-) / h for d = 4) with the boundary values subtracted
+//    at its two ends;
 //  * the pointwise combination of rhs.c (2D :78-86, 3D :149-166) with the second-order
-//    differences of 2nd_order*.c inline;
-//  * the Dirichlet corrections of the edges (2D rhs.c:126-148) or z faces (3D rhs.c:167-174).
+//    differences of 2nd_order*.c inline, and the Dirichlet corrections of the edges (2D rhs.c:126-148)
+//    or z faces (3D rhs.c:167-174) at the points they reach.
+//
+// T^-1 without a sequential pass.  The Thomas recurrence of the reference runs a line from end to end;
+// one thread per line left most of the chip idle (2D 511^2: 0.66 to 0.89 ms per derivative).  Here T
+// is extended to the whole axis by odd reflection at both ends (v_{-1} = 0, v_{-1-k} = -v_{-1+k}), which
+// leaves its solution unchanged, and on the whole axis
+//     (T^-1 v)_i = (v_i - r (F_{i-1} + B_{i+1})) / sqrt(d^2 - 4),  F_i = v_i - r F_{i-1},  B_i = v_i - r B_{i+1},
+// r = (d - sqrt(d^2 - 4)) / 2.  F and B forget their start by r per point (0.101 at d = 10, 0.268 at d = 4), so a
+// thread forms them for its 8 points from W points outside (r^W < 1.3e-17), independently of every other.
 // Arithmetic follows the reference's expression order (complex throughout: where the reference's
 // 3D rhs.c:149 keeps its partial sums in real doubles, here they stay complex; the two agree for
 // real data, which is what the reference's own problems have).
 #include "hh_internal.cuh"
 
+#include <math.h>
 #include <string.h>
 
 #include <algorithm>
@@ -28,225 +35,299 @@ namespace hh {
 
 namespace {
 
-// lines along one axis of the extended grid: line t has interior cross coordinates
-// c1 = t % n1 + 1, c2 = t / n1 + 1; its point m (0..n-1) is at c1 s1 + c2 s2 + (m + 1) sa
-struct AxisLines {
-    int  n, n1;
-    long nlines;
-    long s1, s2, sa;
-    long b2;    // boundary-array stride of the second cross coordinate (the first has stride 1)
-    int  bsh;   // added to c1 when indexing the boundary array (fy_yb is indexed by interior x)
-    long bface; // offset of the far end's boundary values
+constexpr int kPadeThreads = 256, kSegP = 8;
+constexpr int kSpanS = 64;           // outputs of a block along a strided axis: 8 segments x 32 columns
+constexpr int kSpanX = 128, kRowsX = 16; // along x: 16 segments x 16 rows
+
+// One derivative along one axis.  Line (c1, c2), 0 <= c1 < n1, 0 <= c2 < n2, has its interior point m
+// (0 <= m < n) at f[f0 + c1 f1 + c2 f2 + m fa] (its neighbours at distance fa, the boundary points included)
+// and its derivative at out[c1 o1 + c2 o2 + m oa]; its boundary values are bc[b0 + c1 + c2 b2] (near) and
+// bface further on (far).  Strided axes have f1 = o1 = 1 (c1 runs along x), the x axis fa = oa = 1.
+struct PadeJob {
+    const double2 *f, *bc;
+    double2       *out;
+    int            n, n1, n2, w, first, xdir;
+    long           f0, f1, f2, fa, o1, o2, oa, b0, b2, bface;
+    double         scale, scale_lo; // 12 / h^2 (or 3 / h) as a sum of two doubles
+    double         r, inv;          // the decay of F and B, 1 / sqrt(d^2 - 4)
+    unsigned       blocks, gx, gy;  // the job's blocks: gx by gy by (rest)
+};
+struct PadeJobs {
+    PadeJob j[3];
+    int     count;
 };
 
-__global__ void k_pade_lines(const double2 *__restrict__ f, double2 *__restrict__ out, AxisLines g, int first,
-                             int plus_first, double h, const double2 *__restrict__ bc, const double *__restrict__ Lf,
-                             const double *__restrict__ Uf) {
-    const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (t >= g.nlines) return;
-    const long c1 = t % g.n1 + 1, c2 = t / g.n1 + 1;
-    const long base = c1 * g.s1 + c2 * g.s2;
-    const int  n = g.n;
-    for (int m = 0; m < n; m++) {
-        const long    e = base + (long)(m + 1) * g.sa;
-        const double2 lo = f[e - g.sa], c = f[e], hi = f[e + g.sa];
-        double2       v;
-        if (first) {
-            v = make_double2(3.0 * (hi.x - lo.x) / h, 3.0 * (hi.y - lo.y) / h);
-        } else if (plus_first) { // 12 (f_+ - 2 f_0 + f_-) / h / h
-            v = make_double2(12.0 * (hi.x - 2.0 * c.x + lo.x) / h / h, 12.0 * (hi.y - 2.0 * c.y + lo.y) / h / h);
-        } else { // 12 (f_- - 2 f_0 + f_+) / h / h
-            v = make_double2(12.0 * (lo.x - 2.0 * c.x + hi.x) / h / h, 12.0 * (lo.y - 2.0 * c.y + hi.y) / h / h);
-        }
-        if (bc && (m == 0 || m == n - 1)) {
-            const long    bi = c1 + g.bsh + c2 * g.b2 + (m == 0 ? 0 : g.bface);
-            const double2 b = bc[bi];
-            v = make_double2(v.x - b.x, v.y - b.y);
-            if (n == 1) { // a one-point line subtracts both ends
-                const double2 b1 = bc[c1 + g.bsh + c2 * g.b2 + g.bface];
-                v = make_double2(v.x - b1.x, v.y - b1.y);
-            }
-        }
-        out[e] = v;
-    }
-    // tridiag(1, diag, 1): v_m -= L_m v_{m-1};  v_{n-1} /= U_{n-1};  v_m = (v_m - v_{m+1}) / U_m
-    double2 prev = out[base + g.sa];
-    for (int m = 1; m < n; m++) {
-        const long e = base + (long)(m + 1) * g.sa;
-        double2    v = out[e];
-        v = make_double2(v.x - Lf[m] * prev.x, v.y - Lf[m] * prev.y);
-        out[e] = v;
-        prev = v;
-    }
-    {
-        const long e = base + (long)n * g.sa;
-        const double2 v = out[e];
-        prev = make_double2(v.x / Uf[n - 1], v.y / Uf[n - 1]);
-        out[e] = prev;
-    }
-    for (int m = n - 2; m >= 0; m--) {
-        const long e = base + (long)(m + 1) * g.sa;
-        const double2 v = out[e];
-        prev = make_double2((v.x - prev.x) / Uf[m], (v.y - prev.y) / Uf[m]);
-        out[e] = prev;
-    }
+__device__ __forceinline__ double2 zaxpy_r(double2 a, double b, double2 c) { // a + b c, b real
+    return make_double2(fma(b, c.x, a.x), fma(b, c.y, a.y));
 }
 
-// values of an extended-grid array on two opposite faces: face value (c1, c2) of the near face
-// (index c1 + c2 * b2 of src) at c1 s1 + c2 s2 (+ far * sa), for c1 < n1, c2 < n2
-__global__ void k_fill_faces(double2 *__restrict__ dst, const double2 *__restrict__ src, int n1, int n2, long s1,
-                             long s2, long far_off, long b2, long bface) {
-    const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (t >= (long)n1 * n2) return;
-    const long c1 = t % n1, c2 = t / n1;
-    const double2 z = make_double2(0.0, 0.0);
-    dst[c1 * s1 + c2 * s2] = src ? src[c1 + c2 * b2] : z;
-    dst[c1 * s1 + c2 * s2 + far_off] = src ? src[c1 + c2 * b2 + bface] : z;
+// v_m of a line, extended by odd reflection
+__device__ __forceinline__ double2 pade_rhs(const PadeJob &J, int c1, int c2, int m) {
+    double sgn = 1.0;
+    if (m < 0 || m >= J.n) {
+        const int per = 2 * (J.n + 1);
+        int       q = (m + 1) % per;
+        if (q < 0) q += per;
+        if (q == 0 || q == J.n + 1) return make_double2(0.0, 0.0);
+        if (q > J.n + 1) {
+            q = per - q;
+            sgn = -1.0;
+        }
+        m = q - 1;
+    }
+    const double2 *e = J.f + J.f0 + c1 * J.f1 + c2 * J.f2 + (long)m * J.fa;
+    const double2  lo = __ldg(e - J.fa), hi = __ldg(e + J.fa);
+    double2        v;
+    if (J.first) {
+        v = make_double2(hi.x - lo.x, hi.y - lo.y);
+    } else {
+        const double2 c = __ldg(e);
+        v = make_double2(lo.x - 2.0 * c.x + hi.x, lo.y - 2.0 * c.y + hi.y);
+    }
+    v = make_double2(fma(v.x, J.scale, v.x * J.scale_lo), fma(v.y, J.scale, v.y * J.scale_lo));
+    if (J.bc && (m == 0 || m == J.n - 1)) {
+        const double2 b = J.bc[J.b0 + c1 + c2 * J.b2 + (m == 0 ? 0 : J.bface)];
+        v = make_double2(v.x - b.x, v.y - b.y);
+    }
+    return make_double2(sgn * v.x, sgn * v.y);
+}
+
+// Bound by shared memory and by the loads of f (each value read three times, from L1 and L2): the
+// segment of 8 points costs 2 (W + 8) steps of one fused multiply-add per component.  All derivatives of an
+// assembly share one launch (2D 511^2, with the combination: 2.31 ms -> 30 us; 3D 125^3: 0.73 -> 0.14 ms).
+__global__ void __launch_bounds__(kPadeThreads) k_pade(const __grid_constant__ PadeJobs jobs) {
+    extern __shared__ __align__(16) double2 pade_sm[];
+    unsigned blk = blockIdx.x;
+    int      ji = 0;
+    while (ji + 1 < jobs.count && blk >= jobs.j[ji].blocks) blk -= jobs.j[ji++].blocks;
+    const PadeJob &J = jobs.j[ji];
+    const int      t = threadIdx.x, W = J.w;
+    const unsigned bx = blk % J.gx, by = blk / J.gx % J.gy, bz = blk / J.gx / J.gy;
+    const double2  zero = make_double2(0.0, 0.0);
+    if (!J.xdir) {
+        // 32 neighbouring columns, kSpanS points: tile [point][column]
+        const int x0 = (int)bx * 32, m0 = (int)by * kSpanS, c2 = (int)bz;
+        const int len = min(kSpanS, J.n - m0) + 2 * W;
+        for (int e = t; e < len * 32; e += kPadeThreads) {
+            const int c = x0 + (e & 31);
+            pade_sm[e] = c < J.n1 ? pade_rhs(J, c, c2, m0 - W + (e >> 5)) : zero;
+        }
+        __syncthreads();
+        const int c = t & 31, i0 = (t >> 5) * kSegP; // the thread's first point within the span
+        if (m0 + i0 >= J.n || x0 + c >= J.n1) return;
+        const double2 *v = pade_sm + (i0 + W) * 32 + c;
+        const int      top = min(kSegP, J.n - m0 - i0); // points of this segment
+        double2        B = zero, Bn[kSegP], F = zero;
+        for (int m = top + W - 1; m >= kSegP; m--) B = zaxpy_r(v[m * 32], -J.r, B);
+#pragma unroll
+        for (int m = kSegP - 1; m >= 0; m--) {
+            Bn[m] = B;
+            if (m < top + W) B = zaxpy_r(v[m * 32], -J.r, B);
+        }
+        for (int m = -W; m < 0; m++) F = zaxpy_r(v[m * 32], -J.r, F);
+        double2 *o = J.out + (x0 + c) + c2 * J.o2 + (long)(m0 + i0) * J.oa;
+#pragma unroll
+        for (int m = 0; m < kSegP; m++) {
+            if (m < top) {
+                const double2 vm = v[m * 32];
+                const double2 u = zaxpy_r(vm, -J.r, make_double2(F.x + Bn[m].x, F.y + Bn[m].y));
+                o[m * J.oa] = make_double2(u.x * J.inv, u.y * J.inv);
+                F = zaxpy_r(vm, -J.r, F);
+            }
+        }
+    } else {
+        // kRowsX neighbouring rows, kSpanX points: tile [row][point + point / 8] (the segments of 8 start on
+        // different banks)
+        const int  m0 = (int)bx * kSpanX, len = min(kSpanX, J.n - m0) + 2 * W;
+        const int  pitch = (kSpanX + 2 * W) * 9 / 8 + 1;
+        const long row0 = (long)by * kRowsX, rows = (long)J.n1 * J.n2;
+        const int  nr = (int)min((long)kRowsX, rows - row0);
+        for (int r = t >> 5; r < nr; r += kPadeThreads / 32) {
+            const int c1 = (int)((row0 + r) % J.n1), c2 = (int)((row0 + r) / J.n1);
+            for (int e = t & 31; e < len; e += 32) pade_sm[r * pitch + e + (e >> 3)] = pade_rhs(J, c1, c2, m0 - W + e);
+        }
+        __syncthreads();
+        const int  r = t >> 4, i0 = (t & 15) * kSegP;
+        const bool live = r < nr && m0 + i0 < J.n;
+        const int  top = live ? min(kSegP, J.n - m0 - i0) : 0;
+        double2    u[kSegP];
+        if (live) {
+            double2 *row = pade_sm + r * pitch;
+            auto     V = [&](int m) { const int e = i0 + W + m; return row[e + (e >> 3)]; };
+            double2  B = zero, Bn[kSegP], F = zero;
+            for (int m = top + W - 1; m >= kSegP; m--) B = zaxpy_r(V(m), -J.r, B);
+#pragma unroll
+            for (int m = kSegP - 1; m >= 0; m--) {
+                Bn[m] = B;
+                if (m < top + W) B = zaxpy_r(V(m), -J.r, B);
+            }
+            for (int m = -W; m < 0; m++) F = zaxpy_r(V(m), -J.r, F);
+#pragma unroll
+            for (int m = 0; m < kSegP; m++) {
+                if (m < top) {
+                    const double2 vm = V(m);
+                    u[m] = zaxpy_r(vm, -J.r, make_double2(F.x + Bn[m].x, F.y + Bn[m].y));
+                    F = zaxpy_r(vm, -J.r, F);
+                }
+            }
+        }
+        __syncthreads(); // the tile takes the results, for contiguous stores
+#pragma unroll
+        for (int m = 0; m < kSegP; m++)
+            if (m < top) {
+                const int e = i0 + m;
+                pade_sm[r * pitch + e + (e >> 3)] = make_double2(u[m].x * J.inv, u[m].y * J.inv);
+            }
+        __syncthreads();
+        for (int q = t >> 5; q < nr; q += kPadeThreads / 32) {
+            const int c1 = (int)((row0 + q) % J.n1), c2 = (int)((row0 + q) / J.n1);
+            double2  *o = J.out + c1 * J.o1 + c2 * J.o2 + m0;
+            for (int e = t & 31; e < len - 2 * W; e += 32) o[e] = pade_sm[q * pitch + e + (e >> 3)];
+        }
+    }
 }
 
 __device__ __forceinline__ double2 zmul(double2 a, double2 b) { return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
 __device__ __forceinline__ double2 zadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 zsub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ double2 rmul(double a, double2 b) { return make_double2(a * b.x, a * b.y); }
-__device__ __forceinline__ double2 rdiv(double2 a, double b) { return make_double2(a.x / b, a.y / b); }
-// (a - 2 b + c) / h / h
-__device__ __forceinline__ double2 d2h(double2 a, double2 b, double2 c, double h) {
-    return make_double2((a.x - 2.0 * b.x + c.x) / h / h, (a.y - 2.0 * b.y + c.y) / h / h);
+// a - 2 b + c
+__device__ __forceinline__ double2 d2(double2 a, double2 b, double2 c) {
+    return make_double2(a.x - 2.0 * b.x + c.x, a.y - 2.0 * b.y + c.y);
 }
 
-// 2D combination, rhs.c:78-86 (order 6); orders 4 and 2, rhs.c:4-38
-__global__ void k_rhs2d_combine(int nx, int ny, int order, double hx, double hy, const double2 *__restrict__ fe,
-                                const double2 *__restrict__ fxx, const double2 *__restrict__ fyy,
-                                const double2 *__restrict__ fy, const double2 *__restrict__ k2c,
-                                const double2 *__restrict__ k2y, double2 *__restrict__ rhs) {
-    const long q = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (q >= (long)nx * ny) return;
-    const int  i = (int)(q % nx), j = (int)(q / nx);
-    const long E = nx + 2;
-    const long c = (i + 1) + (long)(j + 1) * E;
-    const double hy2 = hy * hy;
-    if (order == 6) {
-        const double  hy4 = hy2 * hy2, hx2 = hx * hx, hyy = hy * hy;
-        const double2 fxxxx = rdiv(zadd(zsub(fxx[c - 1], rmul(2.0, fxx[c])), fxx[c + 1]), hx2);
-        const double2 fxxyy = rdiv(zadd(zsub(fxx[c - E], rmul(2.0, fxx[c])), fxx[c + E]), hyy);
-        const double2 fyyyy = rdiv(zadd(zsub(fyy[c - E], rmul(2.0, fyy[c])), fyy[c + E]), hyy);
-        const double2 k2 = k2c[j];
-        const double2 t1 = zmul(make_double2(1.0 - k2.x * hy2 / 20.0, -(k2.y * hy2 / 20.0)), fe[c]);
-        const double2 t2 = rdiv(rmul(hy2, zadd(fxx[c], fyy[c])), 12.0);
-        const double2 t3 = rdiv(rmul(hy4, zadd(fxxxx, fyyyy)), 360.0);
-        const double2 t4 = rdiv(rmul(hy4, fxxyy), 90.0);
-        const double2 t5 = rdiv(zmul(rmul(hy4, k2y[j]), fy[c]), 60.0);
-        rhs[q] = rmul(hy2, zadd(zadd(zadd(zadd(t1, t2), t3), t4), t5));
-    } else if (order == 4) {
+// a field of derivatives at interior points, with its values on the boundary in two pairs of face arrays
+// (null: zero)
+struct Rhs2DArgs {
+    const double2 *fe, *fxx, *fyy, *fy, *k2c, *k2y;
+    const double2 *fxx_xb, *fxx_yb, *fyy_yb;
+    const double2 *subt, *diagt, *supt; // plan rows [4][prow]: sub (bm at [1], am at [3]), diag (b at [1]), super (bp, ap)
+    const double  *ux, *uy;
+    double2       *rhs;
+    int            nx, ny, order, prow;
+    double         h2, h2_20, c_f, c_xxxx, c_yyyy, c_xxyy, c_y; // h^2, h^2/20, h^2/12, h^4/(360 hx^2), ..., h^4/60
+};
+
+// 2D combination, rhs.c:78-86 (order 6); orders 4 and 2, rhs.c:4-38; then the Dirichlet corrections of
+// the points next to an edge, rhs.c:126-148 (the ring's corners belong to the edges y = const)
+__global__ void __launch_bounds__(256) k_rhs2d_combine(const __grid_constant__ Rhs2DArgs A) {
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31), j = blockIdx.y * 8 + (threadIdx.x >> 5);
+    if (i >= A.nx || j >= A.ny) return;
+    const int  nx = A.nx, ny = A.ny;
+    const long E = nx + 2, c = (i + 1) + (long)(j + 1) * E, q = i + (long)j * nx;
+    double2    r;
+    if (A.order == 6) {
+        const double2 zero = make_double2(0.0, 0.0);
+        auto face = [&](const double2 *b, long at) { return b ? b[at] : zero; };
+        const double2 xx = A.fxx[q], yy = A.fyy[q];
+        const double2 xl = i > 0 ? A.fxx[q - 1] : face(A.fxx_xb, j + 1);
+        const double2 xr = i + 1 < nx ? A.fxx[q + 1] : face(A.fxx_xb, ny + 2 + j + 1);
+        const double2 xd = j > 0 ? A.fxx[q - nx] : face(A.fxx_yb, i + 1);
+        const double2 xu = j + 1 < ny ? A.fxx[q + nx] : face(A.fxx_yb, E + i + 1);
+        const double2 yd = j > 0 ? A.fyy[q - nx] : face(A.fyy_yb, i + 1);
+        const double2 yu = j + 1 < ny ? A.fyy[q + nx] : face(A.fyy_yb, E + i + 1);
+        const double2 k2 = A.k2c[j];
+        const double2 t1 = zmul(make_double2(1.0 - k2.x * A.h2_20, -(k2.y * A.h2_20)), A.fe[c]);
+        const double2 t2 = rmul(A.c_f, zadd(xx, yy));
+        const double2 t3 = zadd(rmul(A.c_xxxx, d2(xl, xx, xr)), rmul(A.c_yyyy, d2(yd, yy, yu)));
+        const double2 t4 = rmul(A.c_xxyy, d2(xd, xx, xu));
+        const double2 t5 = zmul(rmul(A.c_y, A.k2y[j]), A.fy[q]);
+        r = rmul(A.h2, zadd(zadd(zadd(zadd(t1, t2), t3), t4), t5));
+    } else if (A.order == 4) {
         const double  a = 2.0 / 3.0, b = 1.0 / 12.0;
-        const double2 s = zadd(zadd(zadd(fe[c - E], fe[c + E]), fe[c - 1]), fe[c + 1]);
-        rhs[q] = rmul(hy2, zadd(rmul(a, fe[c]), rmul(b, s)));
+        const double2 s = zadd(zadd(zadd(A.fe[c - E], A.fe[c + E]), A.fe[c - 1]), A.fe[c + 1]);
+        r = rmul(A.h2, zadd(rmul(a, A.fe[c]), rmul(b, s)));
     } else {
-        rhs[q] = rmul(hy * hy, fe[c]);
+        r = rmul(A.h2, A.fe[c]);
     }
+    if ((A.ux || A.uy) && (i == 0 || j == 0 || i == nx - 1 || j == ny - 1)) {
+        auto U = [&](const double *a, long at) { return a ? a[at] : 0.0; };
+        auto ring = [&](int ie, int je) { // Dirichlet value at a point of the ring, zero inside
+            if (je == 0) return U(A.uy, ie);
+            if (je == ny + 1) return U(A.uy, E + ie);
+            if (ie == 0) return U(A.ux, je);
+            return ie == nx + 1 ? U(A.ux, ny + 2 + je) : 0.0;
+        };
+        auto sub = [&](double2 co, double u) { r = make_double2(r.x - co.x * u, r.y - co.y * u); };
+        const int p = A.prow;
+        sub(A.subt[p + j], ring(i, j));
+        sub(A.subt[3 * p + j], ring(i + 1, j));
+        sub(A.subt[p + j], ring(i + 2, j));
+        sub(A.diagt[p + j], ring(i, j + 1));
+        sub(A.diagt[p + j], ring(i + 2, j + 1));
+        sub(A.supt[p + j], ring(i, j + 2));
+        sub(A.supt[3 * p + j], ring(i + 1, j + 2));
+        sub(A.supt[p + j], ring(i + 2, j + 2));
+    }
+    A.rhs[q] = r;
 }
 
-// 2D Dirichlet corrections of the edges and corners, rhs.c:126-148.  t[] are the plan's row
-// tables [4][prow]: sub (bm at [1], am at [3]), diag (b at [1]), super (bp at [1], ap at [3]).
-__global__ void k_rhs2d_dirichlet(int nx, int ny, int prow, const double2 *__restrict__ subt,
-                                  const double2 *__restrict__ diagt, const double2 *__restrict__ supt,
-                                  const double *__restrict__ ux, const double *__restrict__ uy, double2 *__restrict__ rhs) {
-    const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    auto U = [&](const double *a, long i) { return a ? a[i] : 0.0; };
-    auto bm = [&](int j) { return subt[prow + j]; };
-    auto am = [&](int j) { return subt[3 * prow + j]; };
-    auto b = [&](int j) { return diagt[prow + j]; };
-    auto bp = [&](int j) { return supt[prow + j]; };
-    auto ap = [&](int j) { return supt[3 * prow + j]; };
-    auto sub = [&](long q, double2 co, double u) { rhs[q] = make_double2(rhs[q].x - co.x * u, rhs[q].y - co.y * u); };
-    const long xb1 = ny + 2, yb1 = nx + 2, top = (long)(ny - 1) * nx;
-    if (t == 0) {
-        sub(0, bm(0), U(uy, 0)); sub(0, am(0), U(uy, 1)); sub(0, bm(0), U(uy, 2));
-        sub(0, b(0), U(ux, 1)); sub(0, bp(0), U(ux, 2));
-        const long r = nx - 1;
-        sub(r, bm(0), U(uy, nx - 1)); sub(r, am(0), U(uy, nx)); sub(r, bm(0), U(uy, nx + 1));
-        sub(r, b(0), U(ux, xb1 + 1)); sub(r, bp(0), U(ux, xb1 + 2));
-        const int J = ny - 1;
-        sub(top, bm(J), U(ux, ny - 1)); sub(top, b(J), U(ux, ny));
-        sub(top, bp(J), U(uy, yb1 + 0)); sub(top, ap(J), U(uy, yb1 + 1)); sub(top, bp(J), U(uy, yb1 + 2));
-        const long tr = nx - 1 + top;
-        sub(tr, bm(J), U(ux, xb1 + ny - 1)); sub(tr, b(J), U(ux, xb1 + ny));
-        sub(tr, bp(J), U(uy, yb1 + nx + 1)); sub(tr, ap(J), U(uy, yb1 + nx)); sub(tr, bp(J), U(uy, yb1 + nx - 1));
-    } else if (t - 1 < ny - 2) {
-        const int  j = (int)(t - 1) + 1;
-        const long my = (long)j * nx;
-        sub(my, b(j), U(ux, j + 1)); sub(my, bm(j), U(ux, j)); sub(my, bp(j), U(ux, j + 2));
-        const long r = my + nx - 1;
-        sub(r, b(j), U(ux, xb1 + j + 1)); sub(r, bm(j), U(ux, xb1 + j)); sub(r, bp(j), U(ux, xb1 + j + 2));
-    } else if (t - 1 - (ny - 2) < nx - 2) {
-        const int i = (int)(t - 1 - (ny - 2)) + 1;
-        sub(i, am(0), U(uy, i + 1)); sub(i, bm(0), U(uy, i)); sub(i, bm(0), U(uy, i + 2));
-        const long r = i + top;
-        const int  J = ny - 1;
-        sub(r, ap(J), U(uy, yb1 + i + 1)); sub(r, bp(J), U(uy, yb1 + i)); sub(r, bp(J), U(uy, yb1 + i + 2));
-    }
-}
+struct Rhs3DArgs {
+    const double2 *f, *fxx, *fyy, *fzz, *k2_ext, *kp;
+    const double2 *fxx_b, *fyy_b, *fzz_b; // face values, each near face then far face
+    const double2 *subt, *supt, *ue;
+    double2       *rhs;
+    int            nx, ny, nz, order, prow;
+    double h2_20, c_f, c_xxxx, c_yyyy, c_zzzz, c_xxyy, c_xxzz, c_yyzz, c_z; // hz^2/20, hz^2/12, hz^4/(360 hx^2), ..., hz^3/120
+};
 
-// 3D combination, rhs.c:149-166 (order 6); orders 4 and 2, rhs.c:13-62
-__global__ void k_rhs3d_combine(int nx, int ny, int nz, int order, double hx, double hy, double hz,
-                                const double2 *__restrict__ f, const double2 *__restrict__ fxx,
-                                const double2 *__restrict__ fyy, const double2 *__restrict__ fzz,
-                                const double2 *__restrict__ k2_ext, const double2 *__restrict__ kp,
-                                double2 *__restrict__ rhs) {
-    const long q = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    const long nxy = (long)nx * ny;
-    if (q >= nxy * nz) return;
-    const int  i = (int)(q % nx), j = (int)((q / nx) % ny), l = (int)(q / nxy);
-    const long Ex = nx + 2, Exy = (long)(nx + 2) * (ny + 2);
-    const long C = (i + 1) + (j + 1) * Ex + (l + 1) * Exy;
-    const long W = C - 1, E = C + 1, S = C - Ex, N = C + Ex, D = C - Exy, Up = C + Exy;
-    if (order == 6) {
-        const double2 fxxxx = d2h(fxx[W], fxx[C], fxx[E], hx), fyyyy = d2h(fyy[S], fyy[C], fyy[N], hy);
-        const double2 fzzzz = d2h(fzz[D], fzz[C], fzz[Up], hz), fxxyy = d2h(fxx[S], fxx[C], fxx[N], hy);
-        const double2 fxxzz = d2h(fxx[D], fxx[C], fxx[Up], hz), fyyzz = d2h(fyy[D], fyy[C], fyy[Up], hz);
-        const double2 k2 = k2_ext[l + 1];
-        const double2 first = zmul(make_double2(1.0 - k2.x * hz * hz / 20.0, -(k2.y * hz * hz / 20.0)), f[C]);
-        const double2 second = rmul(hz * hz / 12.0, zadd(zadd(fxx[C], fyy[C]), fzz[C]));
-        const double2 third = rmul(hz * hz * hz * hz / 360.0, zadd(zadd(fxxxx, fyyyy), fzzzz));
-        const double2 fourth = rmul(hz * hz * hz * hz / 90.0, zadd(zadd(fxxyy, fxxzz), fyyzz));
-        const double2 fifth = zmul(rmul(hz * hz * hz / 120.0, kp[l]), zsub(f[Up], f[D]));
-        rhs[q] = zadd(zadd(zadd(zadd(first, second), third), fourth), fifth);
-    } else if (order == 4) {
-        const double2 nb = zadd(zadd(zadd(zadd(zadd(f[W], f[E]), f[S]), f[N]), f[D]), f[Up]);
-        rhs[q] = zadd(f[C], rmul(1.0 / 12.0, zsub(nb, rmul(6.0, f[C]))));
+// 3D combination, rhs.c:149-166 (order 6); orders 4 and 2, rhs.c:13-62; then the z-face Dirichlet terms,
+// rhs.c:24-29, 55-62, 167-174: layer 0 with the sub-diagonal layer's stencil (am, bm, cm, dm of layer
+// 0), layer nz-1 with the super-diagonal one (ap..dp of nz-1).  fxx on the y and z faces, fyy on the x
+// and z faces and fzz on the x and y faces are zero, as the reference leaves them.
+__global__ void __launch_bounds__(256) k_rhs3d_combine(const __grid_constant__ Rhs3DArgs A) {
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31), j = blockIdx.y * 8 + (threadIdx.x >> 5), l = blockIdx.z;
+    if (i >= A.nx || j >= A.ny) return;
+    const int     nx = A.nx, ny = A.ny, nz = A.nz;
+    const long    Ex = nx + 2, Ey = ny + 2, Exy = Ex * Ey, nxy = (long)nx * ny;
+    const long    C = (i + 1) + (j + 1) * Ex + (l + 1) * Exy, q = i + (long)j * nx + l * nxy;
+    const double2 zero = make_double2(0.0, 0.0);
+    double2       r;
+    if (A.order == 6) {
+        auto face = [&](const double2 *b, long at) { return b ? b[at] : zero; };
+        const double2 xx = A.fxx[q], yy = A.fyy[q], zz = A.fzz[q];
+        const double2 xw = i > 0 ? A.fxx[q - 1] : face(A.fxx_b, (j + 1) + (l + 1) * Ey);
+        const double2 xe = i + 1 < nx ? A.fxx[q + 1] : face(A.fxx_b, (j + 1) + (l + 1) * Ey + Ey * (nz + 2));
+        const double2 xs = j > 0 ? A.fxx[q - nx] : zero, xn = j + 1 < ny ? A.fxx[q + nx] : zero;
+        const double2 xd = l > 0 ? A.fxx[q - nxy] : zero, xu = l + 1 < nz ? A.fxx[q + nxy] : zero;
+        const double2 ys = j > 0 ? A.fyy[q - nx] : face(A.fyy_b, (i + 1) + (l + 1) * Ex);
+        const double2 yn = j + 1 < ny ? A.fyy[q + nx] : face(A.fyy_b, (i + 1) + (l + 1) * Ex + Ex * (nz + 2));
+        const double2 yd = l > 0 ? A.fyy[q - nxy] : zero, yu = l + 1 < nz ? A.fyy[q + nxy] : zero;
+        const double2 zd = l > 0 ? A.fzz[q - nxy] : face(A.fzz_b, (i + 1) + (j + 1) * Ex);
+        const double2 zu = l + 1 < nz ? A.fzz[q + nxy] : face(A.fzz_b, (i + 1) + (j + 1) * Ex + Exy);
+        const double2 k2 = A.k2_ext[l + 1];
+        const double2 first = zmul(make_double2(1.0 - k2.x * A.h2_20, -(k2.y * A.h2_20)), A.f[C]);
+        const double2 second = rmul(A.c_f, zadd(zadd(xx, yy), zz));
+        const double2 third = zadd(zadd(rmul(A.c_xxxx, d2(xw, xx, xe)), rmul(A.c_yyyy, d2(ys, yy, yn))),
+                                   rmul(A.c_zzzz, d2(zd, zz, zu)));
+        const double2 fourth = zadd(zadd(rmul(A.c_xxyy, d2(xs, xx, xn)), rmul(A.c_xxzz, d2(xd, xx, xu))),
+                                    rmul(A.c_yyzz, d2(yd, yy, yu)));
+        const double2 fifth = zmul(rmul(A.c_z, A.kp[l]), zsub(A.f[C + Exy], A.f[C - Exy]));
+        r = zadd(zadd(zadd(zadd(first, second), third), fourth), fifth);
+    } else if (A.order == 4) {
+        const double2 nb = zadd(zadd(zadd(zadd(zadd(A.f[C - 1], A.f[C + 1]), A.f[C - Ex]), A.f[C + Ex]), A.f[C - Exy]), A.f[C + Exy]);
+        r = zadd(A.f[C], rmul(1.0 / 12.0, zsub(nb, rmul(6.0, A.f[C]))));
     } else {
-        rhs[q] = f[C];
+        r = A.f[C];
     }
-}
-
-// 3D z-face Dirichlet terms, rhs.c:24-29, 55-62, 167-174: layer 0 with the sub-diagonal layer's
-// stencil (am, bm, cm, dm of layer 0), layer nz-1 with the super-diagonal one (ap..dp of nz-1)
-__global__ void k_rhs3d_zfaces(int nx, int ny, int nz, int order, int prow, const double2 *__restrict__ subt,
-                               const double2 *__restrict__ supt, const double2 *__restrict__ ue,
-                               double2 *__restrict__ rhs) {
-    const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (t >= (long)nx * ny) return;
-    const int  i = (int)(t % nx), j = (int)(t / nx);
-    const long Ex = nx + 2, Exy = (long)(nx + 2) * (ny + 2), nxy = (long)nx * ny;
-    const long b = t, top = t + (long)(nz - 1) * nxy;
-    auto X = [&](int ie, int je, long le) { return ue[ie + je * Ex + le * Exy]; };
-    if (order == 2) {
-        rhs[b] = zsub(rhs[b], X(i + 1, j + 1, 0));
-        rhs[top] = zsub(rhs[top], X(i + 1, j + 1, nz + 1));
-        return;
+    if (A.ue) {
+        for (int far = 0; far < 2; far++) {
+            if (l != (far ? nz - 1 : 0)) continue;
+            const double2 *e = A.ue + (far ? (nz + 1) * Exy : 0);
+            auto           X = [&](int ie, int je) { return e[ie + je * Ex]; };
+            if (A.order == 2) {
+                r = zsub(r, X(i + 1, j + 1));
+                continue;
+            }
+            const double2 *tab = far ? A.supt : A.subt;
+            const double2  a = tab[l], bb = tab[A.prow + l], cc = tab[2 * A.prow + l], dd = tab[3 * A.prow + l];
+            r = zsub(r, zmul(a, zadd(zadd(zadd(X(i, j), X(i + 2, j)), X(i, j + 2)), X(i + 2, j + 2))));
+            r = zsub(r, zmul(bb, zadd(X(i, j + 1), X(i + 2, j + 1))));
+            r = zsub(r, zmul(cc, zadd(X(i + 1, j), X(i + 1, j + 2))));
+            r = zsub(r, zmul(dd, X(i + 1, j + 1)));
+        }
     }
-    for (int face = 0; face < 2; face++) {
-        const long   le = face ? nz + 1 : 0, q = face ? top : b;
-        const double2 *tab = face ? supt : subt;
-        const int      row = face ? nz - 1 : 0;
-        const double2  a = tab[row], bb = tab[prow + row], cc = tab[2 * prow + row], dd = tab[3 * prow + row];
-        double2 r = rhs[q];
-        r = zsub(r, zmul(a, zadd(zadd(zadd(X(i, j, le), X(i + 2, j, le)), X(i, j + 2, le)), X(i + 2, j + 2, le))));
-        r = zsub(r, zmul(bb, zadd(X(i, j + 1, le), X(i + 2, j + 1, le))));
-        r = zsub(r, zmul(cc, zadd(X(i + 1, j, le), X(i + 1, j + 2, le))));
-        r = zsub(r, zmul(dd, X(i + 1, j + 1, le)));
-        rhs[q] = r;
-    }
+    A.rhs[q] = r;
 }
 
 // Pade factors of tridiag(1, diag, 1) over n points, as the reference forms them
@@ -311,26 +392,77 @@ static int upload_tables(Ctx *c, TableArea &ta, char **dev) {
         HH_CUDA(cudaMalloc(&c->rhs_tab, ta.host.size()));
         c->rhs_tab_bytes = ta.host.size();
     }
+    // a copy from pageable memory returns once the values are staged, so the caller may free them; a
+    // capture would record their address instead
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    HH_CUDA(cudaStreamIsCapturing(c->stream, &cap));
+    if (cap != cudaStreamCaptureStatusNone) {
+        set_error("the order-6 right-hand side copies its k profile from the host: not during stream capture");
+        return HH_ERR_CUDA;
+    }
     HH_CUDA(cudaMemcpyAsync(c->rhs_tab, ta.host.data(), ta.host.size(), cudaMemcpyHostToDevice, c->stream));
-    // the upload reads pageable host memory the caller is about to free: wait for it
-    HH_CUDA(cudaStreamSynchronize(c->stream));
     *dev = static_cast<char *>(c->rhs_tab);
     return HH_OK;
 }
 
-static unsigned blocks_for(long n, int nt) { return (unsigned)std::max<long>(1, (n + nt - 1) / nt); }
+// a derivative job over tridiag(1, diag, 1) (10: second derivative, 4: first) with spacing h
+static PadeJob pade_job(const double2 *f, double2 *out, const double *bc, int n, int n1, int n2, int diag, double h, bool xdir) {
+    PadeJob J{};
+    J.f = f;
+    J.out = out;
+    J.bc = (const double2 *)bc;
+    J.n = n;
+    J.n1 = n1;
+    J.n2 = n2;
+    J.first = diag == 4;
+    J.xdir = xdir;
+    J.w = diag == 4 ? 30 : 17; // r^w: 7e-18, 1.2e-17
+    const long double hl = h, sc = diag == 4 ? 3.0L / hl : 12.0L / (hl * hl);
+    J.scale = (double)sc;
+    J.scale_lo = (double)(sc - (long double)J.scale);
+    const long double root = sqrtl((long double)diag * diag - 4.0L);
+    J.r = (double)(2.0L / (diag + root));
+    J.inv = (double)(1.0L / root);
+    if (xdir) {
+        J.gx = (unsigned)((n + kSpanX - 1) / kSpanX);
+        J.gy = (unsigned)(((long)n1 * n2 + kRowsX - 1) / kRowsX);
+        J.blocks = J.gx * J.gy;
+    } else {
+        J.gx = (unsigned)((n1 + 31) / 32);
+        J.gy = (unsigned)((n + kSpanS - 1) / kSpanS);
+        J.blocks = J.gx * J.gy * (unsigned)n2;
+    }
+    return J;
+}
+
+static int launch_pade(Ctx *c, const PadeJobs &jobs) {
+    long   blocks = 0;
+    size_t shm = 0;
+    for (int i = 0; i < jobs.count; i++) {
+        const PadeJob &J = jobs.j[i];
+        blocks += J.blocks;
+        shm = std::max(shm, sizeof(double2) * (J.xdir ? (size_t)kRowsX * ((kSpanX + 2 * J.w) * 9 / 8 + 1)
+                                                      : (size_t)(kSpanS + 2 * J.w) * 32));
+    }
+    if (blocks > 0x7fffffffL) {
+        set_error("right-hand side: grid too large");
+        return HH_ERR_UNSUPPORTED;
+    }
+    HH_CUDA(cudaFuncSetAttribute(k_pade, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+    k_pade<<<(unsigned)blocks, kPadeThreads, shm, c->stream>>>(jobs);
+    HH_CUDA(cudaGetLastError());
+    c->launches++;
+    return HH_OK;
+}
 
 int assemble_rhs2d(Plan *p, const hh_rhs2d_data *d, double2 *rhs) {
-    Ctx      *c = p->ctx;
-    const int nx = p->nx, ny = p->ny, order = d->order;
-    const long E = nx + 2, next = E * (ny + 2);
-    const double2 *fe = (const double2 *)d->f_ext;
+    Ctx       *c = p->ctx;
+    const int  nx = p->nx, ny = p->ny, order = d->order;
+    const long E = nx + 2, nxy = (long)nx * ny;
+    Rhs2DArgs  A{};
+    A.fe = (const double2 *)d->f_ext;
     if (order == 6) {
-        double2 *w;
-        HH_TRY(rhs_work(c, 3 * next, &w));
-        double2 *fxx = w, *fyy = w + next, *fy = w + 2 * next;
-        HH_CUDA(cudaMemsetAsync(w, 0, sizeof(double2) * 3 * (size_t)next, c->stream));
-        // host: the k profiles (O(ny)) and the Pade factors
+        // host: the k profiles (O(ny))
         std::vector<double2> k2c((size_t)ny), k2y((size_t)ny);
         const double2       *ke = (const double2 *)d->k_ext;
         for (int j = 0; j < ny; j++) {
@@ -344,76 +476,59 @@ int assemble_rhs2d(Plan *p, const hh_rhs2d_data *d, double2 *rhs) {
             k2y[(size_t)ny - 1] = make_double2(k2y[(size_t)ny - 1].x - bc[1].x, k2y[(size_t)ny - 1].y - bc[1].y);
         }
         pade_host(k2y, 4.0);
-        std::vector<double> L4y, U4y, L10y, U10y, L10x, U10x;
-        pade_factors(ny, 4.0, L4y, U4y);
-        pade_factors(ny, 10.0, L10y, U10y);
-        pade_factors(nx, 10.0, L10x, U10x);
-        TableArea ta{c, {}, {}};
+        TableArea    ta{c, {}, {}};
         const size_t o_k2c = ta.add(k2c.data(), 16 * k2c.size()), o_k2y = ta.add(k2y.data(), 16 * k2y.size());
-        const size_t o_l4 = ta.add(L4y.data(), 8 * L4y.size()), o_u4 = ta.add(U4y.data(), 8 * U4y.size());
-        const size_t o_l10y = ta.add(L10y.data(), 8 * L10y.size()), o_u10y = ta.add(U10y.data(), 8 * U10y.size());
-        const size_t o_l10x = ta.add(L10x.data(), 8 * L10x.size()), o_u10x = ta.add(U10x.data(), 8 * U10x.size());
-        char *tab;
+        char        *tab;
         HH_TRY(upload_tables(c, ta, &tab));
-        auto T = [&](size_t off) { return reinterpret_cast<const double *>(tab + off); };
-        const int nt = 128;
+        double2 *w;
+        HH_TRY(rhs_work(c, 3 * nxy, &w));
+        double2 *fxx = w, *fyy = w + nxy, *fy = w + 2 * nxy;
+        PadeJobs jobs;
+        jobs.count = 3;
         // f_y: [1 4 1] along y (4th_order_first_derivative.c:60-98), boundary values fy_yb (interior x)
-        {
-            AxisLines g{ny, nx, (long)nx, 1, 0, E, 0, -1, (long)nx};
-            k_pade_lines<<<blocks_for(nx, nt), nt, 0, c->stream>>>(fe, fy, g, 1, 0, d->hy, (const double2 *)d->fy_yb, T(o_l4),
-                                                                   T(o_u4));
-        }
-        // f_yy: [1 10 1] along y (4th_order_second_derivative.c:61-120), then its edge values
-        {
-            AxisLines g{ny, nx, (long)nx, 1, 0, E, 0, 0, E};
-            k_pade_lines<<<blocks_for(nx, nt), nt, 0, c->stream>>>(fe, fyy, g, 0, 1, d->hy, (const double2 *)d->fyy_yb,
-                                                                   T(o_l10y), T(o_u10y));
-            k_fill_faces<<<blocks_for(E, nt), nt, 0, c->stream>>>(fyy, (const double2 *)d->fyy_yb, (int)E, 1, 1, 0,
-                                                                  (long)(ny + 1) * E, 0, E);
-            k_fill_faces<<<blocks_for(ny + 2, nt), nt, 0, c->stream>>>(fyy, (const double2 *)d->fyy_xb, ny + 2, 1, E, 0,
-                                                                       nx + 1, 0, ny + 2);
-        }
-        // f_xx: [1 10 1] along x (4th_order_second_derivative.c:4-59), then its edge values
-        {
-            AxisLines g{nx, ny, (long)ny, E, 0, 1, 0, 0, ny + 2};
-            k_pade_lines<<<blocks_for(ny, nt), nt, 0, c->stream>>>(fe, fxx, g, 0, 1, d->hx, (const double2 *)d->fxx_xb,
-                                                                   T(o_l10x), T(o_u10x));
-            k_fill_faces<<<blocks_for(E, nt), nt, 0, c->stream>>>(fxx, (const double2 *)d->fxx_yb, (int)E, 1, 1, 0,
-                                                                  (long)(ny + 1) * E, 0, E);
-            k_fill_faces<<<blocks_for(ny + 2, nt), nt, 0, c->stream>>>(fxx, (const double2 *)d->fxx_xb, ny + 2, 1, E, 0,
-                                                                       nx + 1, 0, ny + 2);
-        }
-        k_rhs2d_combine<<<blocks_for((long)nx * ny, 256), 256, 0, c->stream>>>(
-            nx, ny, 6, d->hx, d->hy, fe, fxx, fyy, fy, reinterpret_cast<const double2 *>(tab + o_k2c),
-            reinterpret_cast<const double2 *>(tab + o_k2y), rhs);
-        c->launches += 8;
-    } else {
-        k_rhs2d_combine<<<blocks_for((long)nx * ny, 256), 256, 0, c->stream>>>(nx, ny, order, d->hx, d->hy, fe, nullptr,
-                                                                              nullptr, nullptr, nullptr, nullptr, rhs);
-        c->launches++;
+        PadeJob &Y1 = jobs.j[0] = pade_job(A.fe, fy, d->fy_yb, ny, nx, 1, 4, d->hy, false);
+        Y1.f0 = 1 + E, Y1.f1 = 1, Y1.fa = E, Y1.o1 = 1, Y1.oa = nx, Y1.b0 = 0, Y1.bface = nx;
+        // f_yy: [1 10 1] along y (4th_order_second_derivative.c:61-120)
+        PadeJob &Y2 = jobs.j[1] = pade_job(A.fe, fyy, d->fyy_yb, ny, nx, 1, 10, d->hy, false);
+        Y2.f0 = 1 + E, Y2.f1 = 1, Y2.fa = E, Y2.o1 = 1, Y2.oa = nx, Y2.b0 = 1, Y2.bface = E;
+        // f_xx: [1 10 1] along x (4th_order_second_derivative.c:4-59)
+        PadeJob &X2 = jobs.j[2] = pade_job(A.fe, fxx, d->fxx_xb, nx, ny, 1, 10, d->hx, true);
+        X2.f0 = 1 + E, X2.f1 = E, X2.fa = 1, X2.o1 = nx, X2.oa = 1, X2.b0 = 1, X2.bface = ny + 2;
+        HH_TRY(launch_pade(c, jobs));
+        A.fxx = fxx, A.fyy = fyy, A.fy = fy;
+        A.k2c = reinterpret_cast<const double2 *>(tab + o_k2c);
+        A.k2y = reinterpret_cast<const double2 *>(tab + o_k2y);
+        A.fxx_xb = (const double2 *)d->fxx_xb;
+        A.fxx_yb = (const double2 *)d->fxx_yb;
+        A.fyy_yb = (const double2 *)d->fyy_yb;
     }
+    const double hx2 = d->hx * d->hx, hy2 = d->hy * d->hy, hy4 = hy2 * hy2;
+    A.h2 = hy2;
+    A.h2_20 = hy2 / 20.0;
+    A.c_f = hy2 / 12.0;
+    A.c_xxxx = hy4 / hx2 / 360.0;
+    A.c_yyyy = hy2 / 360.0;
+    A.c_xxyy = hy2 / 90.0;
+    A.c_y = hy4 / 60.0;
+    A.subt = p->subt, A.diagt = p->diagt, A.supt = p->rowc;
+    A.ux = d->u_xb, A.uy = d->u_yb;
+    A.rhs = rhs;
+    A.nx = nx, A.ny = ny, A.order = order, A.prow = p->prow;
+    dim3 grid((unsigned)((nx + 31) / 32), (unsigned)((ny + 7) / 8));
+    k_rhs2d_combine<<<grid, 256, 0, c->stream>>>(A);
     HH_CUDA(cudaGetLastError());
-    if (d->u_xb || d->u_yb) {
-        k_rhs2d_dirichlet<<<blocks_for(1 + (ny - 2) + (nx - 2), 128), 128, 0, c->stream>>>(
-            nx, ny, p->prow, p->subt, p->diagt, p->rowc, d->u_xb, d->u_yb, rhs);
-        HH_CUDA(cudaGetLastError());
-        c->launches++;
-    }
+    c->launches++;
     return HH_OK;
 }
 
 int assemble_rhs3d(Plan *p, const hh_rhs3d_data *d, double2 *rhs) {
     Ctx       *c = p->ctx;
     const int  nx = p->nx, ny = p->ny, nz = p->nz, order = d->order;
-    const long Ex = nx + 2, Ey = ny + 2, Exy = Ex * Ey, next = Exy * (nz + 2);
-    const double2 *f = (const double2 *)d->f_ext;
-    const int  nt = 128;
+    const long Ex = nx + 2, Ey = ny + 2, Exy = Ex * Ey, nxy = (long)nx * ny, n3 = nxy * nz;
+    Rhs3DArgs  A{};
+    A.f = (const double2 *)d->f_ext;
     if (order == 6) {
-        double2 *w;
-        HH_TRY(rhs_work(c, 3 * next, &w));
-        double2 *fxx = w, *fyy = w + next, *fzz = w + 2 * next;
-        HH_CUDA(cudaMemsetAsync(w, 0, sizeof(double2) * 3 * (size_t)next, c->stream));
-        // host: d(k^2)/dz by the [1 4 1] scheme (4th_order_partials.c:296-340), Pade factors
+        // host: d(k^2)/dz by the [1 4 1] scheme (4th_order_partials.c:296-340)
         const double2       *k2 = (const double2 *)d->k2_ext;
         std::vector<double2> kp((size_t)nz);
         for (int l = 0; l < nz; l++)
@@ -424,58 +539,56 @@ int assemble_rhs3d(Plan *p, const hh_rhs3d_data *d, double2 *rhs) {
             kp[(size_t)nz - 1] = make_double2(kp[(size_t)nz - 1].x + bc[1].x, kp[(size_t)nz - 1].y + bc[1].y);
         }
         pade_host(kp, 4.0);
-        std::vector<double> Lx, Ux, Ly, Uy, Lz, Uz;
-        pade_factors(nx, 10.0, Lx, Ux);
-        pade_factors(ny, 10.0, Ly, Uy);
-        pade_factors(nz, 10.0, Lz, Uz);
-        TableArea ta{c, {}, {}};
+        TableArea    ta{c, {}, {}};
         const size_t o_kp = ta.add(kp.data(), 16 * kp.size()), o_k2 = ta.add(k2, 16 * (size_t)(nz + 2));
-        const size_t o_lx = ta.add(Lx.data(), 8 * Lx.size()), o_ux = ta.add(Ux.data(), 8 * Ux.size());
-        const size_t o_ly = ta.add(Ly.data(), 8 * Ly.size()), o_uy = ta.add(Uy.data(), 8 * Uy.size());
-        const size_t o_lz = ta.add(Lz.data(), 8 * Lz.size()), o_uz = ta.add(Uz.data(), 8 * Uz.size());
-        char *tab;
+        char        *tab;
         HH_TRY(upload_tables(c, ta, &tab));
-        auto T = [&](size_t off) { return reinterpret_cast<const double *>(tab + off); };
+        double2 *w;
+        HH_TRY(rhs_work(c, 3 * n3, &w));
+        double2 *fxx = w, *fyy = w + n3, *fzz = w + 2 * n3;
+        PadeJobs jobs;
+        jobs.count = 3;
+        const long f0 = 1 + Ex + Exy;
         // f_xx along x (4th_order_partials.c:94-160): lines (j, l), boundary layout j + l (ny+2)
-        {
-            AxisLines g{nx, ny, (long)ny * nz, Ex, Exy, 1, Ey, 0, Ey * (nz + 2)};
-            k_pade_lines<<<blocks_for(g.nlines, nt), nt, 0, c->stream>>>(f, fxx, g, 0, 0, d->hx, (const double2 *)d->fxx_b,
-                                                                         T(o_lx), T(o_ux));
-            k_fill_faces<<<blocks_for(Ey * (nz + 2), nt), nt, 0, c->stream>>>(fxx, (const double2 *)d->fxx_b, (int)Ey, nz + 2,
-                                                                              Ex, Exy, nx + 1, Ey, Ey * (nz + 2));
-        }
+        PadeJob &X = jobs.j[0] = pade_job(A.f, fxx, d->fxx_b, nx, ny, nz, 10, d->hx, true);
+        X.f0 = f0, X.f1 = Ex, X.f2 = Exy, X.fa = 1, X.o1 = nx, X.o2 = nxy, X.oa = 1;
+        X.b0 = 1 + Ey, X.b2 = Ey, X.bface = Ey * (nz + 2);
         // f_yy along y (:162-227): lines (i, l), boundary layout i + l (nx+2)
-        {
-            AxisLines g{ny, nx, (long)nx * nz, 1, Exy, Ex, Ex, 0, Ex * (nz + 2)};
-            k_pade_lines<<<blocks_for(g.nlines, nt), nt, 0, c->stream>>>(f, fyy, g, 0, 0, d->hy, (const double2 *)d->fyy_b,
-                                                                         T(o_ly), T(o_uy));
-            k_fill_faces<<<blocks_for(Ex * (nz + 2), nt), nt, 0, c->stream>>>(fyy, (const double2 *)d->fyy_b, (int)Ex, nz + 2,
-                                                                              1, Exy, (long)(ny + 1) * Ex, Ex, Ex * (nz + 2));
-        }
+        PadeJob &Y = jobs.j[1] = pade_job(A.f, fyy, d->fyy_b, ny, nx, nz, 10, d->hy, false);
+        Y.f0 = f0, Y.f1 = 1, Y.f2 = Exy, Y.fa = Ex, Y.o1 = 1, Y.o2 = nxy, Y.oa = nx;
+        Y.b0 = 1 + Ex, Y.b2 = Ex, Y.bface = Ex * (nz + 2);
         // f_zz along z (:229-294): lines (i, j), boundary layout i + j (nx+2)
-        {
-            AxisLines g{nz, nx, (long)nx * ny, 1, Ex, Exy, Ex, 0, Exy};
-            k_pade_lines<<<blocks_for(g.nlines, nt), nt, 0, c->stream>>>(f, fzz, g, 0, 0, d->hz, (const double2 *)d->fzz_b,
-                                                                         T(o_lz), T(o_uz));
-            k_fill_faces<<<blocks_for(Exy, nt), nt, 0, c->stream>>>(fzz, (const double2 *)d->fzz_b, (int)Ex, (int)Ey, 1, Ex,
-                                                                    (long)(nz + 1) * Exy, Ex, Exy);
-        }
-        k_rhs3d_combine<<<blocks_for((long)nx * ny * nz, 256), 256, 0, c->stream>>>(
-            nx, ny, nz, 6, d->hx, d->hy, d->hz, f, fxx, fyy, fzz, reinterpret_cast<const double2 *>(tab + o_k2),
-            reinterpret_cast<const double2 *>(tab + o_kp), rhs);
-        c->launches += 7;
-    } else {
-        k_rhs3d_combine<<<blocks_for((long)nx * ny * nz, 256), 256, 0, c->stream>>>(
-            nx, ny, nz, order, d->hx, d->hy, d->hz, f, nullptr, nullptr, nullptr, nullptr, nullptr, rhs);
-        c->launches++;
+        PadeJob &Z = jobs.j[2] = pade_job(A.f, fzz, d->fzz_b, nz, nx, ny, 10, d->hz, false);
+        Z.f0 = f0, Z.f1 = 1, Z.f2 = Ex, Z.fa = Exy, Z.o1 = 1, Z.o2 = nx, Z.oa = nxy;
+        Z.b0 = 1 + Ex, Z.b2 = Ex, Z.bface = Exy;
+        HH_TRY(launch_pade(c, jobs));
+        A.fxx = fxx, A.fyy = fyy, A.fzz = fzz;
+        A.k2_ext = reinterpret_cast<const double2 *>(tab + o_k2);
+        A.kp = reinterpret_cast<const double2 *>(tab + o_kp);
+        A.fxx_b = (const double2 *)d->fxx_b;
+        A.fyy_b = (const double2 *)d->fyy_b;
+        A.fzz_b = (const double2 *)d->fzz_b;
     }
+    const double hx2 = d->hx * d->hx, hy2 = d->hy * d->hy, hz2 = d->hz * d->hz, hz4 = hz2 * hz2;
+    A.h2_20 = hz2 / 20.0;
+    A.c_f = hz2 / 12.0;
+    A.c_xxxx = hz4 / hx2 / 360.0;
+    A.c_yyyy = hz4 / hy2 / 360.0;
+    A.c_zzzz = hz2 / 360.0;
+    A.c_xxyy = hz4 / hy2 / 90.0;
+    A.c_xxzz = A.c_yyzz = hz2 / 90.0;
+    A.c_z = hz2 * d->hz / 120.0;
+    A.subt = p->subt, A.supt = p->rowc, A.ue = (const double2 *)d->ue_ext;
+    A.rhs = rhs;
+    A.nx = nx, A.ny = ny, A.nz = nz, A.order = order, A.prow = p->prow;
+    if (nz > 65535 || (ny + 7) / 8 > 65535) {
+        set_error("hh_rhs3d: %d x %d x %d is too large", nx, ny, nz);
+        return HH_ERR_UNSUPPORTED;
+    }
+    dim3 grid((unsigned)((nx + 31) / 32), (unsigned)((ny + 7) / 8), (unsigned)nz);
+    k_rhs3d_combine<<<grid, 256, 0, c->stream>>>(A);
     HH_CUDA(cudaGetLastError());
-    if (d->ue_ext) {
-        k_rhs3d_zfaces<<<blocks_for((long)nx * ny, 128), 128, 0, c->stream>>>(nx, ny, nz, order, p->prow, p->subt, p->rowc,
-                                                                             (const double2 *)d->ue_ext, rhs);
-        HH_CUDA(cudaGetLastError());
-        c->launches++;
-    }
+    c->launches++;
     return HH_OK;
 }
 

@@ -193,3 +193,55 @@ def test_reference_2d_problem_through_the_gpu(ctx):
     err = float(np.abs(sol.cpu().numpy() - d["exact"]).max())
     assert err < 1e-6 and abs(err - err_ref) < 1e-12 + 1e-6 * err_ref, (err, err_ref)
     plan.close()
+
+
+@pytest.mark.parametrize("n", [3, 5, 16, 17, 33, 63, 64, 65, 100, 129, 260])
+def test_rhs2d_segment_and_tile_edges(ctx, oracle, n):
+    """Lines shorter than the sweeps' reach (17 and 30 points: several reflections), around the segments
+    of 8, the spans of 64 and 128 and the blocks of 16 and 32 lines."""
+    rng = np.random.default_rng(n)
+    f_ext = _c(rng, (n + 2, n + 2))
+    k_ext = np.ascontiguousarray(8.0 + 4.0 * rng.random(n + 2) + 1j * rng.random(n + 2))
+    bnd = dict(k2y_ext=_c(rng, n + 2), k2yy=_c(rng, n), fxx_xb=_c(rng, 2 * (n + 2)), fxx_yb=_c(rng, 2 * (n + 2)),
+               fyy_xb=_c(rng, 2 * (n + 2)), fyy_yb=_c(rng, 2 * (n + 2)), fy_yb=_c(rng, 2 * n),
+               u_xb=rng.standard_normal(2 * (n + 2)), u_yb=rng.standard_normal(2 * (n + 2)))
+    # the two edges' arrays agree at the corners, as samples of one function do
+    for nm in ("u_xb", "u_yb"):
+        assert bnd[nm].shape == (2 * (n + 2),)
+    for far_x in (0, 1):
+        for far_y in (0, 1):
+            bnd["u_xb"][far_x * (n + 2) + far_y * (n + 1)] = bnd["u_yb"][far_y * (n + 2) + far_x * (n + 1)]
+    pb, keep = oracle.problem2d(n, 6, k_ext, f_ext, **bnd)
+    co = oracle.coefficients_2d(pb)
+    want = oracle.rhs_2d(pb, co)
+    plan = hh.Plan.from_coefficients_2d(ctx, n, n, co)
+    rhs = torch.empty((n, n), dtype=torch.complex128, device="cuda")
+    dev = {nm: _dev(bnd[nm]) for nm in ("fxx_xb", "fxx_yb", "fyy_xb", "fyy_yb", "fy_yb", "u_xb", "u_yb")}
+    plan.assemble_rhs(rhs, 6, (pb.hx, pb.hy), f_ext=_dev(f_ext), k_ext=k_ext,
+                      k2y_bc=[bnd["k2y_ext"][0], bnd["k2y_ext"][n + 1]], **dev)
+    ctx.synchronize()
+    assert rel_err(rhs.cpu().numpy(), want) < TOL
+    plan.close()
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(3, 4, 5), (16, 65, 8), (129, 7, 33), (31, 130, 66)])
+def test_rhs3d_segment_and_tile_edges(ctx, oracle, nx, ny, nz):
+    rng = np.random.default_rng(nx + ny + nz)
+    hx, hy, hz = 1.0 / (nx + 1), 0.9 / (ny + 1), 1.1 / (nz + 1)
+    k2_ext = _c(rng, nz + 2, 30.0)
+    data = dict(kz_bc=_c(rng, 2), kzz_bc=_c(rng, 2), ue_ext=_c(rng, (nz + 2, ny + 2, nx + 2)),
+                fxx_b=_c(rng, 2 * (ny + 2) * (nz + 2)), fyy_b=_c(rng, 2 * (nx + 2) * (nz + 2)),
+                fzz_b=_c(rng, 2 * (nx + 2) * (ny + 2)))
+    rhs_ext = _c(rng, (nz + 2, ny + 2, nx + 2))
+    pb, keep = oracle.problem3d(nx, 6, k2_ext, rhs_ext, hz, nxyz=(nx, ny, nz), **data)
+    pb.hx, pb.hy = hx, hy
+    co = oracle.coefficients_3d(pb)
+    want = oracle.rhs_3d(pb, co)
+    plan = hh.Plan.from_coefficients_3d(ctx, nx, ny, nz, co)
+    rhs = torch.empty((nz, ny, nx), dtype=torch.complex128, device="cuda")
+    plan.assemble_rhs(rhs, 6, (hx, hy, hz), f_ext=_dev(rhs_ext), k2_ext=k2_ext, kz_bc=data["kz_bc"],
+                      fxx_b=_dev(data["fxx_b"]), fyy_b=_dev(data["fyy_b"]), fzz_b=_dev(data["fzz_b"]),
+                      ue_ext=_dev(data["ue_ext"]))
+    ctx.synchronize()
+    assert rel_err(rhs.cpu().numpy(), want) < TOL
+    plan.close()
