@@ -59,6 +59,18 @@ int cuda_fail(cudaError_t e, const char *what, const char *file, int line) {
     return e == cudaErrorMemoryAllocation ? HH_ERR_NOMEM : HH_ERR_CUDA;
 }
 
+bool may_start_early(Ctx *c) {
+    const bool fresh = c->fresh;
+    c->fresh = false;
+    if (fresh || c->pool) return false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return cap == cudaStreamCaptureStatusNone;
+}
+
 static int upload(Ctx *c, void *dst, const void *src, size_t bytes) {
     HH_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream));
     return HH_OK;
@@ -160,6 +172,7 @@ extern "C" int hh_ctx_set_stream(hh_ctx *x, void *stream) {
     if (!x) return HH_ERR_INVALID;
     if (x->c.own_stream) { cudaStreamDestroy(x->c.stream); x->c.own_stream = false; }
     x->c.stream = (cudaStream_t)stream;
+    x->c.fresh = true;
     return HH_OK;
 }
 
@@ -367,6 +380,7 @@ static int plan_pade(hh_plan *pl) {
     }
     HH_TRY(dalloc(p.ctx, (void **)&p.pade_l, sizeof(double) * (size_t)p.prow));
     HH_TRY(dalloc(p.ctx, (void **)&p.pade_u, sizeof(double) * (size_t)p.prow));
+    p.ctx->fresh = true;
     HH_TRY(upload(p.ctx, p.pade_l, L.data(), sizeof(double) * (size_t)p.prow));
     HH_TRY(upload(p.ctx, p.pade_u, Ui.data(), sizeof(double) * (size_t)p.prow));
     return HH_OK;
@@ -423,6 +437,7 @@ static int plan_factor(hh_plan *pl, const std::vector<double2> &sub, const std::
     };
     const std::vector<double2> psub = padded(sub), pdia = padded(dia), psup = padded(sup);
     const size_t tb = sizeof(double2) * 4 * (size_t)p.prow;
+    c->fresh = true;
     int rc = upload(c, p.subt, psub.data(), tb);
     if (rc == HH_OK) rc = upload(c, p.diagt, pdia.data(), tb);
     if (rc == HH_OK) rc = upload(c, p.rowc, psup.data(), tb);

@@ -215,6 +215,8 @@ __global__ void __launch_bounds__(DstGeom<M>::NT)
     double2  *buf = reinterpret_cast<double2 *>(smem + G::HDR + slot * G::SLOT_BYTES);
     double2  *red = red_all + slot * G::WARPS;
 
+    pdl_wait();
+    pdl_next();
     const long line = (long)blockIdx.x * S + slot;
     const bool live = line < nlines;
     const long ibase = (long)blockIdx.y * in_plane, obase = (long)blockIdx.y * out_plane;
@@ -762,7 +764,13 @@ __global__ void __launch_bounds__(32 * WCfg<M>::WPC, WCfg<M>::MINB)
     auto dst_of = [&](long g) {
         return nplanes == 1 ? out + g * out_ld : out + (g / nlines) * out_plane + (g % nlines) * out_ld;
     };
+    WConst<M> K;
+    K.load(l, tw, sn);
     int injected = 0;
+    if (lane == 0) { // the fields are touched after a line group has arrived, so this lane's wait is enough
+        pdl_wait();
+        pdl_next();
+    }
     if (lane == 0 && inj && blockIdx.x == 0 && wq == 0) injected = atomicExch(inj, 0);
     injected = __shfl_sync(0xffffffffu, injected, 0);
     // lane 0: bring in line group `grp` to buffer set `s` (`extra`: injected bytes that never come)
@@ -783,8 +791,6 @@ __global__ void __launch_bounds__(32 * WCfg<M>::WPC, WCfg<M>::MINB)
         fetch(g0, 0, injected ? kInjectBytes : 0u);
         if (NBUF == 2 && g0 + stride < groups) fetch(g0 + stride, 1, 0u);
     }
-    WConst<M> K;
-    K.load(l, tw, sn);
 
     int  it = 0;
     long failed = -1;
@@ -886,14 +892,16 @@ __global__ void __launch_bounds__(32 * WCfg<M>::RWPC, 2)
             gen[b] = 0;
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        pdl_wait();
+        pdl_next();
         for (int b = 0; b < NS && b < tickets; b++) {
             fetch(b);
             gen[b] = 1;
         }
     }
-    __syncthreads();
     WConst<M> K;
     K.load(l, tw, sn);
+    __syncthreads();
 
     int failed = -1;
     for (int t = wq; t < tickets; t += WPC) {
@@ -1111,6 +1119,8 @@ __global__ void __launch_bounds__(64 * W2Geom<M>::TPC, 1)
             gen[b] = 0;
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        pdl_wait();
+        pdl_next();
         for (int b = 0; b < NS && b < tickets; b++) {
             fetch(b);
             gen[b] = 1;
@@ -1323,10 +1333,13 @@ __global__ void __launch_bounds__(32 * WCfg<M>::CWPC, 3)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
-    if (lane == 0)
-        for (int u = 0; u < NT && g0 + u * stride < groups; u++) fetch(g0 + u * stride, u);
     WConst<M> K;
     K.load(l, tw, sn);
+    if (lane == 0) {
+        pdl_wait();
+        pdl_next();
+        for (int u = 0; u < NT && g0 + u * stride < groups; u++) fetch(g0 + u * stride, u);
+    }
 
     int  it = 0;
     long failed = -1;
@@ -1432,11 +1445,13 @@ __global__ void __launch_bounds__(32 * WTile<M>::WPC)
     if (threadIdx.x == 0) {
         for (int u = 0; u < NT; u++) mbar_init(&full[u], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        pdl_wait();
+        pdl_next();
         for (int u = 0; u < NT && u < tickets; u++) fetch(u);
     }
-    __syncthreads();
     WConst<M> K;
     K.load(l, tw, sn);
+    __syncthreads();
 
     int failed = -1;
     for (int t = 0; t < tickets; t++) {
@@ -1502,6 +1517,7 @@ int tables_for(Ctx *c, int m, const double2 **tw, const double **sn) {
         k_make_tables<<<(m + 255) / 256, 256, 0, c->stream>>>(m, t2, s1);
         HH_CUDA(cudaGetLastError());
         c->launches++;
+        c->fresh = true;
         c->tw[m] = t2;
         c->sn[m] = s1;
         it = c->tw.find(m);
@@ -1540,11 +1556,8 @@ template <int M, bool IS, bool OS> static int launch_fft(Ctx *c, const DstArgs &
     HH_TRY(tables_for(c, M, &tw, &sn));
     HH_CUDA(cudaFuncSetAttribute(k_dst1<M, IS, OS>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM));
     dim3 grid((unsigned)((a.nlines + G::S - 1) / G::S), (unsigned)a.planes);
-    k_dst1<M, IS, OS><<<grid, G::NT, G::SMEM, c->stream>>>(a.in, a.out, a.nlines, a.in_ld, a.out_ld, a.in_plane,
+    return launch_kernel(c, k_dst1<M, IS, OS>, grid, G::NT, G::SMEM, a.in, a.out, a.nlines, a.in_ld, a.out_ld, a.in_plane,
                                                             a.out_plane, tw, sn, c->err_word);
-    HH_CUDA(cudaGetLastError());
-    c->launches++;
-    return HH_OK;
 }
 
 template <int M, bool LP, bool UPD = false> static int launch_wr(Ctx *c, const DstArgs &a) {
@@ -1560,11 +1573,8 @@ template <int M, bool LP, bool UPD = false> static int launch_wr(Ctx *c, const D
     HH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dst1_wr<M, LP, UPD>, 32 * RG::WPC, RG::SMEM));
     const long groups = (a.nlines * a.planes + G::LPW - 1) / G::LPW;
     const long ctas = std::min<long>((groups + RG::WPC - 1) / RG::WPC, (long)std::max(1, per_sm) * sms);
-    k_dst1_wr<M, LP, UPD><<<(unsigned)ctas, 32 * RG::WPC, RG::SMEM, c->stream>>>(
+    return launch_kernel(c, k_dst1_wr<M, LP, UPD>, dim3((unsigned)ctas), 32 * RG::WPC, RG::SMEM,
         a.in, a.out, a.nlines, a.planes, a.in_ld, a.out_ld, a.in_plane, a.out_plane, tw, sn, c->err_word);
-    HH_CUDA(cudaGetLastError());
-    c->launches++;
-    return HH_OK;
 }
 
 template <int M, bool LP, bool UPD = false> static int launch_wp(Ctx *c, const DstArgs &a) {
@@ -1579,12 +1589,9 @@ template <int M, bool LP, bool UPD = false> static int launch_wp(Ctx *c, const D
     HH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dst1_w<M, LP, UPD>, 32 * G::WPC, G::SMEM));
     const long groups = (a.nlines * a.planes + G::LPW - 1) / G::LPW;
     const long ctas = std::min<long>((groups + G::WPC - 1) / G::WPC, (long)std::max(1, per_sm) * sms);
-    k_dst1_w<M, LP, UPD><<<(unsigned)ctas, 32 * G::WPC, G::SMEM, c->stream>>>(a.in, a.out, a.nlines, a.planes, a.in_ld, a.out_ld,
+    return launch_kernel(c, k_dst1_w<M, LP, UPD>, dim3((unsigned)ctas), 32 * G::WPC, G::SMEM, a.in, a.out, a.nlines, a.planes, a.in_ld, a.out_ld,
                                                                      a.in_plane, a.out_plane, tw, sn, c->err_word,
                                                                      c->inject_word);
-    HH_CUDA(cudaGetLastError());
-    c->launches++;
-    return HH_OK;
 }
 
 template <int M, bool LP, bool UPD = false> static int launch_w2(Ctx *c, const DstArgs &a) {
@@ -1599,12 +1606,9 @@ template <int M, bool LP, bool UPD = false> static int launch_w2(Ctx *c, const D
     HH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dst1_w2<M, LP, UPD>, 64 * G::TPC, G::SMEM));
     const long lines = a.nlines * a.planes;
     const long ctas = std::min<long>((lines + G::TPC - 1) / G::TPC, (long)std::max(1, per_sm) * sms);
-    k_dst1_w2<M, LP, UPD><<<(unsigned)ctas, 64 * G::TPC, G::SMEM, c->stream>>>(a.in, a.out, a.nlines, a.planes, a.in_ld,
+    return launch_kernel(c, k_dst1_w2<M, LP, UPD>, dim3((unsigned)ctas), 64 * G::TPC, G::SMEM, a.in, a.out, a.nlines, a.planes, a.in_ld,
                                                                         a.out_ld, a.in_plane, a.out_plane, tw, sn,
                                                                         c->err_word);
-    HH_CUDA(cudaGetLastError());
-    c->launches++;
-    return HH_OK;
 }
 
 // rows kernel: a.rows_kernel 1 = the CTA ring, 2 = per-warp buffers, 0 = the length's default
@@ -1741,10 +1745,7 @@ static int launch_wc(Ctx *c, long ncols, long planes, const double2 *in, long ld
     HH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * CG::WPC, CG::SMEM));
     const long groups = (ncols + G::LPW - 1) / G::LPW * planes;
     const long ctas = std::min<long>((groups + CG::WPC - 1) / CG::WPC, (long)std::max(1, per_sm) * sms);
-    kern<<<(unsigned)ctas, 32 * CG::WPC, CG::SMEM, c->stream>>>(in_map, out_map, ncols, planes, tw, sn, c->err_word);
-    HH_CUDA(cudaGetLastError());
-    c->launches++;
-    return HH_OK;
+    return launch_kernel(c, kern, dim3((unsigned)ctas), 32 * CG::WPC, CG::SMEM, in_map, out_map, ncols, planes, tw, sn, c->err_word);
 }
 
 // (double, row, plane) map of column tiles: boxes of 16 doubles (8 complex columns) by br rows,
@@ -1776,10 +1777,7 @@ static int launch_wt(Ctx *c, long ncols, long planes, const double2 *in, long ld
     HH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * TG::WPC, TG::SMEM));
     const long groups = (ncols + TG::TC - 1) / TG::TC * planes;
     const long ctas = std::min<long>(groups, (long)std::max(1, per_sm) * sms);
-    kern<<<(unsigned)ctas, 32 * TG::WPC, TG::SMEM, c->stream>>>(in_map, out_map, ncols, planes, tw, sn, c->err_word);
-    HH_CUDA(cudaGetLastError());
-    c->launches++;
-    return HH_OK;
+    return launch_kernel(c, kern, dim3((unsigned)ctas), 32 * TG::WPC, TG::SMEM, in_map, out_map, ncols, planes, tw, sn, c->err_word);
 }
 
 int launch_dst_cols(Ctx *c, int n, long ncols, long planes, const double2 *in, long ld, long plane_stride,

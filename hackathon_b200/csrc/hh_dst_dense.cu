@@ -74,6 +74,8 @@ __global__ void __launch_bounds__(kMmaThreads, 3)
     in += (long)blockIdx.y * in_plane + (COLS ? l0 : l0 * in_ld);
     out += (long)blockIdx.y * out_plane + (COLS ? l0 : l0 * out_ld);
 
+    pdl_wait();
+    pdl_next();
     // ---- a_j and d_j of every line; zeros past the halves and for lines past the end
     auto put = [&](int at, int j, double2 x, double2 m) {
         const bool mid = 2 * j + 1 == n;
@@ -209,6 +211,8 @@ __global__ void __launch_bounds__(kDenseThreads)
     const long line = blockIdx.x;
     in += (long)blockIdx.y * in_plane;
     out += (long)blockIdx.y * out_plane;
+    pdl_wait();
+    pdl_next();
     for (int m = threadIdx.x; m < n; m += blockDim.x) x[m] = STRIDED ? in[line + (long)m * in_ld] : in[line * in_ld + m];
     __syncthreads();
     const double coef = sqrt(2.0 / (n + 1));
@@ -255,11 +259,8 @@ int launch_mma(Ctx *c, int n, long nlines, long planes, const double2 *in, long 
     const size_t shm = mma_smem(COLS, n, nl);
     HH_CUDA(cudaFuncSetAttribute(k_dst1_mma<COLS, NTW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
     dim3 grid((unsigned)((nlines + nl - 1) / nl), (unsigned)planes);
-    k_dst1_mma<COLS, NTW><<<grid, kMmaThreads, shm, c->stream>>>(in, out, n, nlines, in_ld, out_ld, in_plane, out_plane,
+    return launch_kernel(c, k_dst1_mma<COLS, NTW>, grid, kMmaThreads, shm, in, out, n, nlines, in_ld, out_ld, in_plane, out_plane,
                                                                  groups, tab);
-    HH_CUDA(cudaGetLastError());
-    c->launches++;
-    return HH_OK;
 }
 
 } // namespace
@@ -278,6 +279,7 @@ int dense_for(Ctx *c, int n, const double **mat) {
         }
         HH_CUDA(cudaGetLastError());
         c->launches++;
+        c->fresh = true;
         c->dense[n] = d;
         it = c->dense.find(n);
     }
@@ -294,10 +296,7 @@ int launch_dst_dense(Ctx *c, int n, bool cols, long nlines, long planes, const d
         auto         kern = cols ? k_dst1_dense<true> : k_dst1_dense<false>;
         HH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
         dim3 grid((unsigned)nlines, (unsigned)planes);
-        kern<<<grid, kDenseThreads, shm, c->stream>>>(in, out, n, in_ld, out_ld, in_plane, out_plane, mat);
-        HH_CUDA(cudaGetLastError());
-        c->launches++;
-        return HH_OK;
+        return launch_kernel(c, kern, grid, kDenseThreads, shm, in, out, n, in_ld, out_ld, in_plane, out_plane, mat);
     }
     const double2 *tab = reinterpret_cast<const double2 *>(mat);
     int ntw = 1, groups = 1;

@@ -660,6 +660,8 @@ __global__ void __launch_bounds__(NT, MINB)
             const int b0 = b_begin, b1 = b_end;
             for (int u = 0; u < NBUF; u++) mbar_init(tio.bar + u, 1);
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            pdl_wait(); // (the fields are written after a tile has arrived: this thread's wait is enough)
+            pdl_next();
             for (int u = 0; u < NBUF && b0 + u < b1; u++) {
                 double2 *dst = tio.tin + (long)u * tio.tile;
                 mbar_expect_tx(tio.bar + u, tio.tile_bytes);
@@ -772,6 +774,10 @@ __global__ void __launch_bounds__(NT, MINB)
     }
     __syncthreads();
 
+    if constexpr (!TIO) {
+        pdl_wait();
+        pdl_next();
+    }
     const long off0 = (long)r0 * row_stride + qq;
     // warps whose rows all lie in [9, rows) use the constant Pade factors
     const bool tint = (w * SPW * KS >= 9) && ((w + 1) * SPW * KS <= rows);
@@ -852,12 +858,9 @@ static int launch_sym_t(Plan *p, const double2 *in, double2 *out, int batch, con
     const int rb = pick_rb(groups, batch, std::max(1, blocks_per_sm) * sms, NR);
     const int chunks = multi ? multi->nchunks : (batch + rb - 1) / rb;
     dim3 grid((unsigned)groups, (unsigned)chunks);
-    k_line_solve_sym<SRC, NT, CW, MINB, NR, KS, TIO, MT><<<grid, NT, shm, p->ctx->stream>>>(
+    return launch_kernel(p->ctx, k_line_solve_sym<SRC, NT, CW, MINB, NR, KS, TIO, MT>, grid, NT, (size_t)shm,
         in, out, p->lines, p->rows, p->row_stride, p->field, batch, rb, p->Pv, p->subt, p->diagt, p->prow, p->mu, sp,
         in_map, p->ctx->err_word, multi ? multi->refs : nullptr, multi ? multi->chunks : nullptr);
-    HH_CUDA(cudaGetLastError());
-    p->ctx->launches++;
-    return HH_OK;
 }
 
 // The two builds of the kernel (hh_line_sym_real.cu, hh_line_sym_cplx.cu).

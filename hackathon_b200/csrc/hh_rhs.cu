@@ -104,6 +104,8 @@ __global__ void __launch_bounds__(kPadeThreads) k_pade(const __grid_constant__ P
     const int      t = threadIdx.x, W = J.w;
     const unsigned bx = blk % J.gx, by = blk / J.gx % J.gy, bz = blk / J.gx / J.gy;
     const double2  zero = make_double2(0.0, 0.0);
+    pdl_wait();
+    pdl_next();
     if (!J.xdir) {
         // 32 neighbouring columns, kSpanS points: tile [point][column]
         const int x0 = (int)bx * 32, m0 = (int)by * kSpanS, c2 = (int)bz;
@@ -212,6 +214,8 @@ struct Rhs2DArgs {
 // the points next to an edge, rhs.c:126-148 (the ring's corners belong to the edges y = const)
 __global__ void __launch_bounds__(256) k_rhs2d_combine(const __grid_constant__ Rhs2DArgs A) {
     const int i = blockIdx.x * 32 + (threadIdx.x & 31), j = blockIdx.y * 8 + (threadIdx.x >> 5);
+    pdl_wait();
+    pdl_next();
     if (i >= A.nx || j >= A.ny) return;
     const int  nx = A.nx, ny = A.ny;
     const long E = nx + 2, c = (i + 1) + (long)(j + 1) * E, q = i + (long)j * nx;
@@ -277,6 +281,8 @@ struct Rhs3DArgs {
 // and z faces and fzz on the x and y faces are zero, as the reference leaves them.
 __global__ void __launch_bounds__(256) k_rhs3d_combine(const __grid_constant__ Rhs3DArgs A) {
     const int i = blockIdx.x * 32 + (threadIdx.x & 31), j = blockIdx.y * 8 + (threadIdx.x >> 5), l = blockIdx.z;
+    pdl_wait();
+    pdl_next();
     if (i >= A.nx || j >= A.ny) return;
     const int     nx = A.nx, ny = A.ny, nz = A.nz;
     const long    Ex = nx + 2, Ey = ny + 2, Exy = Ex * Ey, nxy = (long)nx * ny;
@@ -449,10 +455,7 @@ static int launch_pade(Ctx *c, const PadeJobs &jobs) {
         return HH_ERR_UNSUPPORTED;
     }
     HH_CUDA(cudaFuncSetAttribute(k_pade, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-    k_pade<<<(unsigned)blocks, kPadeThreads, shm, c->stream>>>(jobs);
-    HH_CUDA(cudaGetLastError());
-    c->launches++;
-    return HH_OK;
+    return launch_kernel(c, k_pade, dim3((unsigned)blocks), kPadeThreads, shm, jobs);
 }
 
 int assemble_rhs2d(Plan *p, const hh_rhs2d_data *d, double2 *rhs) {
@@ -515,10 +518,7 @@ int assemble_rhs2d(Plan *p, const hh_rhs2d_data *d, double2 *rhs) {
     A.rhs = rhs;
     A.nx = nx, A.ny = ny, A.order = order, A.prow = p->prow;
     dim3 grid((unsigned)((nx + 31) / 32), (unsigned)((ny + 7) / 8));
-    k_rhs2d_combine<<<grid, 256, 0, c->stream>>>(A);
-    HH_CUDA(cudaGetLastError());
-    c->launches++;
-    return HH_OK;
+    return launch_kernel(c, k_rhs2d_combine, grid, 256, 0, A);
 }
 
 int assemble_rhs3d(Plan *p, const hh_rhs3d_data *d, double2 *rhs) {
@@ -586,10 +586,7 @@ int assemble_rhs3d(Plan *p, const hh_rhs3d_data *d, double2 *rhs) {
         return HH_ERR_UNSUPPORTED;
     }
     dim3 grid((unsigned)((nx + 31) / 32), (unsigned)((ny + 7) / 8), (unsigned)nz);
-    k_rhs3d_combine<<<grid, 256, 0, c->stream>>>(A);
-    HH_CUDA(cudaGetLastError());
-    c->launches++;
-    return HH_OK;
+    return launch_kernel(c, k_rhs3d_combine, grid, 256, 0, A);
 }
 
 } // namespace hh

@@ -338,6 +338,8 @@ __global__ void __launch_bounds__(NT, MINB)
         }
         cp_async_commit();
     };
+    pdl_wait();
+    pdl_next();
     prefetch(b_begin);
     int par = 0;
     for (int b = b_begin; b < b_end; b++) {
@@ -502,12 +504,9 @@ static int launch_solve_t(Plan *p, const double2 *in, double2 *out, int batch) {
     while (rb < batch && groups * ((batch + 2 * rb - 1) / (2 * rb)) >= 2L * MINB * 148) rb *= 2;
     const int chunks = (batch + rb - 1) / rb;
     dim3 grid((unsigned)groups, (unsigned)chunks);
-    k_line_solve<SRC, CR, NT, MINB><<<grid, NT, shm, p->ctx->stream>>>(in, out, p->lines, p->rows, p->prow,
+    return launch_kernel(p->ctx, k_line_solve<SRC, CR, NT, MINB>, grid, NT, (size_t)shm, in, out, p->lines, p->rows, p->prow,
                                                                        p->row_stride, p->field, batch, rb, CW, p->Pv,
                                                                        p->subt, p->diagt, p->rowc, p->mu, sp);
-    HH_CUDA(cudaGetLastError());
-    p->ctx->launches++;
-    return HH_OK;
 }
 
 template <bool CR, int NT, int MINB>
@@ -639,6 +638,7 @@ int launch_line_solve_multi(Plan *const *plans, const int *nrhs, int nplans, con
     HH_CUDA(cudaMemcpyAsync(tab, refs.data(), sizeof(SymPlanRef) * refs.size(), cudaMemcpyHostToDevice, p0->ctx->stream));
     HH_CUDA(cudaMemcpyAsync(tab + sizeof(SymPlanRef) * refs.size(), chunks.data(), sizeof(SymChunk) * chunks.size(),
                             cudaMemcpyHostToDevice, p0->ctx->stream));
+    p0->ctx->fresh = true; // the kernel's set-up reads the table
     SymMulti m;
     m.refs = reinterpret_cast<const SymPlanRef *>(tab);
     m.chunks = reinterpret_cast<const SymChunk *>(tab + sizeof(SymPlanRef) * refs.size());
