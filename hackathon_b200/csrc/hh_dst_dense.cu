@@ -236,7 +236,8 @@ __global__ void __launch_bounds__(kDenseThreads)
 //    at 2 against 196 at 1, two CTAs per SM with 3: 179), then 2 with two CTAs (n = 700: 228 us, 241 at
 //    1), then 1 (n = 1000: 655 us, 771 at 2).  Columns take the width (up to 5) that
 //    leaves the fewest idle columns in a plane's last tile (100 columns: 48 us at 5, 52 at 4).
-//  * fewer lines per CTA where the launch would leave SMs without one.
+//  * fewer lines per CTA where the launch would not give every SM two (7688 rows of n = 31: 4.8 us at 24
+//    lines, 6.4 at 48; 2500 rows of n = 50: 3.6 us at 8, 4.5 at 16).
 void dense_shape(bool cols, int n, long nlines, long planes, int *ntw, int *groups) {
     const int units = out_tiles(n);
     int       g = units >= kMmaWarps ? 1 : std::min(4, kMmaWarps / units), w = 0;
@@ -246,8 +247,9 @@ void dense_shape(bool cols, int n, long nlines, long planes, int *ntw, int *grou
         if (per_sm(v) >= 3 && (w == 0 || (cols && padded(v) < padded(w)))) w = v;
     if (w == 0) w = per_sm(2) >= 2 ? 2 : 1;
     auto ctas = [&]() { return padded(w) / (4L * w * g) * planes; };
+    while (w > 2 && ctas() < 296) w--;
+    while (g > 1 && ctas() < 296) g--;
     while (w > 1 && ctas() < 148) w--;
-    while (g > 1 && ctas() < 148) g--;
     *ntw = w;
     *groups = g;
 }

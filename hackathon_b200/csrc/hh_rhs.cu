@@ -483,7 +483,7 @@ int assemble_rhs2d(Plan *p, const hh_rhs2d_data *d, double2 *rhs) {
         const size_t o_k2c = ta.add(k2c.data(), 16 * k2c.size()), o_k2y = ta.add(k2y.data(), 16 * k2y.size());
         char        *tab;
         HH_TRY(upload_tables(c, ta, &tab));
-        double2 *w;
+        double2 *w = nullptr;
         HH_TRY(rhs_work(c, 3 * nxy, &w));
         double2 *fxx = w, *fyy = w + nxy, *fy = w + 2 * nxy;
         PadeJobs jobs;
@@ -543,7 +543,7 @@ int assemble_rhs3d(Plan *p, const hh_rhs3d_data *d, double2 *rhs) {
         const size_t o_kp = ta.add(kp.data(), 16 * kp.size()), o_k2 = ta.add(k2, 16 * (size_t)(nz + 2));
         char        *tab;
         HH_TRY(upload_tables(c, ta, &tab));
-        double2 *w;
+        double2 *w = nullptr;
         HH_TRY(rhs_work(c, 3 * n3, &w));
         double2 *fxx = w, *fyy = w + n3, *fzz = w + 2 * n3;
         PadeJobs jobs;
