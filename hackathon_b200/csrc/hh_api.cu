@@ -409,6 +409,12 @@ static int plan_factor(hh_plan *pl, const std::vector<double2> &sub, const std::
         const double2 a = sub[(size_t)k * p.rows], b = sup[(size_t)k * p.rows];
         p.sym = a.x == b.x && a.y == b.y;
     }
+    auto all_real = [](const std::vector<double2> &t) {
+        for (const double2 &v : t)
+            if (v.y != 0.0) return false;
+        return true;
+    };
+    p.real_rows = all_real(sub) && all_real(dia) && all_real(sup);
     p.real_coef = p.sym; // k2 (the source operator's k^2) is real then as well: k^2 h^2 is in every diagonal
     for (int k = 0; k < 4 && p.real_coef; k++)
         p.real_coef = sub[(size_t)k * p.rows].y == 0.0 && dia[(size_t)k * p.rows].y == 0.0;

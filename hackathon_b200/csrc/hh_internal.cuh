@@ -169,6 +169,7 @@ struct Plan {
                                  // (n + 1 = 2048): 0, 1 two warps per line, 2 the Stockham kernel
     bool     sym = false;        // const_rows and sub == super on every line (constant k)
     bool     real_coef = false;  // sym, and every coefficient of the lines real (k^2 real)
+    bool     real_rows = false;  // every per-row coefficient real
     bool     pf_ok = false;      // order-6 partial fractions well conditioned on every line
     double2 *subt = nullptr, *diagt = nullptr; // sub/diagonal row tables (4 * rows each)
     // super-diagonal(row, line) = rowc[0][row] mu[0][line] + rowc[1][row] mu[1][line] + rowc[2][row] mu[2][line] + rowc[3][row]

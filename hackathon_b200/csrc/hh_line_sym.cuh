@@ -30,44 +30,6 @@ namespace hh {
 //    checks |10 s - d| against |d|, |s| on every line before it selects this path.
 // =====================================================================================
 
-// a + b c and a - b c with two fused multiply-adds per component
-__device__ __forceinline__ double2 zfma(double2 a, double2 b, double2 c) {
-    return make_double2(fma(b.x, c.x, fma(-b.y, c.y, a.x)), fma(b.x, c.y, fma(b.y, c.x, a.y)));
-}
-__device__ __forceinline__ double2 zfms(double2 a, double2 b, double2 c) {
-    return make_double2(fma(-b.x, c.x, fma(b.y, c.y, a.x)), fma(-b.x, c.y, fma(-b.y, c.x, a.y)));
-}
-__device__ __forceinline__ double2 zaxpy(double2 a, double b, double2 c) { // a + b c, b real
-    return make_double2(fma(b, c.x, a.x), fma(b, c.y, a.y));
-}
-
-// The line coefficients are complex (MT = double2) or, where k^2 is real, real (MT = double).  On
-// real coefficients the real form does the arithmetic of the complex one without its exact zeros:
-// every finite result has the same bits, with half the fused multiply-adds, half the latency of
-// each recurrence step and half the registers and shared memory of the multipliers (tile input, line
-// solve, complex -> real: 2D 1023^2 x 64 order 6 678 -> 597 us, order 4 528 -> 507 us; 2047^2 x 16 order 6
-// 845 -> 726 us; 3D 255^3 x 4 order 6 709 -> 552 us).
-__device__ __forceinline__ double2 zfma(double2 a, double b, double2 c) { return zaxpy(a, b, c); }
-__device__ __forceinline__ double2 zfms(double2 a, double b, double2 c) { return zaxpy(a, -b, c); }
-__device__ __forceinline__ double2 cmul(double a, double2 b) { return make_double2(a * b.x, a * b.y); }
-__device__ __forceinline__ double  cmul(double a, double b) { return a * b; }
-__device__ __forceinline__ double2 mneg(double2 a) { return make_double2(-a.x, -a.y); }
-__device__ __forceinline__ double  mneg(double a) { return -a; }
-// crcp, factor_step and first_pivot on a zero imaginary part (the products rounded on their own, as there)
-__device__ __forceinline__ double crcp(double x) { return x * (1.0 / __dmul_rn(x, x)); }
-__device__ __forceinline__ double first_pivot(double dia) { return crcp(dia); }
-__device__ __forceinline__ double factor_step(double sub, double dia, double sup_prev, double ui_prev, double &L) {
-    L = sub * ui_prev;
-    return crcp(dia - __dmul_rn(L, sup_prev));
-}
-template <typename MT> __device__ __forceinline__ MT coef_of(double2 v) {
-    if constexpr (std::is_same_v<MT, double>) return v.x;
-    else return v;
-}
-__device__ __forceinline__ double coef_re(double v) { return v; }
-__device__ __forceinline__ double coef_re(double2 v) { return v.x; }
-template <typename MT> constexpr bool is_real_v = std::is_same_v<MT, double>;
-
 template <int NT> __host__ __device__ constexpr int ilog2_t() { return NT <= 1 ? 0 : 1 + ilog2_t<NT / 2>(); }
 
 template <int NW, int CW, int NR, typename MT> struct SymSmem {

@@ -226,10 +226,10 @@ __device__ __forceinline__ double pade_u(const ScanSmem<NW> &sm, const SrcParams
 
 // SRC = 0: the input already is the transformed RHS.  SRC = 2/4/6: the input is the transformed
 // source g and the compact operator of that order is applied first (see the file header).
-// CONST_ROWS: the stencil rows do not vary along the line (constant k).
+// The stencil rows do not vary along the line (constant k); k_line_solve_rows below takes those that do.
 // Rows past the end of a line are neutral: zero data, zero reciprocal pivots, zero Pade factors,
 // so the sweeps run without per-row conditions.
-template <int SRC, bool CONST_ROWS, int NT, int MINB>
+template <int SRC, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
     k_line_solve(const double2 *__restrict__ in, double2 *__restrict__ out, int lines, int rows, int prow,
                  long row_stride, long field, int batch, int rb, int CW, const double2 *__restrict__ Pv,
@@ -256,39 +256,27 @@ __global__ void __launch_bounds__(NT, MINB)
     const double2 one = make_double2(1.0, 0.0), zero = make_double2(0.0, 0.0);
 
     // ---- factors of this thread's rows, kept in registers for the whole chunk
-    double2 sub_c = zero, sup_c = zero;
-    if constexpr (CONST_ROWS) {
-        sub_c = shifted(subt, prow, 0, m0, m1, m2);
-        sup_c = shifted(supt, prow, 0, m0, m1, m2);
-    }
+    const double2 sub_c = shifted(subt, prow, 0, m0, m1, m2), sup_c = shifted(supt, prow, 0, m0, m1, m2);
     const double2 ui_in = (live && r0 > 0 && r0 < rows) ? Pv[(long)L.s * lines + q] : zero; // 1/P of row r0-1
     double2 ui[kSeg];
     double2 Af = one, Ab = one;
     {
         double2 uprev = ui_in;
-        const double2 dia_c = CONST_ROWS ? shifted(diagt, prow, 0, m0, m1, m2) : zero;
+        const double2 dia_c = shifted(diagt, prow, 0, m0, m1, m2);
 #pragma unroll
         for (int u = 0; u < kSeg; u++) {
             const int r = r0 + u;
             double2   Lr = zero;
             ui[u] = zero;
             if (live && r < rows) {
-                const double2 dia = CONST_ROWS ? dia_c : shifted(diagt, prow, r, m0, m1, m2);
-                if (r == 0) {
-                    ui[u] = first_pivot(dia);
-                } else {
-                    const double2 sb = CONST_ROWS ? sub_c : shifted(subt, prow, r, m0, m1, m2);
-                    const double2 sp_ = CONST_ROWS ? sup_c : shifted(supt, prow, r - 1, m0, m1, m2);
-                    ui[u] = factor_step(sb, dia, sp_, uprev, Lr);
-                }
+                if (r == 0) ui[u] = first_pivot(dia_c);
+                else ui[u] = factor_step(sub_c, dia_c, sup_c, uprev, Lr);
             } else if (live && r > 0 && u > 0) {
-                const double2 sb = CONST_ROWS ? sub_c : shifted(subt, prow, r, m0, m1, m2);
-                Lr = cmul(sb, uprev); // first padded row: L is still formed from the last real pivot
+                Lr = cmul(sub_c, uprev); // first padded row: L is still formed from the last real pivot
             }
             uprev = ui[u];
             Af = cmul(Af, make_double2(-Lr.x, -Lr.y));
-            const double2 sp2 = CONST_ROWS ? sup_c : shifted(supt, prow, r, m0, m1, m2);
-            const double2 tau = cmul(sp2, ui[u]);
+            const double2 tau = cmul(sup_c, ui[u]);
             Ab = cmul(Ab, make_double2(-tau.x, -tau.y));
         }
     }
@@ -418,15 +406,13 @@ __global__ void __launch_bounds__(NT, MINB)
         double2 yh = zero;
 #pragma unroll
         for (int u = 0; u < kSeg; u++) {
-            const double2 sb = CONST_ROWS ? sub_c : shifted(subt, prow, r0 + u, m0, m1, m2);
-            yh = cfms(v[u], cmul(sb, u == 0 ? ui_in : ui[u - 1]), yh);
+            yh = cfms(v[u], cmul(sub_c, u == 0 ? ui_in : ui[u - 1]), yh);
         }
         double2 y = scan_forward(Af, yh, L, sm, par);
         par ^= 1;
 #pragma unroll
         for (int u = 0; u < kSeg; u++) {
-            const double2 sb = CONST_ROWS ? sub_c : shifted(subt, prow, r0 + u, m0, m1, m2);
-            y = cfms(v[u], cmul(sb, u == 0 ? ui_in : ui[u - 1]), y);
+            y = cfms(v[u], cmul(sub_c, u == 0 ? ui_in : ui[u - 1]), y);
             v[u] = y;
         }
 
@@ -434,18 +420,133 @@ __global__ void __launch_bounds__(NT, MINB)
         double2 xh = zero;
 #pragma unroll
         for (int u = kSeg - 1; u >= 0; u--) {
-            const double2 sp2 = CONST_ROWS ? sup_c : shifted(supt, prow, r0 + u, m0, m1, m2);
-            xh = cmul(cfms(v[u], sp2, xh), ui[u]);
+            xh = cmul(cfms(v[u], sup_c, xh), ui[u]);
         }
         double2 x = scan_backward(Ab, xh, L, sm, par);
         par ^= 1;
 #pragma unroll
         for (int u = kSeg - 1; u >= 0; u--) {
-            const double2 sp2 = CONST_ROWS ? sup_c : shifted(supt, prow, r0 + u, m0, m1, m2);
-            x = cmul(cfms(v[u], sp2, x), ui[u]);
+            x = cmul(cfms(v[u], sup_c, x), ui[u]);
             v[u] = x;
         }
 
+        double2 *dst = out + (long)b * field + off0;
+#pragma unroll
+        for (int u = 0; u < kSeg; u++)
+            if (live && r0 + u < rows) dst[(long)u * row_stride] = v[u];
+    }
+}
+
+// Per-row coefficients (variable k), assembled right-hand sides.  The same segments and scans, with the
+// thread's multipliers kept: forming them from the four per-row tables at each use (two sweeps each
+// way) read 4 complex values a row and sweep through L1 and bounded the solve.  MT = double: every table is
+// real (real k), so the multipliers are, and the products lose their zero halves.
+//   y_r = f_r - L_r y_{r-1},  x_r = (1/P_r) y_r - tau_r x_{r+1},  tau_r = super_r / P_r
+// (3D 125^3, real k: 60 -> 40 us; 2D 511^2, complex k: 16.4 -> 11.8 us.)
+template <typename MT> __device__ __forceinline__ MT row_coef(const double2 *__restrict__ tab, int rows, int r, double m0,
+                                                              double m1, double m2) {
+    if constexpr (is_real_v<MT>) {
+        const double *t = reinterpret_cast<const double *>(tab);
+        return ((__ldg(t + 2 * r) * m0 + __ldg(t + 2 * (rows + r)) * m1) + __ldg(t + 2 * (2 * rows + r)) * m2) +
+               __ldg(t + 2 * (3 * rows + r));
+    } else {
+        return shifted(tab, rows, r, m0, m1, m2);
+    }
+}
+
+template <int NT, int MINB, typename MT>
+__global__ void __launch_bounds__(NT, MINB)
+    k_line_solve_rows(const double2 *__restrict__ in, double2 *__restrict__ out, int lines, int rows, int prow,
+                      long row_stride, long field, int batch, int rb, int CW, const double2 *__restrict__ Pv,
+                      const double2 *__restrict__ subt, const double2 *__restrict__ diagt,
+                      const double2 *__restrict__ supt, const double *__restrict__ mu) {
+    constexpr int NW = NT / 32;
+    __shared__ ScanSmem<NW> sm;
+    extern __shared__ double2 pre[]; // [kSeg][NT] prefetch of the next right-hand side
+    Lane L;
+    L.lane = threadIdx.x & 31;
+    L.w = threadIdx.x >> 5;
+    L.CW = CW;
+    L.SPW = 32 / CW;
+    L.c = threadIdx.x % CW;
+    L.s = threadIdx.x / CW;
+    L.sl = L.lane / CW;
+    const int  q = blockIdx.x * CW + L.c;
+    const bool live = q < lines;
+    const int  qq = live ? q : 0;
+    const int  r0 = L.s * kSeg;
+    const double m0 = live ? mu[q] : 0.0, m1 = live ? mu[lines + q] : 0.0, m2 = live ? mu[2 * lines + q] : 0.0;
+    const double2 zero = make_double2(0.0, 0.0);
+
+    // ---- factors of this thread's rows, kept for the whole chunk.  Rows past the end of a line are neutral
+    // (zero data, zero reciprocal pivots), so the sweeps run without per-row conditions.
+    MT Lr[kSeg], ui[kSeg], tau[kSeg];
+    MT Af = coef_of<MT>(make_double2(1.0, 0.0)), Ab = Af;
+    {
+        MT uprev = (live && r0 > 0 && r0 < rows) ? coef_of<MT>(Pv[(long)L.s * lines + q]) : MT{}; // 1/P of row r0-1
+        MT sp = r0 > 0 && r0 <= prow ? row_coef<MT>(supt, prow, r0 - 1, m0, m1, m2) : MT{};
+#pragma unroll
+        for (int u = 0; u < kSeg; u++) {
+            const int r = r0 + u;
+            Lr[u] = MT{};
+            ui[u] = MT{};
+            tau[u] = MT{};
+            if (live && r < rows) {
+                const MT dia = row_coef<MT>(diagt, prow, r, m0, m1, m2);
+                if (r == 0) ui[u] = first_pivot(dia);
+                else ui[u] = factor_step(row_coef<MT>(subt, prow, r, m0, m1, m2), dia, sp, uprev, Lr[u]);
+                sp = row_coef<MT>(supt, prow, r, m0, m1, m2);
+                tau[u] = cmul(sp, ui[u]);
+            }
+            uprev = ui[u];
+            Af = cmul(Af, mneg(Lr[u]));
+            Ab = cmul(Ab, mneg(tau[u]));
+        }
+    }
+    const double2 Afc = coef_full(Af), Abc = coef_full(Ab); // (the scans compose complex maps)
+
+    const int  b_begin = blockIdx.y * rb;
+    const int  b_end = min(batch, b_begin + rb);
+    const long off0 = (long)r0 * row_stride + qq;
+    auto prefetch = [&](int b) {
+        const double2 *src = in + (long)b * field + off0;
+#pragma unroll
+        for (int u = 0; u < kSeg; u++) {
+            const bool ok = live && r0 + u < rows;
+            cp_async16(&pre[u * NT + threadIdx.x], ok ? src + (long)u * row_stride : in, ok ? 16 : 0);
+        }
+        cp_async_commit();
+    };
+    pdl_wait();
+    pdl_next();
+    prefetch(b_begin);
+    int par = 0;
+    for (int b = b_begin; b < b_end; b++) {
+        double2 v[kSeg];
+        cp_async_wait_all();
+#pragma unroll
+        for (int u = 0; u < kSeg; u++) v[u] = pre[u * NT + threadIdx.x];
+        if (b + 1 < b_end) prefetch(b + 1);
+        double2 yh = zero;
+#pragma unroll
+        for (int u = 0; u < kSeg; u++) yh = zfms(v[u], Lr[u], yh);
+        double2 y = scan_forward(Afc, yh, L, sm, par);
+        par ^= 1;
+#pragma unroll
+        for (int u = 0; u < kSeg; u++) {
+            y = zfms(v[u], Lr[u], y);
+            v[u] = cmul(ui[u], y);
+        }
+        double2 xh = zero;
+#pragma unroll
+        for (int u = kSeg - 1; u >= 0; u--) xh = zfms(v[u], tau[u], xh);
+        double2 x = scan_backward(Abc, xh, L, sm, par);
+        par ^= 1;
+#pragma unroll
+        for (int u = kSeg - 1; u >= 0; u--) {
+            x = zfms(v[u], tau[u], x);
+            v[u] = x;
+        }
         double2 *dst = out + (long)b * field + off0;
 #pragma unroll
         for (int u = 0; u < kSeg; u++)
@@ -484,7 +585,27 @@ int padded_rows(int rows) {
 
 int solve_variant_count() { return kNumVariants + 5; }
 
-template <int SRC, bool CR, int NT, int MINB>
+// the chunk of right-hand sides per CTA: enough CTAs to fill the SMs twice, factors reused within a chunk
+static int rows_chunk(long groups, int batch, int minb) {
+    int rb = 1;
+    while (rb < batch && groups * ((batch + 2 * rb - 1) / (2 * rb)) >= 2L * minb * 148) rb *= 2;
+    return rb;
+}
+
+template <int NT, int MINB, typename MT>
+static int launch_solve_rows(Plan *p, const double2 *in, double2 *out, int batch) {
+    int CW, P;
+    HH_TRY(solve_geometry(p->rows, NT, &CW, &P));
+    const int shm = (int)(sizeof(double2) * kSeg * NT);
+    HH_CUDA(cudaFuncSetAttribute(k_line_solve_rows<NT, MINB, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
+    const long groups = (p->lines + CW - 1) / CW;
+    const int  rb = rows_chunk(groups, batch, MINB);
+    dim3 grid((unsigned)groups, (unsigned)((batch + rb - 1) / rb));
+    return launch_kernel(p->ctx, k_line_solve_rows<NT, MINB, MT>, grid, NT, (size_t)shm, in, out, p->lines, p->rows, p->prow,
+                         p->row_stride, p->field, batch, rb, CW, p->Pv, p->subt, p->diagt, p->rowc, p->mu);
+}
+
+template <int SRC, int NT, int MINB>
 static int launch_solve_t(Plan *p, const double2 *in, double2 *out, int batch) {
     int CW, P;
     HH_TRY(solve_geometry(p->rows, NT, &CW, &P));
@@ -497,32 +618,42 @@ static int launch_solve_t(Plan *p, const double2 *in, double2 *out, int batch) {
     sp.linf = p->pade_linf;
     sp.uinf = p->pade_uinf;
     const int shm = (int)(sizeof(double2) * kSeg * NT) * (SRC == 6 ? 2 : 1);
-    HH_CUDA(cudaFuncSetAttribute(k_line_solve<SRC, CR, NT, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
-    // right-hand sides per CTA: enough CTAs to fill the SMs twice, factors reused within a chunk
+    HH_CUDA(cudaFuncSetAttribute(k_line_solve<SRC, NT, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
     const long groups = (p->lines + CW - 1) / CW;
-    int rb = 1;
-    while (rb < batch && groups * ((batch + 2 * rb - 1) / (2 * rb)) >= 2L * MINB * 148) rb *= 2;
+    const int  rb = rows_chunk(groups, batch, MINB);
     const int chunks = (batch + rb - 1) / rb;
     dim3 grid((unsigned)groups, (unsigned)chunks);
-    return launch_kernel(p->ctx, k_line_solve<SRC, CR, NT, MINB>, grid, NT, (size_t)shm, in, out, p->lines, p->rows, p->prow,
+    return launch_kernel(p->ctx, k_line_solve<SRC, NT, MINB>, grid, NT, (size_t)shm, in, out, p->lines, p->rows, p->prow,
                                                                        p->row_stride, p->field, batch, rb, CW, p->Pv,
                                                                        p->subt, p->diagt, p->rowc, p->mu, sp);
 }
 
-template <bool CR, int NT, int MINB>
+template <int NT, int MINB>
 static int launch_solve_v(Plan *p, const double2 *in, double2 *out, int batch, int src) {
     switch (src) {
-    case 0: return launch_solve_t<0, CR, NT, MINB>(p, in, out, batch);
-    case 2: return launch_solve_t<2, CR, NT, MINB>(p, in, out, batch);
-    case 4: return launch_solve_t<4, CR, NT, MINB>(p, in, out, batch);
-    case 6: return launch_solve_t<6, CR, NT, MINB>(p, in, out, batch);
+    case 0: return launch_solve_t<0, NT, MINB>(p, in, out, batch);
+    case 2: return launch_solve_t<2, NT, MINB>(p, in, out, batch);
+    case 4: return launch_solve_t<4, NT, MINB>(p, in, out, batch);
+    case 6: return launch_solve_t<6, NT, MINB>(p, in, out, batch);
     default: set_error("source operator order %d", src); return HH_ERR_INVALID;
     }
 }
 
-template <bool CR> static int launch_solve_cr(Plan *p, const double2 *in, double2 *out, int batch, int src) {
-    if (p->variant == 1) return launch_solve_v<CR, 256, 2>(p, in, out, batch, src);
-    return launch_solve_v<CR, 512, 1>(p, in, out, batch, src);
+static int launch_solve_const(Plan *p, const double2 *in, double2 *out, int batch, int src) {
+    if (p->variant == 1) return launch_solve_v<256, 2>(p, in, out, batch, src);
+    return launch_solve_v<512, 1>(p, in, out, batch, src);
+}
+
+// Per-row coefficients: variant 1 takes 256 threads; variant 0 512 with real coefficients, and 256 where 512
+// would leave SMs without a line group or where complex ones would not fit 128 registers.  Lines past 2048
+// rows only fit 512.
+static int launch_solve_rows_any(Plan *p, const double2 *in, double2 *out, int batch) {
+    int CW, P;
+    HH_TRY(solve_geometry(p->rows, 512, &CW, &P));
+    const bool small = p->rows <= 256 * kSeg && (p->variant == 1 || !p->real_rows || (p->lines + CW - 1) / CW < 148);
+    if (p->real_rows)
+        return small ? launch_solve_rows<256, 2, double>(p, in, out, batch) : launch_solve_rows<512, 1, double>(p, in, out, batch);
+    return small ? launch_solve_rows<256, 1, double2>(p, in, out, batch) : launch_solve_rows<512, 1, double2>(p, in, out, batch);
 }
 
 int launch_line_solve_sym(Plan *p, const double2 *in, double2 *out, int batch, int src_order);
@@ -534,8 +665,12 @@ int launch_line_solve(Plan *p, const double2 *in, double2 *out, int batch, int s
         set_error("order-6 source operator needs a Helmholtz plan");
         return HH_ERR_INVALID;
     }
-    return p->const_rows ? launch_solve_cr<true>(p, in, out, batch, src_order)
-                         : launch_solve_cr<false>(p, in, out, batch, src_order);
+    if (p->const_rows) return launch_solve_const(p, in, out, batch, src_order);
+    if (src_order != 0) {
+        set_error("the source operator needs a Helmholtz plan");
+        return HH_ERR_INVALID;
+    }
+    return launch_solve_rows_any(p, in, out, batch);
 }
 
 int segment_count(int rows) { return (rows + kSeg - 1) / kSeg; }

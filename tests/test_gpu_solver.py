@@ -406,3 +406,26 @@ def test_real_and_complex_line_coefficients(ctx, oracle, dim, n, order, k):
         assert np.array_equal(both[0].cpu().numpy(), u)
     plan.close()
     other.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(5, 1), (9, 2), (100, 8), (63, 9), (300, 100), (200, 255), (31, 511), (7, 2047), (5, 2049)])
+@pytest.mark.parametrize("imag", [0.0, 1.0])
+def test_per_row_coefficients(ctx, oracle, nx, ny, imag):
+    """Plans with coefficients that vary along the line, real and complex, over line lengths around the 8-row
+    segments and the block sizes (256 and 512 threads), and batches: against the reference's Thomas solve
+    of the same right-hand sides in the oracle."""
+    rng = np.random.default_rng(nx + ny)
+
+    def row(scale, off):
+        return np.ascontiguousarray(off + scale * (rng.random(ny) + 1j * imag * rng.random(ny)), dtype=np.complex128)
+
+    coef = dict(bp=row(0.05, 0.15), ap=row(0.1, 0.6), b=row(0.1, 0.6), a=row(0.5, -4.5), bm=row(0.05, 0.15), am=row(0.1, 0.6))
+    plan = hh.Plan.from_coefficients_2d(ctx, nx, ny, coef)
+    rhs = rng.standard_normal((3, ny, nx)) + 1j * rng.standard_normal((3, ny, nx))
+    L, U, Up = oracle.lu_2d(nx, ny, coef)
+    want = np.stack([oracle.solver_2d(r, L, U, Up) for r in rhs])
+    for v in (0, 1) if ny <= 2048 else (0,):
+        plan.variant = v
+        assert rel_err(plan.solve_host(rhs), want) < TOL
+        assert rel_err(plan.solve_host(rhs[1]), want[1]) < TOL
+    plan.close()
