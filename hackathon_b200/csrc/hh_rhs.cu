@@ -36,6 +36,7 @@ namespace hh {
 namespace {
 
 constexpr int kPadeThreads = 256, kSegP = 8;
+constexpr int kReach10 = 17, kReach4 = 30; // points before r^w is below rounding: 1.2e-17 (d = 10), 7e-18 (d = 4)
 constexpr int kSpanS = 64;           // outputs of a block along a strided axis: 8 segments x 32 columns
 constexpr int kSpanX = 128, kRowsX = 16; // along x: 16 segments x 16 rows
 
@@ -46,10 +47,10 @@ constexpr int kSpanX = 128, kRowsX = 16; // along x: 16 segments x 16 rows
 struct PadeJob {
     const double2 *f, *bc;
     double2       *out;
-    int            n, n1, n2, w, first, xdir;
+    int            n, n1, n2, w, xdir;
     long           f0, f1, f2, fa, o1, o2, oa, b0, b2, bface;
-    double         scale, scale_lo; // 12 / h^2 (or 3 / h) as a sum of two doubles
-    double         r, inv;          // the decay of F and B, 1 / sqrt(d^2 - 4)
+    double         scale, scale_lo; // 12 / h^2 (or 3 / h) over sqrt(d^2 - 4), as a sum of two doubles
+    double         r, bscale;       // the decay of F and B; h^2 / 12 (or h / 3)
     unsigned       blocks, gx, gy;  // the job's blocks: gx by gy by (rest)
 };
 struct PadeJobs {
@@ -61,132 +62,174 @@ __device__ __forceinline__ double2 zaxpy_r(double2 a, double b, double2 c) { // 
     return make_double2(fma(b, c.x, a.x), fma(b, c.y, a.y));
 }
 
-// v_m of a line, extended by odd reflection
-__device__ __forceinline__ double2 pade_rhs(const PadeJob &J, int c1, int c2, int m) {
-    double sgn = 1.0;
-    if (m < 0 || m >= J.n) {
+__device__ __forceinline__ void pade_async16(double2 *dst, const double2 *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+                 "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void pade_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// The difference of f that point m takes, f_{m+1} - f_{m-1} (FIRST) or f_{m-1} - 2 f_m + f_{m+1}; p at m's
+// extended position, `step` values between neighbours
+template <bool FIRST> __device__ __forceinline__ double2 pade_diff(double2 lo, double2 mid, double2 hi) {
+    if (FIRST) return make_double2(hi.x - lo.x, hi.y - lo.y);
+    return make_double2(fma(-2.0, mid.x, lo.x + hi.x), fma(-2.0, mid.y, lo.y + hi.y));
+}
+
+// v_m of line (c1, c2) over 12 / h^2 (or 3 / h): odd reflection outside the line, the boundary value off the end
+// points' v; F(e) is f at extended position e of the line (interior point m at m + 1)
+template <int W, bool FIRST, typename Src>
+__device__ __forceinline__ double2 pade_rhs(const PadeJob &J, int c1, int c2, int m, Src F) {
+    bool neg = false;
+    if (J.n > W) { // one reflection reaches the line (v = 0 at -1 and n)
+        neg = (unsigned)m >= (unsigned)J.n;
+        m = m < 0 ? -2 - m : (m >= J.n ? 2 * J.n - m : m);
+        if ((unsigned)m >= (unsigned)J.n) return make_double2(0.0, 0.0);
+    } else {
         const int per = 2 * (J.n + 1);
         int       q = (m + 1) % per;
         if (q < 0) q += per;
         if (q == 0 || q == J.n + 1) return make_double2(0.0, 0.0);
-        if (q > J.n + 1) {
-            q = per - q;
-            sgn = -1.0;
-        }
-        m = q - 1;
+        neg = q > J.n + 1;
+        m = (neg ? per - q : q) - 1;
     }
-    const double2 *e = J.f + J.f0 + c1 * J.f1 + c2 * J.f2 + (long)m * J.fa;
-    const double2  lo = __ldg(e - J.fa), hi = __ldg(e + J.fa);
-    double2        v;
-    if (J.first) {
-        v = make_double2(hi.x - lo.x, hi.y - lo.y);
-    } else {
-        const double2 c = __ldg(e);
-        v = make_double2(lo.x - 2.0 * c.x + hi.x, lo.y - 2.0 * c.y + hi.y);
-    }
-    v = make_double2(fma(v.x, J.scale, v.x * J.scale_lo), fma(v.y, J.scale, v.y * J.scale_lo));
+    double2 v = pade_diff<FIRST>(F(m), F(m + 1), F(m + 2));
     if (J.bc && (m == 0 || m == J.n - 1)) {
         const double2 b = J.bc[J.b0 + c1 + c2 * J.b2 + (m == 0 ? 0 : J.bface)];
-        v = make_double2(v.x - b.x, v.y - b.y);
+        v = make_double2(fma(-J.bscale, b.x, v.x), fma(-J.bscale, b.y, v.y));
     }
-    return make_double2(sgn * v.x, sgn * v.y);
+    return neg ? make_double2(-v.x, -v.y) : v;
 }
 
-// Bound by shared memory and by the loads of f (each value read three times, from L1 and L2): the
-// segment of 8 points costs 2 (W + 8) steps of one fused multiply-add per component.  All derivatives of an
-// assembly share one launch (2D 511^2, with the combination: 2.31 ms -> 30 us; 3D 125^3: 0.73 -> 0.14 ms).
-__global__ void __launch_bounds__(kPadeThreads) k_pade(const __grid_constant__ PadeJobs jobs) {
+// The two sweeps of one segment of `top` <= 8 points; V(m) is v at the segment's point m, W points reached on
+// either side, put(m, value) takes the results.
+template <int W, typename Val, typename Put>
+__device__ __forceinline__ void pade_segment(Val V, int top, const PadeJob &J, Put put) {
+    const double r = J.r;
+    double2 B = make_double2(0.0, 0.0), F = B, Bn[kSegP];
+#pragma unroll
+    for (int m = kSegP + W - 1; m >= 0; m--) {
+        if (m < kSegP) Bn[m] = B;
+        if (m < top + W) B = zaxpy_r(V(m), -r, B);
+    }
+#pragma unroll
+    for (int m = -W; m < 0; m++) F = zaxpy_r(V(m), -r, F);
+#pragma unroll
+    for (int m = 0; m < kSegP; m++) {
+        if (m < top) {
+            const double2 vm = V(m);
+            const double2 u = zaxpy_r(vm, -r, make_double2(F.x + Bn[m].x, F.y + Bn[m].y));
+            put(m, make_double2(fma(u.x, J.scale, u.x * J.scale_lo), fma(u.y, J.scale, u.y * J.scale_lo)));
+            F = zaxpy_r(vm, -r, F);
+        }
+    }
+}
+
+// One block: the values of f that its span reaches come in with asynchronous copies, v is formed from them
+// and takes their place, then every thread sweeps one segment.
+template <int W> __device__ __forceinline__ void pade_block(const PadeJob &J, unsigned blk, double2 *sm) {
+    const int      t = threadIdx.x;
+    const unsigned bx = blk % J.gx, by = blk / J.gx % J.gy, bz = blk / J.gx / J.gy;
+    const double2  zero = make_double2(0.0, 0.0);
+    constexpr bool FIRST = W == kReach4;
+    if (!J.xdir) {
+        // 32 neighbouring columns, kSpanS points: tiles [point][column]
+        const int x0 = (int)bx * 32, m0 = (int)by * kSpanS, c2 = (int)bz, cc = t & 31, c = x0 + cc;
+        const int span = min(kSpanS, J.n - m0), len = span + 2 * W;
+        const int e0 = max(0, m0 - W), e1 = min(J.n + 1, m0 + span + W + 1); // extended positions needed
+        const bool in = c < J.n1;
+        {
+            const double2 *f = J.f + J.f0 - J.fa + (in ? c : 0) * J.f1 + c2 * J.f2;
+            for (int e = e0 + (t >> 5); e <= e1; e += kPadeThreads / 32)
+                pade_async16(sm + (e - e0) * 32 + cc, f + (long)e * J.fa);
+        }
+        pade_async_wait();
+        __syncthreads();
+        constexpr int NV = (kSpanS + 2 * W + 7) / 8;
+        double2       vv[NV];
+#pragma unroll
+        for (int i = 0; i < NV; i++) {
+            const int r = (t >> 5) + 8 * i;
+            vv[i] = zero;
+            if (in && r < len)
+                vv[i] = pade_rhs<W, FIRST>(J, c, c2, m0 - W + r, [&](int e) { return sm[(e - e0) * 32 + cc]; });
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < NV; i++) {
+            const int r = (t >> 5) + 8 * i;
+            if (r < len) sm[r * 32 + cc] = vv[i];
+        }
+        __syncthreads();
+        const int i0 = (t >> 5) * kSegP; // the thread's first point within the span
+        if (i0 >= span || !in) return;
+        const double2 *v = sm + (i0 + W) * 32 + cc;
+        double2       *o = J.out + c + c2 * J.o2 + (long)(m0 + i0) * J.oa;
+        pade_segment<W>([&](int m) { return v[m * 32]; }, min(kSegP, span - i0), J,
+                        [&](int m, double2 u) { o[m * J.oa] = u; });
+    } else {
+        // kRowsX neighbouring rows, kSpanX points: tiles [row][point + point / 8] (the segments of 8 start on
+        // different banks)
+        constexpr int pitch = (kSpanX + 2 * W + 2) * 9 / 8 + 1;
+        const int     m0 = (int)bx * kSpanX, span = min(kSpanX, J.n - m0), len = span + 2 * W;
+        const int     e0 = max(0, m0 - W), e1 = min(J.n + 1, m0 + span + W + 1);
+        const long    row0 = (long)by * kRowsX, rows = (long)J.n1 * J.n2;
+        const int     nr = (int)min((long)kRowsX, rows - row0);
+        // thread (r, k): row r, positions k + 16 i
+        const int  r = t >> 4, k = t & 15;
+        const bool in = r < nr;
+        const int  c1 = in ? (int)((row0 + r) % J.n1) : 0, c2 = in ? (int)((row0 + r) / J.n1) : 0;
+        double2   *row = sm + r * pitch;
+        auto       at = [](int e) { return e + (e >> 3); };
+        if (in) {
+            const double2 *f = J.f + J.f0 - J.fa + c1 * J.f1 + c2 * J.f2;
+            for (int e = e0 + k; e <= e1; e += 16) pade_async16(row + at(e - e0), f + e);
+        }
+        pade_async_wait();
+        __syncthreads();
+        constexpr int NV = (kSpanX + 2 * W + 15) / 16;
+        double2       vv[NV];
+#pragma unroll
+        for (int i = 0; i < NV; i++) {
+            const int e = k + 16 * i;
+            vv[i] = zero;
+            if (in && e < len)
+                vv[i] = pade_rhs<W, FIRST>(J, c1, c2, m0 - W + e, [&](int y) { return row[at(y - e0)]; });
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < NV; i++) {
+            const int e = k + 16 * i;
+            if (e < len) row[at(e)] = vv[i];
+        }
+        __syncthreads();
+        const int i0 = k * kSegP, top = in ? max(0, min(kSegP, span - i0)) : 0;
+        double2   u[kSegP];
+        if (top > 0)
+            pade_segment<W>([&](int m) { return row[at(i0 + W + m)]; }, top, J, [&](int m, double2 x) { u[m] = x; });
+        __syncthreads(); // the tile takes the results, for contiguous stores
+#pragma unroll
+        for (int m = 0; m < kSegP; m++)
+            if (m < top) row[at(i0 + m)] = u[m];
+        __syncthreads();
+        if (in) {
+            double2 *o = J.out + c1 * J.o1 + c2 * J.o2 + m0;
+            for (int e = k; e < span; e += 16) o[e] = row[at(e)];
+        }
+    }
+}
+
+// Bound by instruction issue and shared memory: a point costs 1.5 to 2 values of v and a segment of 8 points
+// 2 (W + 8) steps of one fused multiply-add per component.  All derivatives of an assembly share one launch.
+__global__ void __launch_bounds__(kPadeThreads, 3) k_pade(const __grid_constant__ PadeJobs jobs) {
     extern __shared__ __align__(16) double2 pade_sm[];
     unsigned blk = blockIdx.x;
     int      ji = 0;
     while (ji + 1 < jobs.count && blk >= jobs.j[ji].blocks) blk -= jobs.j[ji++].blocks;
-    const PadeJob &J = jobs.j[ji];
-    const int      t = threadIdx.x, W = J.w;
-    const unsigned bx = blk % J.gx, by = blk / J.gx % J.gy, bz = blk / J.gx / J.gy;
-    const double2  zero = make_double2(0.0, 0.0);
     pdl_wait();
     pdl_next();
-    if (!J.xdir) {
-        // 32 neighbouring columns, kSpanS points: tile [point][column]
-        const int x0 = (int)bx * 32, m0 = (int)by * kSpanS, c2 = (int)bz;
-        const int len = min(kSpanS, J.n - m0) + 2 * W;
-        for (int e = t; e < len * 32; e += kPadeThreads) {
-            const int c = x0 + (e & 31);
-            pade_sm[e] = c < J.n1 ? pade_rhs(J, c, c2, m0 - W + (e >> 5)) : zero;
-        }
-        __syncthreads();
-        const int c = t & 31, i0 = (t >> 5) * kSegP; // the thread's first point within the span
-        if (m0 + i0 >= J.n || x0 + c >= J.n1) return;
-        const double2 *v = pade_sm + (i0 + W) * 32 + c;
-        const int      top = min(kSegP, J.n - m0 - i0); // points of this segment
-        double2        B = zero, Bn[kSegP], F = zero;
-        for (int m = top + W - 1; m >= kSegP; m--) B = zaxpy_r(v[m * 32], -J.r, B);
-#pragma unroll
-        for (int m = kSegP - 1; m >= 0; m--) {
-            Bn[m] = B;
-            if (m < top + W) B = zaxpy_r(v[m * 32], -J.r, B);
-        }
-        for (int m = -W; m < 0; m++) F = zaxpy_r(v[m * 32], -J.r, F);
-        double2 *o = J.out + (x0 + c) + c2 * J.o2 + (long)(m0 + i0) * J.oa;
-#pragma unroll
-        for (int m = 0; m < kSegP; m++) {
-            if (m < top) {
-                const double2 vm = v[m * 32];
-                const double2 u = zaxpy_r(vm, -J.r, make_double2(F.x + Bn[m].x, F.y + Bn[m].y));
-                o[m * J.oa] = make_double2(u.x * J.inv, u.y * J.inv);
-                F = zaxpy_r(vm, -J.r, F);
-            }
-        }
-    } else {
-        // kRowsX neighbouring rows, kSpanX points: tile [row][point + point / 8] (the segments of 8 start on
-        // different banks)
-        const int  m0 = (int)bx * kSpanX, len = min(kSpanX, J.n - m0) + 2 * W;
-        const int  pitch = (kSpanX + 2 * W) * 9 / 8 + 1;
-        const long row0 = (long)by * kRowsX, rows = (long)J.n1 * J.n2;
-        const int  nr = (int)min((long)kRowsX, rows - row0);
-        for (int r = t >> 5; r < nr; r += kPadeThreads / 32) {
-            const int c1 = (int)((row0 + r) % J.n1), c2 = (int)((row0 + r) / J.n1);
-            for (int e = t & 31; e < len; e += 32) pade_sm[r * pitch + e + (e >> 3)] = pade_rhs(J, c1, c2, m0 - W + e);
-        }
-        __syncthreads();
-        const int  r = t >> 4, i0 = (t & 15) * kSegP;
-        const bool live = r < nr && m0 + i0 < J.n;
-        const int  top = live ? min(kSegP, J.n - m0 - i0) : 0;
-        double2    u[kSegP];
-        if (live) {
-            double2 *row = pade_sm + r * pitch;
-            auto     V = [&](int m) { const int e = i0 + W + m; return row[e + (e >> 3)]; };
-            double2  B = zero, Bn[kSegP], F = zero;
-            for (int m = top + W - 1; m >= kSegP; m--) B = zaxpy_r(V(m), -J.r, B);
-#pragma unroll
-            for (int m = kSegP - 1; m >= 0; m--) {
-                Bn[m] = B;
-                if (m < top + W) B = zaxpy_r(V(m), -J.r, B);
-            }
-            for (int m = -W; m < 0; m++) F = zaxpy_r(V(m), -J.r, F);
-#pragma unroll
-            for (int m = 0; m < kSegP; m++) {
-                if (m < top) {
-                    const double2 vm = V(m);
-                    u[m] = zaxpy_r(vm, -J.r, make_double2(F.x + Bn[m].x, F.y + Bn[m].y));
-                    F = zaxpy_r(vm, -J.r, F);
-                }
-            }
-        }
-        __syncthreads(); // the tile takes the results, for contiguous stores
-#pragma unroll
-        for (int m = 0; m < kSegP; m++)
-            if (m < top) {
-                const int e = i0 + m;
-                pade_sm[r * pitch + e + (e >> 3)] = make_double2(u[m].x * J.inv, u[m].y * J.inv);
-            }
-        __syncthreads();
-        for (int q = t >> 5; q < nr; q += kPadeThreads / 32) {
-            const int c1 = (int)((row0 + q) % J.n1), c2 = (int)((row0 + q) / J.n1);
-            double2  *o = J.out + c1 * J.o1 + c2 * J.o2 + m0;
-            for (int e = t & 31; e < len - 2 * W; e += 32) o[e] = pade_sm[q * pitch + e + (e >> 3)];
-        }
-    }
+    if (jobs.j[ji].w == kReach10) pade_block<kReach10>(jobs.j[ji], blk, pade_sm);
+    else pade_block<kReach4>(jobs.j[ji], blk, pade_sm);
 }
 
 __device__ __forceinline__ double2 zmul(double2 a, double2 b) { return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
@@ -279,61 +322,90 @@ struct Rhs3DArgs {
 // rhs.c:24-29, 55-62, 167-174: layer 0 with the sub-diagonal layer's stencil (am, bm, cm, dm of layer
 // 0), layer nz-1 with the super-diagonal one (ap..dp of nz-1).  fxx on the y and z faces, fyy on the x
 // and z faces and fzz on the x and y faces are zero, as the reference leaves them.
+//
+// A thread marches through kZRun layers of its (i, j) with the layers below, at and above in registers, the
+// one after those on its way: each field crosses L2 once instead of three times.
+constexpr int kZRun = 16;
 __global__ void __launch_bounds__(256) k_rhs3d_combine(const __grid_constant__ Rhs3DArgs A) {
-    const int i = blockIdx.x * 32 + (threadIdx.x & 31), j = blockIdx.y * 8 + (threadIdx.x >> 5), l = blockIdx.z;
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31), j = blockIdx.y * 8 + (threadIdx.x >> 5);
     pdl_wait();
     pdl_next();
     if (i >= A.nx || j >= A.ny) return;
-    const int     nx = A.nx, ny = A.ny, nz = A.nz;
+    const int     nx = A.nx, ny = A.ny, nz = A.nz, l0 = blockIdx.z * kZRun, l1 = min(nz, l0 + kZRun);
     const long    Ex = nx + 2, Ey = ny + 2, Exy = Ex * Ey, nxy = (long)nx * ny;
-    const long    C = (i + 1) + (j + 1) * Ex + (l + 1) * Exy, q = i + (long)j * nx + l * nxy;
     const double2 zero = make_double2(0.0, 0.0);
-    double2       r;
-    if (A.order == 6) {
-        auto face = [&](const double2 *b, long at) { return b ? b[at] : zero; };
-        const double2 xx = A.fxx[q], yy = A.fyy[q], zz = A.fzz[q];
-        const double2 xw = i > 0 ? A.fxx[q - 1] : face(A.fxx_b, (j + 1) + (l + 1) * Ey);
-        const double2 xe = i + 1 < nx ? A.fxx[q + 1] : face(A.fxx_b, (j + 1) + (l + 1) * Ey + Ey * (nz + 2));
-        const double2 xs = j > 0 ? A.fxx[q - nx] : zero, xn = j + 1 < ny ? A.fxx[q + nx] : zero;
-        const double2 xd = l > 0 ? A.fxx[q - nxy] : zero, xu = l + 1 < nz ? A.fxx[q + nxy] : zero;
-        const double2 ys = j > 0 ? A.fyy[q - nx] : face(A.fyy_b, (i + 1) + (l + 1) * Ex);
-        const double2 yn = j + 1 < ny ? A.fyy[q + nx] : face(A.fyy_b, (i + 1) + (l + 1) * Ex + Ex * (nz + 2));
-        const double2 yd = l > 0 ? A.fyy[q - nxy] : zero, yu = l + 1 < nz ? A.fyy[q + nxy] : zero;
-        const double2 zd = l > 0 ? A.fzz[q - nxy] : face(A.fzz_b, (i + 1) + (j + 1) * Ex);
-        const double2 zu = l + 1 < nz ? A.fzz[q + nxy] : face(A.fzz_b, (i + 1) + (j + 1) * Ex + Exy);
-        const double2 k2 = A.k2_ext[l + 1];
-        const double2 first = zmul(make_double2(1.0 - k2.x * A.h2_20, -(k2.y * A.h2_20)), A.f[C]);
-        const double2 second = rmul(A.c_f, zadd(zadd(xx, yy), zz));
-        const double2 third = zadd(zadd(rmul(A.c_xxxx, d2(xw, xx, xe)), rmul(A.c_yyyy, d2(ys, yy, yn))),
-                                   rmul(A.c_zzzz, d2(zd, zz, zu)));
-        const double2 fourth = zadd(zadd(rmul(A.c_xxyy, d2(xs, xx, xn)), rmul(A.c_xxzz, d2(xd, xx, xu))),
-                                    rmul(A.c_yyzz, d2(yd, yy, yu)));
-        const double2 fifth = zmul(rmul(A.c_z, A.kp[l]), zsub(A.f[C + Exy], A.f[C - Exy]));
-        r = zadd(zadd(zadd(zadd(first, second), third), fourth), fifth);
-    } else if (A.order == 4) {
-        const double2 nb = zadd(zadd(zadd(zadd(zadd(A.f[C - 1], A.f[C + 1]), A.f[C - Ex]), A.f[C + Ex]), A.f[C - Exy]), A.f[C + Exy]);
-        r = zadd(A.f[C], rmul(1.0 / 12.0, zsub(nb, rmul(6.0, A.f[C]))));
-    } else {
-        r = A.f[C];
+    const bool    six = A.order == 6;
+    const long    Cij = (i + 1) + (j + 1) * Ex, qij = i + (long)j * nx;
+    auto face = [&](const double2 *b, long at) { return b ? b[at] : zero; };
+    // the centre values of layer l (f at -1 .. nz, the derivatives zero outside, fzz its face values)
+    auto F = [&](int l) { return A.f[Cij + (l + 1) * Exy]; };
+    auto D = [&](const double2 *d, int l) { return l >= 0 && l < nz ? d[qij + l * nxy] : zero; };
+    auto Z = [&](int l) {
+        if (l < 0) return face(A.fzz_b, Cij);
+        return l < nz ? A.fzz[qij + l * nxy] : face(A.fzz_b, Cij + Exy);
+    };
+    double2 fd = zero, f0 = zero, fu = zero, xd = zero, xx = zero, xu = zero, yd = zero, yy = zero, yu = zero, zd = zero,
+            zz = zero, zu = zero;
+    if (six) {
+        fd = F(l0 - 1), f0 = F(l0), fu = F(l0 + 1);
+        xd = D(A.fxx, l0 - 1), xx = D(A.fxx, l0), xu = D(A.fxx, l0 + 1);
+        yd = D(A.fyy, l0 - 1), yy = D(A.fyy, l0), yu = D(A.fyy, l0 + 1);
+        zd = Z(l0 - 1), zz = Z(l0), zu = Z(l0 + 1);
     }
-    if (A.ue) {
-        for (int far = 0; far < 2; far++) {
-            if (l != (far ? nz - 1 : 0)) continue;
-            const double2 *e = A.ue + (far ? (nz + 1) * Exy : 0);
-            auto           X = [&](int ie, int je) { return e[ie + je * Ex]; };
-            if (A.order == 2) {
-                r = zsub(r, X(i + 1, j + 1));
-                continue;
+    for (int l = l0; l < l1; l++) {
+        const long C = Cij + (l + 1) * Exy, q = qij + l * nxy;
+        double2    r;
+        if (six) {
+            double2 fn = zero, xn2 = zero, yn2 = zero, zn2 = zero; // layer l + 2, on its way
+            if (l + 1 < l1) {
+                fn = F(l + 2);
+                xn2 = D(A.fxx, l + 2);
+                yn2 = D(A.fyy, l + 2);
+                zn2 = Z(l + 2);
             }
-            const double2 *tab = far ? A.supt : A.subt;
-            const double2  a = tab[l], bb = tab[A.prow + l], cc = tab[2 * A.prow + l], dd = tab[3 * A.prow + l];
-            r = zsub(r, zmul(a, zadd(zadd(zadd(X(i, j), X(i + 2, j)), X(i, j + 2)), X(i + 2, j + 2))));
-            r = zsub(r, zmul(bb, zadd(X(i, j + 1), X(i + 2, j + 1))));
-            r = zsub(r, zmul(cc, zadd(X(i + 1, j), X(i + 1, j + 2))));
-            r = zsub(r, zmul(dd, X(i + 1, j + 1)));
+            const double2 xw = i > 0 ? A.fxx[q - 1] : face(A.fxx_b, (j + 1) + (l + 1) * Ey);
+            const double2 xe = i + 1 < nx ? A.fxx[q + 1] : face(A.fxx_b, (j + 1) + (l + 1) * Ey + Ey * (nz + 2));
+            const double2 xs = j > 0 ? A.fxx[q - nx] : zero, xn = j + 1 < ny ? A.fxx[q + nx] : zero;
+            const double2 ys = j > 0 ? A.fyy[q - nx] : face(A.fyy_b, (i + 1) + (l + 1) * Ex);
+            const double2 yn = j + 1 < ny ? A.fyy[q + nx] : face(A.fyy_b, (i + 1) + (l + 1) * Ex + Ex * (nz + 2));
+            const double2 k2 = A.k2_ext[l + 1];
+            const double2 first = zmul(make_double2(1.0 - k2.x * A.h2_20, -(k2.y * A.h2_20)), f0);
+            const double2 second = rmul(A.c_f, zadd(zadd(xx, yy), zz));
+            const double2 third = zadd(zadd(rmul(A.c_xxxx, d2(xw, xx, xe)), rmul(A.c_yyyy, d2(ys, yy, yn))),
+                                       rmul(A.c_zzzz, d2(zd, zz, zu)));
+            const double2 fourth = zadd(zadd(rmul(A.c_xxyy, d2(xs, xx, xn)), rmul(A.c_xxzz, d2(xd, xx, xu))),
+                                        rmul(A.c_yyzz, d2(yd, yy, yu)));
+            const double2 fifth = zmul(rmul(A.c_z, A.kp[l]), zsub(fu, fd));
+            r = zadd(zadd(zadd(zadd(first, second), third), fourth), fifth);
+            fd = f0, f0 = fu, fu = fn;
+            xd = xx, xx = xu, xu = xn2;
+            yd = yy, yy = yu, yu = yn2;
+            zd = zz, zz = zu, zu = zn2;
+        } else if (A.order == 4) {
+            const double2 nb = zadd(zadd(zadd(zadd(zadd(A.f[C - 1], A.f[C + 1]), A.f[C - Ex]), A.f[C + Ex]), A.f[C - Exy]), A.f[C + Exy]);
+            r = zadd(A.f[C], rmul(1.0 / 12.0, zsub(nb, rmul(6.0, A.f[C]))));
+        } else {
+            r = A.f[C];
         }
+        if (A.ue) {
+            for (int far = 0; far < 2; far++) {
+                if (l != (far ? nz - 1 : 0)) continue;
+                const double2 *e = A.ue + (far ? (nz + 1) * Exy : 0);
+                auto           X = [&](int ie, int je) { return e[ie + je * Ex]; };
+                if (A.order == 2) {
+                    r = zsub(r, X(i + 1, j + 1));
+                    continue;
+                }
+                const double2 *tab = far ? A.supt : A.subt;
+                const double2  a = tab[l], bb = tab[A.prow + l], cc = tab[2 * A.prow + l], dd = tab[3 * A.prow + l];
+                r = zsub(r, zmul(a, zadd(zadd(zadd(X(i, j), X(i + 2, j)), X(i, j + 2)), X(i + 2, j + 2))));
+                r = zsub(r, zmul(bb, zadd(X(i, j + 1), X(i + 2, j + 1))));
+                r = zsub(r, zmul(cc, zadd(X(i + 1, j), X(i + 1, j + 2))));
+                r = zsub(r, zmul(dd, X(i + 1, j + 1)));
+            }
+        }
+        A.rhs[q] = r;
     }
-    A.rhs[q] = r;
 }
 
 // Pade factors of tridiag(1, diag, 1) over n points, as the reference forms them
@@ -420,15 +492,14 @@ static PadeJob pade_job(const double2 *f, double2 *out, const double *bc, int n,
     J.n = n;
     J.n1 = n1;
     J.n2 = n2;
-    J.first = diag == 4;
     J.xdir = xdir;
-    J.w = diag == 4 ? 30 : 17; // r^w: 7e-18, 1.2e-17
+    J.w = diag == 4 ? kReach4 : kReach10;
     const long double hl = h, sc = diag == 4 ? 3.0L / hl : 12.0L / (hl * hl);
-    J.scale = (double)sc;
-    J.scale_lo = (double)(sc - (long double)J.scale);
+    J.bscale = (double)(1.0L / sc);
     const long double root = sqrtl((long double)diag * diag - 4.0L);
     J.r = (double)(2.0L / (diag + root));
-    J.inv = (double)(1.0L / root);
+    J.scale = (double)(sc / root);
+    J.scale_lo = (double)(sc / root - (long double)J.scale);
     if (xdir) {
         J.gx = (unsigned)((n + kSpanX - 1) / kSpanX);
         J.gy = (unsigned)(((long)n1 * n2 + kRowsX - 1) / kRowsX);
@@ -447,8 +518,8 @@ static int launch_pade(Ctx *c, const PadeJobs &jobs) {
     for (int i = 0; i < jobs.count; i++) {
         const PadeJob &J = jobs.j[i];
         blocks += J.blocks;
-        shm = std::max(shm, sizeof(double2) * (J.xdir ? (size_t)kRowsX * ((kSpanX + 2 * J.w) * 9 / 8 + 1)
-                                                      : (size_t)(kSpanS + 2 * J.w) * 32));
+        shm = std::max(shm, sizeof(double2) * (J.xdir ? (size_t)kRowsX * ((kSpanX + 2 * J.w + 2) * 9 / 8 + 1)
+                                                      : (size_t)(kSpanS + 2 * J.w + 2) * 32));
     }
     if (blocks > 0x7fffffffL) {
         set_error("right-hand side: grid too large");
@@ -585,7 +656,7 @@ int assemble_rhs3d(Plan *p, const hh_rhs3d_data *d, double2 *rhs) {
         set_error("hh_rhs3d: %d x %d x %d is too large", nx, ny, nz);
         return HH_ERR_UNSUPPORTED;
     }
-    dim3 grid((unsigned)((nx + 31) / 32), (unsigned)((ny + 7) / 8), (unsigned)nz);
+    dim3 grid((unsigned)((nx + 31) / 32), (unsigned)((ny + 7) / 8), (unsigned)((nz + kZRun - 1) / kZRun));
     return launch_kernel(c, k_rhs3d_combine, grid, 256, 0, A);
 }
 
