@@ -144,12 +144,13 @@ extern "C" int hh_ctx_destroy(hh_ctx *x) {
     cudaStreamSynchronize(x->c.stream);
     drain_events(x->c);
     // plans still alive belong to this context: release them with it
-    for (Plan *p : x->c.plans) {
+    std::vector<Plan *> plans;
+    plans.swap(x->c.plans); // (plan_free takes a plan out of the context's list)
+    for (Plan *p : plans) {
         hh_plan *pl = reinterpret_cast<hh_plan *>(p); // Plan is the first member of hh_plan
         plan_free(pl);
         delete pl;
     }
-    x->c.plans.clear();
     for (auto &kv : x->c.tw) cudaFree(kv.second);
     for (auto &kv : x->c.sn) cudaFree(kv.second);
     for (auto &kv : x->c.dense) cudaFree(kv.second);

@@ -429,3 +429,12 @@ def test_per_row_coefficients(ctx, oracle, nx, ny, imag):
         assert rel_err(plan.solve_host(rhs), want) < TOL
         assert rel_err(plan.solve_host(rhs[1]), want[1]) < TOL
     plan.close()
+
+
+def test_context_destroyed_with_several_live_plans():
+    """The context releases the plans still alive on it, each once."""
+    for count in (1, 2, 3, 8):
+        c = hh.Context(0)
+        plans = [hh.Plan.helmholtz(c, 2, 31 + i, 4, 5.0) for i in range(count)]
+        c.close()
+        assert all(p.h is None for p in plans)
