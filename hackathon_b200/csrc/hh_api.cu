@@ -5,7 +5,7 @@
 //   3D  rhs --DST-I x (rows), y (columns)--> F^ --line solves along z--> U^ --DST-I y, x--> u
 // which is the reference's solver() (2D_Program/solver_functions/solver.c:66-90,
 // 3D_Program/solver_functions/solver.c:465-515).  Every stage works in place on the output
-// buffer, so the solve needs no scratch beyond the output itself.
+// buffer, or, for large fields with odd rows, in a padded workspace (see acquire_work).
 #include "hh_internal.cuh"
 
 #include <algorithm>
@@ -137,6 +137,7 @@ extern "C" int hh_ctx_create(int device, void *stream, hh_ctx **out) {
 }
 
 static void plan_free(hh_plan *pl);
+static void work_pool_release(Ctx *c);
 
 extern "C" int hh_ctx_destroy(hh_ctx *x) {
     if (!x) return HH_OK;
@@ -161,6 +162,7 @@ extern "C" int hh_ctx_destroy(hh_ctx *x) {
     cudaFree(x->c.rhs_work);
     cudaFree(x->c.rhs_tab);
     cudaFree(x->stage);
+    work_pool_release(&x->c);
     for (cudaEvent_t e : x->c.chunk_ev) cudaEventDestroy(e);
     if (x->c.copy_in) cudaStreamDestroy(x->c.copy_in);
     if (x->c.copy_out) cudaStreamDestroy(x->c.copy_out);
@@ -619,8 +621,8 @@ extern "C" int hh_plan_set_variant(hh_plan *pl, int variant) {
 
 extern "C" int hh_plan_variant(const hh_plan *pl) { return pl ? pl->p.variant : -1; }
 
-static int transform_forward(Plan &p, const double2 *in, double2 *out, int batch, bool lp = false);
-static int transform_inverse(Plan &p, double2 *buf, int batch, bool lp = false);
+static int transform_forward(Plan &p, const double2 *in, double2 *out, int batch, bool lp = false, long ld = 0);
+static int transform_inverse(Plan &p, double2 *in, double2 *out, int batch, bool lp = false, long ld = 0);
 
 // Times every line-solve variant on `batch` zero right-hand sides (the solve does the same work
 // for any values) and keeps the fastest.  Blocks; must not run inside a stream capture.
@@ -669,7 +671,7 @@ static int tune_measure(hh_plan *pl, int batch) {
             p.rows_kernel = rk;
             auto pass = [&]() -> int {
                 HH_TRY(transform_forward(p, buf, buf, batch));
-                return transform_inverse(p, buf, batch);
+                return transform_inverse(p, buf, buf, batch);
             };
             if ((rc = pass()) != HH_OK) break;
             if (cudaEventRecord(e0, c->stream) != cudaSuccess) { rc = HH_ERR_CUDA; break; }
@@ -706,7 +708,7 @@ static int tune_measure(hh_plan *pl, int batch) {
             p.col_kernel = trial % 2;
             auto pass = [&]() -> int {
                 HH_TRY(transform_forward(p, buf, buf, batch));
-                return transform_inverse(p, buf, batch);
+                return transform_inverse(p, buf, buf, batch);
             };
             if ((rc = pass()) != HH_OK) break;
             if (cudaEventRecord(e0, c->stream) != cudaSuccess) { rc = HH_ERR_CUDA; break; }
@@ -887,31 +889,126 @@ long hh::slab_planes(const Plan &p, long planes) {
     return std::max(1L, std::min(std::min(s, planes), 65535L));
 }
 
-// lp: single-precision transform arithmetic (the refined solve's low-precision solves)
-static int transform_forward(Plan &p, const double2 *in, double2 *out, int batch, bool lp) {
+// lp: single-precision transform arithmetic (the refined solve's low-precision solves).  `ld`: the row pitch of the
+// transformed field (its rows nx long, its layers ld ny apart); the field in physical space is contiguous.
+static int transform_forward(Plan &p, const double2 *in, double2 *out, int batch, bool lp, long ld) {
     Ctx *c = p.ctx;
-    if (p.dim == 2) return launch_dst_rows(c, p.nx, (long)p.ny * batch, in, p.nx, out, p.nx, lp, p.rows_kernel);
-    const long plane = (long)p.nx * p.ny, planes = (long)p.nz * batch, sp = slab_planes(p, planes);
+    if (ld == 0) ld = p.nx;
+    if (p.dim == 2) return launch_dst_rows(c, p.nx, (long)p.ny * batch, in, p.nx, out, ld, lp, p.rows_kernel);
+    const long plane = (long)p.nx * p.ny, lplane = ld * p.ny, planes = (long)p.nz * batch, sp = slab_planes(p, planes);
     for (long p0 = 0; p0 < planes; p0 += sp) {
         const long np = std::min(sp, planes - p0);
-        HH_TRY(launch_dst_rows(c, p.nx, (long)p.ny * np, in + p0 * plane, p.nx, out + p0 * plane, p.nx, lp,
-                               p.rows_kernel));
-        HH_TRY(launch_dst_cols(c, p.ny, p.nx, np, out + p0 * plane, p.nx, plane, out + p0 * plane, lp, p.col_kernel));
+        double2   *o = out + p0 * lplane;
+        HH_TRY(launch_dst_rows(c, p.nx, (long)p.ny * np, in + p0 * plane, p.nx, o, ld, lp, p.rows_kernel));
+        HH_TRY(launch_dst_cols(c, p.ny, p.nx, np, o, ld, lplane, o, lp, p.col_kernel));
     }
     return HH_OK;
 }
 
-static int transform_inverse(Plan &p, double2 *buf, int batch, bool lp) {
+// from the transformed field `in` (row pitch ld; the columns pass of a 3D field works in place on it) to `out`
+static int transform_inverse(Plan &p, double2 *in, double2 *out, int batch, bool lp, long ld) {
     Ctx *c = p.ctx;
-    if (p.dim == 2) return launch_dst_rows(c, p.nx, (long)p.ny * batch, buf, p.nx, buf, p.nx, lp, p.rows_kernel);
-    const long plane = (long)p.nx * p.ny, planes = (long)p.nz * batch, sp = slab_planes(p, planes);
+    if (ld == 0) ld = p.nx;
+    if (p.dim == 2) return launch_dst_rows(c, p.nx, (long)p.ny * batch, in, ld, out, p.nx, lp, p.rows_kernel);
+    const long plane = (long)p.nx * p.ny, lplane = ld * p.ny, planes = (long)p.nz * batch, sp = slab_planes(p, planes);
     for (long p0 = 0; p0 < planes; p0 += sp) {
         const long np = std::min(sp, planes - p0);
-        HH_TRY(launch_dst_cols(c, p.ny, p.nx, np, buf + p0 * plane, p.nx, plane, buf + p0 * plane, lp, p.col_kernel));
-        HH_TRY(launch_dst_rows(c, p.nx, (long)p.ny * np, buf + p0 * plane, p.nx, buf + p0 * plane, p.nx, lp,
-                               p.rows_kernel));
+        double2   *w = in + p0 * lplane;
+        HH_TRY(launch_dst_cols(c, p.ny, p.nx, np, w, ld, lplane, w, lp, p.col_kernel));
+        HH_TRY(launch_dst_rows(c, p.nx, (long)p.ny * np, w, ld, out + p0 * plane, p.nx, lp, p.rows_kernel));
     }
     return HH_OK;
+}
+
+// ---- padded workspace.  Where nx is odd (n = 2^k - 1, the common case) every other row of a field starts in the
+// middle of a 32-byte sector, so the 32- to 128-byte row pieces that the columns transform and the line
+// solve move end in partial sectors and straddle 128-byte lines.  A large solve therefore keeps its transformed
+// field in a workspace with rows of a multiple of 8 values: 3D 255^3 x 4, columns transform 526 -> 426 us, whole solve
+// 2.18 -> 1.99 ms; 2D 2047^2 x 16 1.63 -> 1.56 ms, 1023^2 x 64 1.29 -> 1.26 ms.  Fields that stay in L2 from pass to
+// pass gain nothing (1023^2 x 8: 193 us either way), so the line is at twice the L2.  The arithmetic, and so every
+// bit, is the same.
+//  * The workspace is allocated and freed in stream order from one pool per device, shared by the contexts on it
+//    and destroyed with the last of them, which keeps at most kWorkKeep bytes between solves; a solve that
+//    would need more, or cannot get it, runs in place in the output as smaller ones do.
+//  * In place as well: solves under stream capture (a graph's own allocations would restrict it), the request
+//    loop's (its budget does not know the workspace) and the host-buffer forms (bound by their copies).
+constexpr size_t kWorkKeep = 4ULL << 30;
+struct WorkPool {
+    cudaMemPool_t pool = nullptr;
+    int           users = 0;
+};
+static std::mutex              g_work_mu;
+static std::map<int, WorkPool> g_work;
+
+static cudaMemPool_t work_pool_of(Ctx *c) {
+    if (c->work_pool) return c->work_pool;
+    std::lock_guard<std::mutex> g(g_work_mu);
+    WorkPool &w = g_work[c->device];
+    if (!w.pool) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = c->device;
+        uint64_t keep = kWorkKeep;
+        int      off = 0; // solves on different streams never wait for each other's workspace
+        if (cudaMemPoolCreate(&w.pool, &props) != cudaSuccess ||
+            cudaMemPoolSetAttribute(w.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
+            cudaMemPoolSetAttribute(w.pool, cudaMemPoolReuseAllowInternalDependencies, &off) != cudaSuccess) {
+            cudaGetLastError();
+            if (w.pool) cudaMemPoolDestroy(w.pool);
+            w.pool = nullptr;
+            return nullptr;
+        }
+    }
+    w.users++;
+    return c->work_pool = w.pool;
+}
+
+static void work_pool_release(Ctx *c) {
+    if (!c->work_pool) return;
+    std::lock_guard<std::mutex> g(g_work_mu);
+    WorkPool &w = g_work[c->device];
+    if (--w.users == 0) {
+        cudaMemPoolDestroy(w.pool);
+        w.pool = nullptr;
+    }
+    c->work_pool = nullptr;
+}
+
+// The workspace of a solve of `batch` fields and its row pitch; *work stays null where the solve runs in place.
+static void acquire_work(Plan &p, int batch, int src_order, double2 **work, long *ld) {
+    Ctx *c = p.ctx;
+    *work = nullptr;
+    *ld = p.nx;
+    if (p.nx % 2 == 0 || c->pool) return;
+    if (p.dim == 3 && (p.variant < 2 || !sym_solve_supported(&p, src_order))) return; // needs the line positions
+    const long   pitch = (p.nx + 7) / 8 * 8;
+    const size_t bytes = sizeof(double2) * (size_t)pitch * (size_t)p.ny * (size_t)(p.dim == 3 ? p.nz : 1) * (size_t)batch;
+    if (bytes < 2 * c->l2_bytes || bytes > kWorkKeep) return;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    if (cap != cudaStreamCaptureStatusNone) return;
+    cudaMemPool_t pool = work_pool_of(c);
+    if (!pool) return;
+    void *w = nullptr;
+    if (cudaMallocFromPoolAsync(&w, bytes, pool, c->stream) != cudaSuccess) {
+        cudaGetLastError(); // no memory for it: in place
+        return;
+    }
+    *work = static_cast<double2 *>(w);
+    *ld = pitch;
+}
+
+// the plan over fields with rows of `ld` values
+static Plan padded_plan(const Plan &p, long ld) {
+    Plan q = p;
+    q.row_stride = p.dim == 2 ? ld : ld * p.ny;
+    q.field = q.row_stride * p.rows;
+    if (p.dim == 3) q.pitch = (int)ld;
+    return q;
 }
 
 extern "C" int hh_plan_set_slab(hh_plan *pl, long planes) {
@@ -996,20 +1093,51 @@ extern "C" int hh_solve_lines(hh_plan *pl, const double *in, double *out, int ba
     return hh_solve_lines_strided(pl, in, out, batch, fused, pl->p.row_stride, pl->p.field);
 }
 
-extern "C" int hh_solve(hh_plan *pl, const double *rhs, double *sol, int batch) {
+// One solve: forward transforms, the line solves given by `lines(plan, field)`, inverse transforms, in the output
+// buffer or (padded) in a workspace.
+template <typename Lines>
+static int solve_passes(Plan &p, const double2 *in, double2 *out, int batch, int src_order, bool may_pad, Lines lines) {
+    Ctx     *c = p.ctx;
+    double2 *work = nullptr;
+    long     ld = p.nx;
+    if (may_pad) acquire_work(p, batch, src_order, &work, &ld);
+    double2 *w = work ? work : out;
+    auto     passes = [&]() -> int {
+        HH_TRY(stage_mark(*c, 0));
+        HH_TRY(transform_forward(p, in, w, batch, false, ld));
+        HH_TRY(stage_mark(*c, 1));
+        HH_TRY(lines(w, ld));
+        HH_TRY(stage_mark(*c, 2));
+        HH_TRY(transform_inverse(p, w, out, batch, false, ld));
+        return stage_mark(*c, 3);
+    };
+    int rc = passes();
+    if (work) {
+        const cudaError_t e = cudaFreeAsync(work, c->stream);
+        if (rc == HH_OK && e != cudaSuccess) rc = cuda_fail(e, "cudaFreeAsync", __FILE__, __LINE__);
+    }
+    return rc;
+}
+
+static int solve_one(hh_plan *pl, const double *in, double *out, int batch, int src_order, bool may_pad) {
+    Plan &p = pl->p;
+    HH_CUDA(cudaSetDevice(p.ctx->device));
+    return solve_passes(p, (const double2 *)in, (double2 *)out, batch, src_order, may_pad, [&](double2 *w, long ld) -> int {
+        if (ld == p.nx) return launch_line_solve(&p, w, w, batch, src_order);
+        Plan q = padded_plan(p, ld);
+        return launch_line_solve(&q, w, w, batch, src_order);
+    });
+}
+
+static int solve_assembled(hh_plan *pl, const double *rhs, double *sol, int batch, bool may_pad) {
     HH_TRY(check_batch(pl, batch));
     if (batch == 0) return HH_OK;
     if (!rhs || !sol) { set_error("hh_solve: null buffer"); return HH_ERR_INVALID; }
-    Plan &p = pl->p;
-    HH_CUDA(cudaSetDevice(p.ctx->device));
-    double2 *u = (double2 *)sol;
-    HH_TRY(stage_mark(*p.ctx, 0));
-    HH_TRY(transform_forward(p, (const double2 *)rhs, u, batch));
-    HH_TRY(stage_mark(*p.ctx, 1));
-    HH_TRY(launch_line_solve(&p, u, u, batch, 0));
-    HH_TRY(stage_mark(*p.ctx, 2));
-    HH_TRY(transform_inverse(p, u, batch));
-    return stage_mark(*p.ctx, 3);
+    return solve_one(pl, rhs, sol, batch, 0, may_pad);
+}
+
+extern "C" int hh_solve(hh_plan *pl, const double *rhs, double *sol, int batch) {
+    return solve_assembled(pl, rhs, sol, batch, true);
 }
 
 // The residual maxima buffer of a context (two words, made on first use).
@@ -1077,7 +1205,7 @@ extern "C" int hh_solve_refined(hh_plan *pl, const double *rhs, double *sol, int
     auto low_solve = [&](const double2 *in, double2 *out) -> int {
         HH_TRY(transform_forward(p, in, out, batch, true));
         HH_TRY(launch_line_solve(&p, out, out, batch, 0));
-        return transform_inverse(p, out, batch, true);
+        return transform_inverse(p, out, out, batch, true);
     };
     // a correction u <- u - S(w): the last (rows) pass of the inverse transform subtracts its
     // result from u as it stores, where the rows kernel has that form; else a separate update
@@ -1119,24 +1247,19 @@ extern "C" int hh_solve_refined(hh_plan *pl, const double *rhs, double *sol, int
     return hh_ctx_synchronize(reinterpret_cast<hh_ctx *>(c)); // kernel-reported failures
 }
 
-extern "C" int hh_solve_source(hh_plan *pl, const double *f, double *u, int batch) {
+static int solve_source(hh_plan *pl, const double *f, double *u, int batch, bool may_pad) {
     HH_TRY(check_batch(pl, batch));
     if (batch == 0) return HH_OK;
     if (!f || !u) { set_error("hh_solve_source: null buffer"); return HH_ERR_INVALID; }
-    Plan &p = pl->p;
-    if (p.src_order == 0) {
+    if (pl->p.src_order == 0) {
         set_error("hh_solve_source needs a plan from hh_plan{2,3}d_create_helmholtz");
         return HH_ERR_INVALID;
     }
-    HH_CUDA(cudaSetDevice(p.ctx->device));
-    double2 *w = (double2 *)u;
-    HH_TRY(stage_mark(*p.ctx, 0));
-    HH_TRY(transform_forward(p, (const double2 *)f, w, batch));
-    HH_TRY(stage_mark(*p.ctx, 1));
-    HH_TRY(launch_line_solve(&p, w, w, batch, p.src_order));
-    HH_TRY(stage_mark(*p.ctx, 2));
-    HH_TRY(transform_inverse(p, w, batch));
-    return stage_mark(*p.ctx, 3);
+    return solve_one(pl, f, u, batch, pl->p.src_order, may_pad);
+}
+
+extern "C" int hh_solve_source(hh_plan *pl, const double *f, double *u, int batch) {
+    return solve_source(pl, f, u, batch, true);
 }
 
 // Several wavenumbers in one solve: plans of one shape (dim, sizes, fused order) on one context,
@@ -1152,34 +1275,44 @@ int hh::solve_source_multi(Plan *const *plans, const int *nrhs, int nplans, cons
     int   total = 0;
     for (int i = 0; i < nplans; i++) total += nrhs[i];
     if (total == 0) return HH_OK;
-    HH_TRY(stage_mark(*c, 0));
-    HH_TRY(transform_forward(p0, f, u, total));
-    HH_TRY(stage_mark(*c, 1));
-    if (!table) {
-        const size_t need = line_solve_multi_table_bytes(nplans, total);
-        if (c->multi_tab_bytes < need) {
-            HH_CUDA(cudaStreamSynchronize(c->stream));
-            cudaFree(c->multi_tab);
-            c->multi_tab = nullptr;
-            c->multi_tab_bytes = 0;
-            HH_CUDA(cudaMalloc(&c->multi_tab, need));
-            c->multi_tab_bytes = need;
+    const bool own_table = !table;
+    // the padded form needs the positions of lines, which every plan's line solve must know
+    bool may_pad = own_table;
+    for (int i = 0; i < nplans; i++)
+        may_pad = may_pad && (p0.dim == 2 || (plans[i]->variant >= 2 && sym_solve_supported(plans[i], p0.src_order)));
+    return solve_passes(p0, f, u, total, p0.src_order, may_pad, [&](double2 *w, long ld) -> int {
+        if (own_table) {
+            const size_t need = line_solve_multi_table_bytes(nplans, total);
+            if (c->multi_tab_bytes < need) {
+                HH_CUDA(cudaStreamSynchronize(c->stream));
+                cudaFree(c->multi_tab);
+                c->multi_tab = nullptr;
+                c->multi_tab_bytes = 0;
+                HH_CUDA(cudaMalloc(&c->multi_tab, need));
+                c->multi_tab_bytes = need;
+            }
+            table = c->multi_tab;
         }
-        table = c->multi_tab;
-    }
-    int rc = nplans > 1 ? launch_line_solve_multi(plans, nrhs, nplans, u, u, p0.src_order, table) : HH_ERR_UNSUPPORTED;
-    if (rc == HH_ERR_UNSUPPORTED) { // one launch per plan
-        rc = HH_OK;
-        long off = 0;
-        for (int i = 0; i < nplans && rc == HH_OK; i++) {
-            if (nrhs[i]) rc = launch_line_solve(plans[i], u + off, u + off, nrhs[i], p0.src_order);
-            off += p0.field * nrhs[i];
+        std::vector<Plan>   padded;
+        std::vector<Plan *> ps(plans, plans + nplans);
+        if (ld != p0.nx) {
+            padded.reserve((size_t)nplans);
+            for (int i = 0; i < nplans; i++) {
+                padded.push_back(padded_plan(*plans[i], ld));
+                ps[(size_t)i] = &padded[(size_t)i];
+            }
         }
-    }
-    HH_TRY(rc);
-    HH_TRY(stage_mark(*c, 2));
-    HH_TRY(transform_inverse(p0, u, total));
-    return stage_mark(*c, 3);
+        int rc = nplans > 1 ? launch_line_solve_multi(ps.data(), nrhs, nplans, w, w, p0.src_order, table) : HH_ERR_UNSUPPORTED;
+        if (rc == HH_ERR_UNSUPPORTED) { // one launch per plan
+            rc = HH_OK;
+            long off = 0;
+            for (int i = 0; i < nplans && rc == HH_OK; i++) {
+                if (nrhs[i]) rc = launch_line_solve(ps[(size_t)i], w + off, w + off, nrhs[i], p0.src_order);
+                off += ps[(size_t)i]->field * nrhs[i];
+            }
+        }
+        return rc;
+    });
 }
 
 extern "C" int hh_solve_source_multi(hh_plan *const *plans, const int *nrhs, int nplans, const double *f, double *u) {
@@ -1274,8 +1407,8 @@ static int solve_host_common(hh_plan *pl, const double *in_host, double *out_hos
         HH_CUDA(cudaMemcpyAsync(d, in_host + 2 * off, bytes, cudaMemcpyHostToDevice, c->copy_in));
         HH_CUDA(cudaEventRecord(c->chunk_ev[2 * i], c->copy_in));
         HH_CUDA(cudaStreamWaitEvent(c->stream, c->chunk_ev[2 * i], 0));
-        HH_TRY(source ? hh_solve_source(pl, (const double *)d, (double *)d, nb)
-                      : hh_solve(pl, (const double *)d, (double *)d, nb));
+        HH_TRY(source ? solve_source(pl, (const double *)d, (double *)d, nb, false)
+                      : solve_assembled(pl, (const double *)d, (double *)d, nb, false));
         HH_CUDA(cudaEventRecord(c->chunk_ev[2 * i + 1], c->stream));
         HH_CUDA(cudaStreamWaitEvent(c->copy_out, c->chunk_ev[2 * i + 1], 0));
         HH_CUDA(cudaMemcpyAsync(out_host + 2 * off, d, bytes, cudaMemcpyDeviceToHost, c->copy_out));
@@ -1315,7 +1448,7 @@ extern "C" int hh_solve_source_host_noalloc(hh_plan *pl, const double *f_host, d
     double2 *d = reinterpret_cast<hh_ctx *>(c)->noalloc_stage; // Ctx is the first member of hh_ctx
     const size_t bytes = sizeof(double2) * (size_t)p.field * batch;
     HH_CUDA(cudaMemcpyAsync(d, f_host, bytes, cudaMemcpyHostToDevice, c->stream));
-    HH_TRY(hh_solve_source(pl, (const double *)d, (double *)d, batch));
+    HH_TRY(solve_source(pl, (const double *)d, (double *)d, batch, false));
     HH_CUDA(cudaMemcpyAsync(u_host, d, bytes, cudaMemcpyDeviceToHost, c->stream));
     return hh_ctx_synchronize(reinterpret_cast<hh_ctx *>(c)); // Ctx is the first member of hh_ctx
 }

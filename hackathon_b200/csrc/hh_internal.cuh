@@ -77,6 +77,7 @@ struct Ctx {
     size_t                   l2_bytes = 0;        // the device's L2 size (3D transform slabs)
     std::string              dev_name;            // the device's model name (tuning-cache key)
     // stage timing (hh_ctx_set_stage_timing)
+    cudaMemPool_t            work_pool = nullptr; // the device's shared workspace pool (see solve_padded), referenced
     bool                     timing = false;
     bool                     fresh = true;        // tables, plans or the stream changed since the last launch
     std::vector<cudaEvent_t> ev_pending;          // groups of 4 events per timed solve
@@ -181,6 +182,9 @@ struct Plan {
     double   pade_linf = 0.0, pade_uinf = 0.0;     // their common limit (reached from row 9 on)
     double   h = 0.0;
     double2  k2 = {0.0, 0.0};
+    // padded rows (3D, inside a solve): line i + j nx lies at position i + j pitch of a layer; 0: no padding
+    int      pitch = 0;
+    long     span() const { return pitch ? (long)pitch * (lines / nx) : lines; } // positions of the lines
     // 3D line-range plans (a rank's pencil of a slab/pencil solve): the plan holds lines
     // [line0, line0 + lines) of the nx * ny lines and only solves lines (hh_solve_lines)
     long     line0 = 0;
@@ -220,6 +224,7 @@ int launch_residual(Plan *p, const double2 *u, const double2 *rhs, double2 *res,
 int launch_axpy(Ctx *c, double2 *u, const double2 *v, double s, long n); // u += s v
 int read_device_error(Ctx *c, int *val);
 long slab_planes(const Plan &p, long planes); // 3D transform slab in planes (the plan's or the default)
+bool sym_solve_supported(const Plan *p, int src_order);
 // the fused-source solve of several plans of one shape in one pass (hh_solve_source_multi);
 // table: device memory of line_solve_multi_table_bytes, or nullptr for the context's own
 int solve_source_multi(Plan *const *plans, const int *nrhs, int nplans, const double2 *f, double2 *u, void *table);

@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(NT, MINB)
                      long field, int batch, int rb, const double2 *__restrict__ Pv_one, const double2 *__restrict__ subt_one,
                      const double2 *__restrict__ diagt_one, int prow, const double *__restrict__ mu, SymParams sp,
                      const __grid_constant__ CUtensorMap in_map, int *err, const SymPlanRef *__restrict__ refs,
-                     const SymChunk *__restrict__ chunks) {
+                     const SymChunk *__restrict__ chunks, int pitch, int pitch_nx) {
     constexpr int NW = NT / 32, SPW = 32 / CW, LOG = ilog2_t<SPW>();
     constexpr int HALO = (SRC == 4 || SRC == 6) ? 1 : 0;
     __shared__ SymSmem<NW, CW, NR, MT> sm;
@@ -589,7 +589,11 @@ __global__ void __launch_bounds__(NT, MINB)
 
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     const int c = t % CW, seg = t / CW, sl = lane / CW;
-    const int q = blockIdx.x * CW + c;
+    // the line's position in a row of the field, and its number: with padded rows of `pitch` positions (3D),
+    // position i + j pitch holds line i + j pitch_nx, and the positions from pitch_nx on none
+    const int  at = blockIdx.x * CW + c;
+    const bool gap = pitch && at % pitch >= pitch_nx;
+    const int  q = pitch ? at / pitch * pitch_nx + at % pitch : at;
     // this CTA's right-hand sides and the plan they belong to
     int            b_begin, b_end;
     const double2 *Pv = Pv_one, *subt = subt_one, *diagt = diagt_one;
@@ -632,7 +636,7 @@ __global__ void __launch_bounds__(NT, MINB)
             }
         }
     }
-    const bool live = q < lines;
+    const bool live = q < lines && !gap;
     const int  qq = live ? q : 0;
     const int  r0 = seg * KS;
     const double m0 = mu[qq], m1 = mu[lines + qq], m2 = mu[2 * lines + qq];
@@ -740,7 +744,7 @@ __global__ void __launch_bounds__(NT, MINB)
         pdl_wait();
         pdl_next();
     }
-    const long off0 = (long)r0 * row_stride + qq;
+    const long off0 = (long)r0 * row_stride + (live ? at : 0);
     // warps whose rows all lie in [9, rows) use the constant Pade factors
     const bool tint = (w * SPW * KS >= 9) && ((w + 1) * SPW * KS <= rows);
     if (SRC == 6 && tint)
@@ -774,7 +778,7 @@ static int pick_rb(long groups, int batch, int resident, int nr) {
 // by value and bounded the kernel (line solve, real coefficients: 2D 1023^2 x 64 order 6 597 -> 552 us, order 4
 // 507 -> 467 us; 2D 511^2 x 32 order 4 62 -> 51 us; 3D 255^3 x 4 order 6 552 -> 506 us, order 4 497 -> 386 us)
 static int encode_line_map(CUtensorMap *map, const double2 *base, const Plan *p, int batch, int cw, int br) {
-    const unsigned long long dims[3] = {2ULL * (unsigned long long)p->lines, (unsigned long long)p->rows,
+    const unsigned long long dims[3] = {2ULL * (unsigned long long)p->span(), (unsigned long long)p->rows,
                                         (unsigned long long)batch};
     const unsigned long long strides[2] = {(unsigned long long)p->row_stride * 16, (unsigned long long)p->field * 16};
     const unsigned           box[3] = {2u * (unsigned)cw, (unsigned)br, 1};
@@ -811,7 +815,7 @@ static int launch_sym_t(Plan *p, const double2 *in, double2 *out, int batch, con
     if constexpr (TIO) HH_TRY(encode_line_map(&in_map, in, p, batch, CW, sym_tile_rows_per_box(p->rows)));
     HH_CUDA(cudaFuncSetAttribute(k_line_solve_sym<SRC, NT, CW, MINB, NR, KS, TIO, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  shm));
-    const long groups = (p->lines + CW - 1) / CW;
+    const long groups = (p->span() + CW - 1) / CW;
     int blocks_per_sm = 0, dev = 0, sms = 148;
     HH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, k_line_solve_sym<SRC, NT, CW, MINB, NR, KS, TIO, MT>, NT,
                                                           shm));
@@ -822,7 +826,7 @@ static int launch_sym_t(Plan *p, const double2 *in, double2 *out, int batch, con
     dim3 grid((unsigned)groups, (unsigned)chunks);
     return launch_kernel(p->ctx, k_line_solve_sym<SRC, NT, CW, MINB, NR, KS, TIO, MT>, grid, NT, (size_t)shm,
         in, out, p->lines, p->rows, p->row_stride, p->field, batch, rb, p->Pv, p->subt, p->diagt, p->prow, p->mu, sp,
-        in_map, p->ctx->err_word, multi ? multi->refs : nullptr, multi ? multi->chunks : nullptr);
+        in_map, p->ctx->err_word, multi ? multi->refs : nullptr, multi ? multi->chunks : nullptr, p->pitch, p->nx);
 }
 
 // The two builds of the kernel (hh_line_sym_real.cu, hh_line_sym_cplx.cu).

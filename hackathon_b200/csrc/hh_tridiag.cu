@@ -752,7 +752,7 @@ int launch_line_solve_multi(Plan *const *plans, const int *nrhs, int nplans, con
     // crossing a plan boundary
     const int ks = (p0->variant >= 5) ? 16 : kSeg;
     const int P = sym_segments(p0->rows, ks), CW = 256 / P, nr = (p0->variant == 4 && P > 8) ? 2 : 1;
-    const long groups = (p0->lines + CW - 1) / CW;
+    const long groups = (p0->span() + CW - 1) / CW;
     int dev = 0, sms = 148;
     HH_CUDA(cudaGetDevice(&dev));
     HH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

@@ -1,0 +1,123 @@
+"""Large solves with odd rows keep their transformed field in a padded workspace (fields past twice the L2);
+solves under stream capture work in place.  Both must give the same bits."""
+import gc
+
+import numpy as np
+import pytest
+
+import hackathon_b200 as hh
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def _random(shape, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.view_as_complex(torch.randn(shape + (2,), dtype=torch.float64, device="cuda", generator=g))
+
+
+def _both(stream, call):
+    """call() run directly and from a captured graph; clones of what each leaves."""
+    with torch.cuda.stream(stream):
+        direct = call().clone()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            out = call()
+        out.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        return direct, out.clone()
+
+
+@pytest.mark.parametrize("dim,n,order,k,batch,variant", [(3, 255, 6, 30.0, 1, 6), (3, 255, 4, 30.0, 1, 2), (3, 255, 6, 9 + 2j, 1, 5),
+                                                         (3, 125, 6, 20.0, 9, 6), (3, 125, 2, 20.0, 9, 0), (2, 2047, 6, 100.0, 4, 6),
+                                                         (2, 1023, 4, 50.0, 17, 3), (2, 1023, 6, 50 + 5j, 17, 6),
+                                                         (2, 701, 6, 50.0, 35, 1)])
+def test_padded_solve_same_bits_as_in_place(dim, n, order, k, batch, variant):
+    stream = torch.cuda.Stream()
+    ctx = hh.Context(0, stream.cuda_stream)
+    plan = hh.Plan.helmholtz(ctx, dim, n, order, k)
+    plan.variant = variant
+    torch.cuda.synchronize()
+    f = _random((batch,) + (n,) * dim, n + order)
+    u = torch.empty_like(f)
+    torch.cuda.synchronize()
+
+    def call():
+        plan.solve_source(f, u, batch)
+        return u
+
+    a, b = _both(stream, call)
+    assert torch.isfinite(torch.view_as_real(a)).all()
+    assert torch.equal(a, b)
+    w = f.clone()
+    torch.cuda.synchronize()
+    plan.solve_source(w, w, batch)  # in and out the same buffer
+    ctx.synchronize()
+    assert torch.equal(w, a)
+    plan.close()
+    ctx.close()
+
+
+def test_padded_multi_and_assembled_same_bits(oracle):
+    n, per = 1023, 6
+    stream = torch.cuda.Stream()
+    ctx = hh.Context(0, stream.cuda_stream)
+    plans = [hh.Plan.helmholtz(ctx, 2, n, 4, k) for k in (20.0, 33.0, 50.0 + 1j)]
+    f = _random((3 * per, n, n), 5)
+    u, solo = torch.empty_like(f), torch.empty_like(f)
+    torch.cuda.synchronize()
+    hh.solve_source_multi(plans, [per] * 3, f, u)
+    for i, p in enumerate(plans):  # six fields at a time stay under the line: in place
+        p.solve_source(f[i * per:(i + 1) * per], solo[i * per:(i + 1) * per], per)
+    ctx.synchronize()
+    assert torch.equal(u, solo)
+    rng = np.random.default_rng(3)
+    coef = {nm: np.ascontiguousarray(c + 0.02 * (rng.random(n) + 1j * rng.random(n)), dtype=np.complex128)
+            for nm, c in (("bp", 0.16), ("ap", 0.66), ("b", 0.66), ("a", -3.9), ("bm", 0.16), ("am", 0.66))}
+    plan = hh.Plan.from_coefficients_2d(ctx, n, n, coef)
+    torch.cuda.synchronize()
+
+    def call():
+        plan.solve(f, u, 3 * per)
+        return u
+
+    a, b = _both(stream, call)
+    assert torch.equal(a, b)
+    ctx.close()
+
+
+def test_padded_workspace_shared_and_given_back():
+    """Two contexts on two streams solve at once, each to its own solo result; the last context gives the
+    workspace back."""
+    n, batch = 1023, 17
+    torch.cuda.synchronize()
+    gc.collect()
+    torch.cuda.empty_cache()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    f = [_random((batch, n, n), s) for s in range(2)]
+    u = [torch.empty_like(x) for x in f]
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    ctxs = [hh.Context(0, s.cuda_stream) for s in streams]
+    plans = [hh.Plan.helmholtz(c, 2, n, 6, 30.0 + 10 * i) for i, c in enumerate(ctxs)]
+    want = []
+    for p, x, y, c in zip(plans, f, u, ctxs):
+        p.solve_source(x, y, batch)
+        c.synchronize()
+        want.append(y.clone())
+        y.zero_()
+    torch.cuda.synchronize()
+    for _ in range(4):
+        for p, x, y in zip(plans, f, u):
+            p.solve_source(x, y, batch)
+    for c in ctxs:
+        c.synchronize()
+    for y, w in zip(u, want):
+        assert torch.equal(y, w)
+    del want, w
+    torch.cuda.empty_cache()
+    for c in ctxs:
+        c.close()
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] >= free0 - (64 << 20)
