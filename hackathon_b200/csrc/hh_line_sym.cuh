@@ -562,14 +562,25 @@ struct SymPlanRef {
 struct SymChunk {
     int plan, b0, b1, pad;
 };
+// The table of a multi-plan launch (none: nchunks 0): a small one travels in the kernel's arguments, because the
+// two copies to device memory that larger ones take wait for the kernel before them and hold the line solve back
+// (2D 255^2, 8 plans x 4: 55.7 us a solve with them, 48.4 without).
+struct SymMulti {
+    static constexpr int kPlans = 16, kChunks = 64;
+    int               nchunks = 0;      // the grid's y extent
+    const SymPlanRef *refs = nullptr;   // in device memory, or null: the arrays below
+    const SymChunk   *chunks = nullptr;
+    SymPlanRef        iref[kPlans];
+    SymChunk          ichunk[kChunks];
+};
 
 template <int SRC, int NT, int CW, int MINB, int NR, int KS, bool TIO, typename MT>
 __global__ void __launch_bounds__(NT, MINB)
     k_line_solve_sym(const double2 *__restrict__ in, double2 *__restrict__ out, int lines, int rows, long row_stride,
                      long field, int batch, int rb, const double2 *__restrict__ Pv_one, const double2 *__restrict__ subt_one,
                      const double2 *__restrict__ diagt_one, int prow, const double *__restrict__ mu, SymParams sp,
-                     const __grid_constant__ CUtensorMap in_map, int *err, const SymPlanRef *__restrict__ refs,
-                     const SymChunk *__restrict__ chunks, int pitch, int pitch_nx) {
+                     const __grid_constant__ CUtensorMap in_map, int *err, int pitch, int pitch_nx,
+                     const __grid_constant__ SymMulti tab) {
     constexpr int NW = NT / 32, SPW = 32 / CW, LOG = ilog2_t<SPW>();
     constexpr int HALO = (SRC == 4 || SRC == 6) ? 1 : 0;
     __shared__ SymSmem<NW, CW, NR, MT> sm;
@@ -597,9 +608,9 @@ __global__ void __launch_bounds__(NT, MINB)
     // this CTA's right-hand sides and the plan they belong to
     int            b_begin, b_end;
     const double2 *Pv = Pv_one, *subt = subt_one, *diagt = diagt_one;
-    if (chunks) {
-        const SymChunk   ch = chunks[blockIdx.y];
-        const SymPlanRef pr = refs[ch.plan];
+    if (tab.nchunks) {
+        const SymChunk   ch = tab.chunks ? tab.chunks[blockIdx.y] : tab.ichunk[blockIdx.y];
+        const SymPlanRef pr = tab.chunks ? tab.refs[ch.plan] : tab.iref[ch.plan];
         b_begin = ch.b0;
         b_end = ch.b1;
         Pv = pr.Pv;
@@ -785,14 +796,6 @@ static int encode_line_map(CUtensorMap *map, const double2 *base, const Plan *p,
     return encode_tensor_map(map, base, 3, dims, strides, box);
 }
 
-// A multi-plan launch: the plans' references and the chunk table, in device memory the caller
-// provides, and the chunk count (the grid's y extent).
-struct SymMulti {
-    const SymPlanRef *refs = nullptr;
-    const SymChunk   *chunks = nullptr;
-    int               nchunks = 0;
-};
-
 template <int SRC, int CW, int MINB, int NR, int KS, bool TIO, typename MT>
 static int launch_sym_t(Plan *p, const double2 *in, double2 *out, int batch, const SymMulti *multi) {
     constexpr int NT = 256, SPW = 32 / CW, LOG = ilog2_t<SPW>();
@@ -826,7 +829,7 @@ static int launch_sym_t(Plan *p, const double2 *in, double2 *out, int batch, con
     dim3 grid((unsigned)groups, (unsigned)chunks);
     return launch_kernel(p->ctx, k_line_solve_sym<SRC, NT, CW, MINB, NR, KS, TIO, MT>, grid, NT, (size_t)shm,
         in, out, p->lines, p->rows, p->row_stride, p->field, batch, rb, p->Pv, p->subt, p->diagt, p->prow, p->mu, sp,
-        in_map, p->ctx->err_word, multi ? multi->refs : nullptr, multi ? multi->chunks : nullptr, p->pitch, p->nx);
+        in_map, p->ctx->err_word, p->pitch, p->nx, multi ? *multi : SymMulti{});
 }
 
 // The two builds of the kernel (hh_line_sym_real.cu, hh_line_sym_cplx.cu).

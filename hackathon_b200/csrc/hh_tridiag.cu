@@ -769,15 +769,20 @@ int launch_line_solve_multi(Plan *const *plans, const int *nrhs, int nplans, con
         set_error("multi-plan line solve: %zu chunks", chunks.size());
         return HH_ERR_UNSUPPORTED;
     }
-    char *tab = static_cast<char *>(table_dev);
-    HH_CUDA(cudaMemcpyAsync(tab, refs.data(), sizeof(SymPlanRef) * refs.size(), cudaMemcpyHostToDevice, p0->ctx->stream));
-    HH_CUDA(cudaMemcpyAsync(tab + sizeof(SymPlanRef) * refs.size(), chunks.data(), sizeof(SymChunk) * chunks.size(),
-                            cudaMemcpyHostToDevice, p0->ctx->stream));
-    p0->ctx->fresh = true; // the kernel's set-up reads the table
     SymMulti m;
-    m.refs = reinterpret_cast<const SymPlanRef *>(tab);
-    m.chunks = reinterpret_cast<const SymChunk *>(tab + sizeof(SymPlanRef) * refs.size());
     m.nchunks = (int)chunks.size();
+    if (nplans <= SymMulti::kPlans && chunks.size() <= (size_t)SymMulti::kChunks) {
+        std::copy(refs.begin(), refs.end(), m.iref);
+        std::copy(chunks.begin(), chunks.end(), m.ichunk);
+    } else {
+        char *tab = static_cast<char *>(table_dev);
+        HH_CUDA(cudaMemcpyAsync(tab, refs.data(), sizeof(SymPlanRef) * refs.size(), cudaMemcpyHostToDevice, p0->ctx->stream));
+        HH_CUDA(cudaMemcpyAsync(tab + sizeof(SymPlanRef) * refs.size(), chunks.data(), sizeof(SymChunk) * chunks.size(),
+                                cudaMemcpyHostToDevice, p0->ctx->stream));
+        p0->ctx->fresh = true; // the kernel's set-up reads the table
+        m.refs = reinterpret_cast<const SymPlanRef *>(tab);
+        m.chunks = reinterpret_cast<const SymChunk *>(tab + sizeof(SymPlanRef) * refs.size());
+    }
     // one kernel for all: the complex one (the same bits on a real plan) unless every plan is real
     bool real = true;
     for (int i = 0; i < nplans; i++) real = real && plans[i]->real_coef;

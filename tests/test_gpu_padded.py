@@ -1,6 +1,8 @@
 """Large solves with odd rows keep their transformed field in a padded workspace (fields past twice the L2);
 solves under stream capture work in place.  Both must give the same bits."""
-import gc
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -87,37 +89,46 @@ def test_padded_multi_and_assembled_same_bits(oracle):
     ctx.close()
 
 
+_SHARED = """
+import torch
+import hackathon_b200 as hh
+n, batch = 1023, 17
+streams = [torch.cuda.Stream() for _ in range(2)]
+g = torch.Generator(device="cuda").manual_seed(7)
+f = [torch.view_as_complex(torch.randn((batch, n, n, 2), dtype=torch.float64, device="cuda", generator=g)) for _ in range(2)]
+u = [torch.empty_like(x) for x in f]
+torch.cuda.synchronize()
+free0 = torch.cuda.mem_get_info()[0]
+ctxs = [hh.Context(0, s.cuda_stream) for s in streams]
+plans = [hh.Plan.helmholtz(c, 2, n, 6, 30.0 + 10 * i) for i, c in enumerate(ctxs)]
+want = []
+for p, x, y, c in zip(plans, f, u, ctxs):
+    p.solve_source(x, y, batch)
+    c.synchronize()
+    want.append(y.clone())
+    y.zero_()
+torch.cuda.synchronize()
+for _ in range(4):
+    for p, x, y in zip(plans, f, u):
+        p.solve_source(x, y, batch)
+for c in ctxs:
+    c.synchronize()
+assert all(torch.equal(y, w) for y, w in zip(u, want))
+del want
+torch.cuda.empty_cache()
+held = free0 - torch.cuda.mem_get_info()[0]
+for c in ctxs:
+    c.close()
+torch.cuda.synchronize()
+left = free0 - torch.cuda.mem_get_info()[0]
+assert held >= batch * 1024 * n * 16 and left < batch * 1024 * n * 8, (held, left)
+print("shared ok")
+"""
+
+
 def test_padded_workspace_shared_and_given_back():
     """Two contexts on two streams solve at once, each to its own solo result; the last context gives the
-    workspace back."""
-    n, batch = 1023, 17
-    torch.cuda.synchronize()
-    gc.collect()
-    torch.cuda.empty_cache()
-    streams = [torch.cuda.Stream() for _ in range(2)]
-    f = [_random((batch, n, n), s) for s in range(2)]
-    u = [torch.empty_like(x) for x in f]
-    torch.cuda.synchronize()
-    free0 = torch.cuda.mem_get_info()[0]
-    ctxs = [hh.Context(0, s.cuda_stream) for s in streams]
-    plans = [hh.Plan.helmholtz(c, 2, n, 6, 30.0 + 10 * i) for i, c in enumerate(ctxs)]
-    want = []
-    for p, x, y, c in zip(plans, f, u, ctxs):
-        p.solve_source(x, y, batch)
-        c.synchronize()
-        want.append(y.clone())
-        y.zero_()
-    torch.cuda.synchronize()
-    for _ in range(4):
-        for p, x, y in zip(plans, f, u):
-            p.solve_source(x, y, batch)
-    for c in ctxs:
-        c.synchronize()
-    for y, w in zip(u, want):
-        assert torch.equal(y, w)
-    del want, w
-    torch.cuda.empty_cache()
-    for c in ctxs:
-        c.close()
-    torch.cuda.synchronize()
-    assert torch.cuda.mem_get_info()[0] >= free0 - (64 << 20)
+    workspace back (in a process of its own: the workspace is shared by every context on the device)."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _SHARED], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "shared ok" in r.stdout, r.stdout + r.stderr
