@@ -433,9 +433,9 @@ template <int M> struct WCfg;
 // kernel (2: the next line loads while one is transformed; 1: more warps per SM instead), MINB
 // CTAs per SM the register budget is sized for; CWPC warps per CTA and CNT tiles per warp in the
 // columns kernel (CNT - 1 tiles load while one is transformed); RING: the rows use the CTA-ring
-// kernel with RWPC warps per CTA
+// kernel with RWPC warps per CTA: 0 never, 1 always, 2 from ring_lines() lines on
 template <> struct WCfg<1024> { static constexpr int TL = 32, R = 32, WPC = 2, NBUF = 2, MINB = 3, CWPC = 2, CNT = 2, RWPC = 4, RING = 1; };
-template <> struct WCfg<512>  { static constexpr int TL = 16, R = 32, WPC = 2, NBUF = 2, MINB = 3, CWPC = 2, CNT = 2, RWPC = 4, RING = 0; };
+template <> struct WCfg<512>  { static constexpr int TL = 16, R = 32, WPC = 2, NBUF = 2, MINB = 3, CWPC = 2, CNT = 2, RWPC = 4, RING = 2; };
 template <> struct WCfg<256>  { static constexpr int TL = 16, R = 16, WPC = 4, NBUF = 2, MINB = 3, CWPC = 4, CNT = 2, RWPC = 4, RING = 0; };
 template <> struct WCfg<128>  { static constexpr int TL = 8,  R = 16, WPC = 4, NBUF = 2, MINB = 3, CWPC = 4, CNT = 2, RWPC = 4, RING = 0; };
 template <> struct WCfg<64>   { static constexpr int TL = 8,  R = 8,  WPC = 4, NBUF = 2, MINB = 3, CWPC = 4, CNT = 2, RWPC = 4, RING = 0; };
@@ -1611,9 +1611,21 @@ template <int M, bool LP, bool UPD = false> static int launch_w2(Ctx *c, const D
                                                                         c->err_word);
 }
 
+// The ring's CTAs hold RWPC line groups and stand two on an SM, the per-warp kernel's hold two: with fewer lines
+// than give every SM one ring CTA, the smaller CTAs spread better.  511^2, whole solves, per-warp -> ring:
+// 1 right-hand side (511 lines) 20.6 -> 22.4 us, 2 24.7 -> 28.5, 4 (2044 lines) 35.5 -> 31.9, 32 176.5 -> 162.8;
+// the rows transform of 128: 230 -> 197 us.
+template <int M> static long ring_lines() {
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        sms = 148;
+    return (long)sms * WCfg<M>::RWPC * WGeom<M>::LPW; // 1184 lines of 511
+}
+
 // rows kernel: a.rows_kernel 1 = the CTA ring, 2 = per-warp buffers, 0 = the length's default
 template <int M, bool LP, bool UPD = false> static int launch_w(Ctx *c, const DstArgs &a) {
-    const bool ring = a.rows_kernel == 0 ? (bool)WCfg<M>::RING : a.rows_kernel == 1;
+    const bool ring = a.rows_kernel ? a.rows_kernel == 1
+                                    : WCfg<M>::RING == 1 || (WCfg<M>::RING == 2 && a.nlines * a.planes >= ring_lines<M>());
     return ring ? launch_wr<M, LP, UPD>(c, a) : launch_wp<M, LP, UPD>(c, a);
 }
 

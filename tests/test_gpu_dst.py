@@ -47,6 +47,20 @@ def test_dst_rows_1023_ring_ticket_counts(ctx, oracle, rows):
     assert rel_err(_host(dst), oracle.dst1_rows(x)) < 1e-13
 
 
+@pytest.mark.parametrize("rows", [1183, 1184, 1185, 3553, 5001])
+def test_dst_rows_511_at_the_ring_threshold(ctx, oracle, rows):
+    """511-point rows take the CTA-ring kernel from one block of four two-line groups per SM on
+    (1184 lines on 148 SMs): one line below, at, one above (a half-filled group), one more line
+    than all ring buffers hold, and lines that fall unevenly on the blocks."""
+    n = 511
+    rng = np.random.default_rng(rows + 3)
+    x = rng.standard_normal((rows, n)) + 1j * rng.standard_normal((rows, n))
+    src, dst = _dev(x), torch.empty((rows, n), dtype=torch.complex128, device="cuda")
+    ctx.dst1_rows(n, rows, src, dst)
+    ctx.synchronize()
+    assert rel_err(_host(dst), oracle.dst1_rows(x)) < 1e-13
+
+
 @pytest.mark.parametrize("rows", [1, 3, 593, 888, 889, 3001])
 def test_dst_rows_2047_two_warp_ticket_counts(ctx, oracle, rows):
     """2047-point rows go through the two-warps-per-line kernel (four lines per block, six line
