@@ -15,24 +15,26 @@
 // place), and its warps walk units (8 odd and 8 even outputs) x (NTW tiles of 4 complex lines =
 // 8 real columns): mma.m8n8k4 in FP64 with the sine fragments as A and the lines as B.  The
 // sines come from a table laid out fragment by fragment, the odd and the even matrix side by side,
-// so that a lane reads both of its values with one 16-byte load, four steps ahead, and no shared
+// so that a lane reads both of its values with one 16-byte load, two steps ahead, and no shared
 // memory is spent on them: every CTA reads the table once (4 n^2 bytes, from L1/L2).  The C
 // fragment's two values are the real and imaginary part of one output, and the lane that holds output
 // 2i of a line also holds output 2i + 1, so stores go out as 32-byte pairs.
 //
-// Bound by the FP64 tensor rate from n ~ 200 on (37 TF measured; 4800 rows of n = 300 take 46 us, 23 us
+// Bound by the FP64 tensor rate from n ~ 200 on (37 TF measured; 8000 rows of n = 500 take 139 us, 108 us
 // of it at that rate), below that by the load and store phases.  Against one dot product per thread
-// with uncoalesced sines before: 8000 rows of n = 500 5083 -> 166 us, 40000 rows of n = 100 585 -> 52
-// us, columns 643 -> 48 us.
+// with uncoalesced sines before: 8000 rows of n = 500 5083 -> 139 us, 40000 rows of n = 100 585 -> 43.5
+// us, columns 643 -> 42 us.
 #include "hh_internal.cuh"
 
 #include <algorithm>
+#include <cmath>
 
 namespace hh {
 
 namespace {
 
 constexpr int kMmaThreads = 256, kMmaWarps = kMmaThreads / 32;
+constexpr int kTabAhead = 2; // table steps in flight (a pair per pass of the product loop)
 constexpr int kMmaSmemMax = 227 * 1024;
 // the longest line that fits four to a CTA in both layouts (2 * 1200 * 6 * 16 bytes at n = 2400)
 constexpr int kMmaMaxN = 2400;
@@ -47,27 +49,32 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
 __host__ __device__ inline int half_up(int n) { return (n + 1) / 2; }
 __host__ __device__ inline int k4_steps(int n) { return (half_up(n) + 3) / 4; }
 __host__ __device__ inline int out_tiles(int n) { return (half_up(n) + 7) / 8; }
-// shared-memory pitches in complex values: a B fragment is 4 values of j by 8 real columns, read
+// Shared memory holds blocks of four a_j and then their four d_j, so that a lane reaches a step's both values of
+// a line by constant offsets.  Pitches in complex values: a B fragment is 4 values of j by 8 real columns, read
 // by half warps of 4 x 4; rows (line-major): pitch = 4 mod 8 puts the two lines of a half warp on
 // different 64-byte halves of the banks; columns (j-major): pitch = 2 or 6 mod 8 puts its four j on
 // four different 32-byte quarters
-__host__ __device__ inline int rows_pitch(int n) { return 4 * k4_steps(n) + (k4_steps(n) % 2 ? 0 : 4); }
+__host__ __device__ inline int rows_pitch(int n) { return 8 * k4_steps(n) + 4; }
 __host__ __device__ inline int cols_pitch(int nl) { return nl + 2; } // nl is a multiple of 4
 
 inline size_t mma_smem(bool cols, int n, int nl) {
-    return 2 * sizeof(double2) * (cols ? (size_t)4 * k4_steps(n) * cols_pitch(nl) : (size_t)nl * rows_pitch(n));
+    return sizeof(double2) * (cols ? (size_t)8 * k4_steps(n) * cols_pitch(nl) : (size_t)nl * rows_pitch(n));
 }
 
-// COLS: line c of a plane is column c (element j at c + j ld); otherwise row c (element j at c ld + j)
+// COLS: line c of a plane is column c (element j at c + j ld); otherwise row c (element j at c ld + j).
+// What is not a product counts here: at n = 100 a warp's one unit is 208 of its instructions, and with plain
+// indexing in the three phases it ran 1262, now 776 (40000 rows 49 -> 43.5 us, 8000 rows of n = 500 160 -> 139,
+// 61504 of n = 31 23 -> 17.5, 100 columns x 400 planes 46 -> 42); so the addresses of a phase advance by constants, nothing is computed per thread that the launch can pass, and the first table steps of a unit are on
+// their way before its lines are.
 template <bool COLS, int NTW>
 __global__ void __launch_bounds__(kMmaThreads, 3)
     k_dst1_mma(const double2 *in, double2 *out, int n, long nlines, long in_ld, long out_ld, long in_plane,
-               long out_plane, int groups, const double2 *__restrict__ tab) {
+               long out_plane, int groups, double coef, const double2 *__restrict__ tab) {
     extern __shared__ __align__(16) double2 mma_sm[];
-    const int  h1 = half_up(n), p = n / 2, ks = k4_steps(n), nl = 4 * NTW * groups;
+    const int  h1 = half_up(n), ks = k4_steps(n), nl = 4 * NTW * groups;
     const int  pitch = COLS ? cols_pitch(nl) : rows_pitch(n);
-    double2   *sa = mma_sm, *sd = mma_sm + (COLS ? 4 * ks : nl) * pitch;
     const int  lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int  units = out_tiles(n) * groups;
     const long l0 = (long)blockIdx.x * nl;
     const int  live = (int)min((long)nl, nlines - l0);
     const double2 zero = make_double2(0.0, 0.0);
@@ -76,98 +83,135 @@ __global__ void __launch_bounds__(kMmaThreads, 3)
 
     pdl_wait();
     pdl_next();
+    auto tile_of = [&](int u) { return groups == 1 ? u : u / groups; };
+    // (reads past a tile's last step stay in the table: it ends in kTabAhead spare steps)
+    const double2 *q = tab + (long)tile_of(warp) * ks * 32 + lane;
+    double2        cur[kTabAhead];
+    if (warp < units)
+#pragma unroll
+        for (int i = 0; i < kTabAhead; i++) cur[i] = __ldg(q + i * 32);
+
     // ---- a_j and d_j of every line; zeros past the halves and for lines past the end
-    auto put = [&](int at, int j, double2 x, double2 m) {
-        const bool mid = 2 * j + 1 == n;
-        sa[at] = mid ? x : cadd(x, m);
-        sd[at] = mid ? zero : csub(x, m);
+    const int mid = n & 1 ? n / 2 : -1; // x_mid stands alone
+    double2   x[4], m[4];
+    int       at[4], js[4];
+    auto      put = [&]() {
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            if (at[e] >= 0) {
+                mma_sm[at[e]] = js[e] == mid ? x[e] : cadd(x[e], m[e]);
+                mma_sm[at[e] + (COLS ? 4 * pitch : 4)] = js[e] == mid ? zero : csub(x[e], m[e]);
+            }
     };
     if constexpr (COLS) {
-        for (int e0 = threadIdx.x; e0 < 4 * ks * nl; e0 += 4 * kMmaThreads) {
-            double2 x[4], m[4];
+        const int dj = kMmaThreads / nl, dc = kMmaThreads - dj * nl;
+        int       j = threadIdx.x / nl, c = threadIdx.x - j * nl;
+        while (j < 4 * ks) {
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int j = (e0 + q * kMmaThreads) / nl, c = e0 + q * kMmaThreads - j * nl;
-                x[q] = m[q] = zero;
+            for (int e = 0; e < 4; e++) {
+                x[e] = m[e] = zero;
                 if (j < h1 && c < live) {
-                    x[q] = in[c + (long)j * in_ld];
-                    m[q] = in[c + (long)(n - 1 - j) * in_ld];
+                    x[e] = in[c + j * in_ld];
+                    m[e] = in[c + (n - 1 - j) * in_ld];
+                }
+                at[e] = j < 4 * ks ? (2 * j - (j & 3)) * pitch + c : -1;
+                js[e] = j;
+                j += dj;
+                c += dc;
+                if (c >= nl) {
+                    c -= nl;
+                    j++;
                 }
             }
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int j = (e0 + q * kMmaThreads) / nl, c = e0 + q * kMmaThreads - j * nl;
-                if (j < 4 * ks) put(j * pitch + c, j, x[q], m[q]);
-            }
+            put();
         }
     } else {
-        for (int c = warp; c < nl; c += kMmaWarps)
-            for (int j0 = lane; j0 < 4 * ks; j0 += 128) {
-                double2 x[4], m[4];
+        // a warp takes pieces of 32 j, `pieces` to a line
+        const int pieces = (4 * ks + 31) / 32, dc = kMmaWarps / pieces, dr = kMmaWarps - dc * pieces;
+        int       c = warp / pieces, r = warp - c * pieces;
+        while (c < nl) {
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const int j = j0 + 32 * q;
-                    x[q] = m[q] = zero;
-                    if (j < h1 && c < live) {
-                        x[q] = in[c * in_ld + j];
-                        m[q] = in[c * in_ld + (n - 1 - j)];
-                    }
+            for (int e = 0; e < 4; e++) {
+                const int j = 32 * r + lane;
+                x[e] = m[e] = zero;
+                if (j < h1 && c < live) {
+                    const double2 *line = in + c * in_ld;
+                    x[e] = line[j];
+                    m[e] = line[n - 1 - j];
                 }
-#pragma unroll
-                for (int q = 0; q < 4; q++)
-                    if (j0 + 32 * q < 4 * ks) put(c * pitch + j0 + 32 * q, j0 + 32 * q, x[q], m[q]);
+                at[e] = j < 4 * ks && c < nl ? c * pitch + 2 * j - (j & 3) : -1;
+                js[e] = j;
+                c += dc;
+                r += dr;
+                if (r >= pieces) {
+                    r -= pieces;
+                    c++;
+                }
             }
+            put();
+        }
     }
     __syncthreads();
 
-    const int    kk = lane & 3, nn = lane >> 2; // the lane's j within a step and real column within a tile
-    const int    units = out_tiles(n) * groups;
-    const double coef = sqrt(2.0 / (n + 1));
-    // strides in doubles: from one step of four j to the next, and from one tile of four lines to the next
-    const int kstep = COLS ? 8 * pitch : 8, nstep = COLS ? 8 : 8 * pitch;
-    const int b0 = 2 * (COLS ? kk * pitch + (nn >> 1) : (nn >> 1) * pitch + kk) + (nn & 1);
-    constexpr int PF = 2; // table steps in flight
+    const int     kk = lane & 3, nn = lane >> 2; // the lane's j within a step and real column within a tile
+    const double *lines = reinterpret_cast<const double *>(mma_sm) + (nn & 1);
     for (int u = warp; u < units; u += kMmaWarps) {
-        const int      tile = u / groups, c0 = (u - tile * groups) * 4 * NTW;
-        const double2 *q = tab + ((long)tile * ks) * 32 + lane;
-        const double  *ba = reinterpret_cast<const double *>(sa) + b0 + (c0 / 4) * nstep;
-        const double  *bd = reinterpret_cast<const double *>(sd) + b0 + (c0 / 4) * nstep;
-        double ao[NTW][2], ae[NTW][2];
+        const int tile = tile_of(u), c0 = (u - tile * groups) * 4 * NTW;
+        double    ao[NTW][2], ae[NTW][2];
 #pragma unroll
         for (int t = 0; t < NTW; t++) ao[t][0] = ao[t][1] = ae[t][0] = ae[t][1] = 0.0;
-        double2 cur[PF];
+        // rows: b[t] walks the line of tile t; columns: b[0] and b[1] walk the a_j and the d_j
+        constexpr int NB = COLS ? 2 : NTW;
+        const double *b[NB];
+        if constexpr (COLS) {
+            b[0] = lines + 2 * (kk * pitch + (nn >> 1) + c0);
+            b[1] = b[0] + 8 * pitch;
+        } else {
 #pragma unroll
-        for (int i = 0; i < PF; i++)
-            if (i < ks) cur[i] = __ldg(q + i * 32);
-        for (int k = 0; k < ks; k += PF) {
-            double2 nxt[PF];
+            for (int t = 0; t < NTW; t++) b[t] = lines + 2 * ((c0 + 4 * t + (nn >> 1)) * pitch + kk);
+        }
+        auto step = [&](double2 sine, int i) {
 #pragma unroll
-            for (int i = 0; i < PF; i++)
-                if (k + PF + i < ks) nxt[i] = __ldg(q + (k + PF + i) * 32);
-#pragma unroll
-            for (int i = 0; i < PF; i++) {
-                if (k + i < ks) {
-#pragma unroll
-                    for (int t = 0; t < NTW; t++) {
-                        dmma(ao[t], cur[i].x, ba[(k + i) * kstep + t * nstep]);
-                        dmma(ae[t], cur[i].y, bd[(k + i) * kstep + t * nstep]);
-                    }
-                }
+            for (int t = 0; t < NTW; t++) {
+                dmma(ao[t], sine.x, COLS ? b[0][8 * t] : b[COLS ? 0 : t][16 * i]);
+                dmma(ae[t], sine.y, COLS ? b[1][8 * t] : b[COLS ? 0 : t][16 * i + 8]);
             }
+            if constexpr (COLS) {
+                b[0] += 16 * pitch;
+                b[1] += 16 * pitch;
+            }
+        };
+        for (int k = kTabAhead; k <= ks; k += kTabAhead) {
+            double2 nxt[kTabAhead];
+            q += 32 * kTabAhead;
 #pragma unroll
-            for (int i = 0; i < PF; i++) cur[i] = nxt[i];
+            for (int i = 0; i < kTabAhead; i++) nxt[i] = __ldg(q + i * 32);
+#pragma unroll
+            for (int i = 0; i < kTabAhead; i++) step(cur[i], i);
+            if constexpr (!COLS)
+#pragma unroll
+                for (int t = 0; t < NTW; t++) b[t] += 16 * kTabAhead;
+#pragma unroll
+            for (int i = 0; i < kTabAhead; i++) cur[i] = nxt[i];
+        }
+        static_assert(kTabAhead == 2, "at most one step is left");
+        if (ks & 1) step(cur[0], 0);
+        if (u + kMmaWarps < units) {
+            q = tab + (long)tile_of(u + kMmaWarps) * ks * 32 + lane;
+#pragma unroll
+            for (int i = 0; i < kTabAhead; i++) cur[i] = __ldg(q + i * 32);
         }
         // output 2i (S_{2i+1}) and 2i + 1 (S_{2i+2}) of line c0 + 4 t + kk
-        const int i = 8 * tile + nn;
+        const int  i2 = 16 * tile + 2 * nn;
+        double2   *o = out + (COLS ? c0 + kk + i2 * out_ld : (c0 + kk) * out_ld + i2);
+        const long next = COLS ? out_ld : 1;
 #pragma unroll
         for (int t = 0; t < NTW; t++) {
-            const int c = c0 + 4 * t + kk;
-            if (c < live) {
-                double2   *o = out + (COLS ? c + (long)(2 * i) * out_ld : c * out_ld + 2 * i);
-                const long step = COLS ? out_ld : 1;
-                if (i < h1) o[0] = make_double2(coef * ao[t][0], coef * ao[t][1]);
-                if (i < p) o[step] = make_double2(coef * ae[t][0], coef * ae[t][1]);
+            if (c0 + 4 * t + kk < live) {
+                if (i2 < n) o[0] = make_double2(coef * ao[t][0], coef * ao[t][1]);
+                if (i2 + 1 < n) o[next] = make_double2(coef * ae[t][0], coef * ae[t][1]);
             }
+            o += COLS ? 4 : 4 * out_ld;
         }
     }
 }
@@ -231,11 +275,11 @@ __global__ void __launch_bounds__(kDenseThreads)
 
 // Lines per CTA: 4 ntw lines per warp unit, `groups` units side by side.
 //  * groups: the least that gives all eight warps a unit (n < 64 has fewer than eight output tiles).
-//  * ntw: the widest of 4, 3, 2 whose lines leave room for three CTAs on an SM (n = 100: 52 us at 4
-//    against 54 at 3 and 56 at 2 for 40000 rows; n = 300: 46 us at 3 against 50 at 2; n = 500: 166 us
-//    at 2 against 196 at 1, two CTAs per SM with 3: 179), then 2 with two CTAs (n = 700: 228 us, 241 at
-//    1), then 1 (n = 1000: 655 us, 771 at 2).  Columns take the width (up to 5) that
-//    leaves the fewest idle columns in a plane's last tile (100 columns: 48 us at 5, 52 at 4).
+//  * ntw: the widest of 4, 3, 2 whose lines leave room for three CTAs on an SM (n = 100: 43.5 us at 4
+//    against 44.5 at 3 and 48 at 2 for 40000 rows; n = 300: 38 us at 3 against 41 at 2; n = 500: 139 us
+//    at 2 against 152 at 1, two CTAs per SM with 3: 146), then 2 with two CTAs, then 1 (n = 1000, 2000 rows:
+//    161 us, 169 at 2).  Columns take the width (up to 5) that
+//    leaves the fewest idle columns in a plane's last tile (100 columns: 42 us at 5, 46.5 at 4).
 //  * fewer lines per CTA where the launch would not give every SM two (7688 rows of n = 31: 4.8 us at 24
 //    lines, 6.4 at 48; 2500 rows of n = 50: 3.6 us at 8, 4.5 at 16).
 void dense_shape(bool cols, int n, long nlines, long planes, int *ntw, int *groups) {
@@ -262,7 +306,7 @@ int launch_mma(Ctx *c, int n, long nlines, long planes, const double2 *in, long 
     HH_CUDA(cudaFuncSetAttribute(k_dst1_mma<COLS, NTW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
     dim3 grid((unsigned)((nlines + nl - 1) / nl), (unsigned)planes);
     return launch_kernel(c, k_dst1_mma<COLS, NTW>, grid, kMmaThreads, shm, in, out, n, nlines, in_ld, out_ld, in_plane, out_plane,
-                                                                 groups, tab);
+                                                                 groups, std::sqrt(2.0 / (n + 1)), tab);
 }
 
 } // namespace
@@ -273,7 +317,7 @@ int dense_for(Ctx *c, int n, const double **mat) {
     if (it == c->dense.end()) {
         double *d = nullptr;
         if (n <= kMmaMaxN) {
-            HH_CUDA(cudaMalloc(&d, sizeof(double2) * 32 * (size_t)out_tiles(n) * k4_steps(n)));
+            HH_CUDA(cudaMalloc(&d, sizeof(double2) * 32 * ((size_t)out_tiles(n) * k4_steps(n) + kTabAhead)));
             k_make_mma<<<256, 256, 0, c->stream>>>(n, reinterpret_cast<double2 *>(d));
         } else {
             HH_CUDA(cudaMalloc(&d, sizeof(double) * (size_t)n * (size_t)n));
