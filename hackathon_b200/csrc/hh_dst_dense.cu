@@ -28,12 +28,12 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 namespace hh {
 
 namespace {
 
-constexpr int kMmaThreads = 256, kMmaWarps = kMmaThreads / 32;
 constexpr int kTabAhead = 2; // table steps in flight (a pair per pass of the product loop)
 constexpr int kMmaSmemMax = 227 * 1024;
 // the longest line that fits four to a CTA in both layouts (2 * 1200 * 6 * 16 bytes at n = 2400)
@@ -49,6 +49,10 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
 __host__ __device__ inline int half_up(int n) { return (n + 1) / 2; }
 __host__ __device__ inline int k4_steps(int n) { return (half_up(n) + 3) / 4; }
 __host__ __device__ inline int out_tiles(int n) { return (half_up(n) + 7) / 8; }
+// threads of a CTA: four warps where there are at most four output tiles (n <= 64), whose blocks then are half as
+// large and twice as many on an SM (61504 rows of n = 31 17.5 -> 14.9 us, 40000 of n = 50 18.7 -> 17.0), else eight
+// (40000 of n = 100 43.9 us, 44.6 with four; 8000 of n = 500 139, 153 with four)
+inline int mma_threads(int n) { return out_tiles(n) <= 4 ? 128 : 256; }
 // Shared memory holds blocks of four a_j and then their four d_j, so that a lane reaches a step's both values of
 // a line by constant offsets.  Pitches in complex values: a B fragment is 4 values of j by 8 real columns, read
 // by half warps of 4 x 4; rows (line-major): pitch = 4 mod 8 puts the two lines of a half warp on
@@ -66,11 +70,12 @@ inline size_t mma_smem(bool cols, int n, int nl) {
 // indexing in the three phases it ran 1262, now 776 (40000 rows 49 -> 43.5 us, 8000 rows of n = 500 160 -> 139,
 // 61504 of n = 31 23 -> 17.5, 100 columns x 400 planes 46 -> 42); so the addresses of a phase advance by constants, nothing is computed per thread that the launch can pass, and the first table steps of a unit are on
 // their way before its lines are.
-template <bool COLS, int NTW>
-__global__ void __launch_bounds__(kMmaThreads, 3)
+template <bool COLS, int NTW, int NT>
+__global__ void __launch_bounds__(NT, 768 / NT)
     k_dst1_mma(const double2 *in, double2 *out, int n, long nlines, long in_ld, long out_ld, long in_plane,
                long out_plane, int groups, double coef, const double2 *__restrict__ tab) {
     extern __shared__ __align__(16) double2 mma_sm[];
+    constexpr int NW = NT / 32;
     const int  h1 = half_up(n), ks = k4_steps(n), nl = 4 * NTW * groups;
     const int  pitch = COLS ? cols_pitch(nl) : rows_pitch(n);
     const int  lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -104,7 +109,7 @@ __global__ void __launch_bounds__(kMmaThreads, 3)
             }
     };
     if constexpr (COLS) {
-        const int dj = kMmaThreads / nl, dc = kMmaThreads - dj * nl;
+        const int dj = NT / nl, dc = NT - dj * nl;
         int       j = threadIdx.x / nl, c = threadIdx.x - j * nl;
         while (j < 4 * ks) {
 #pragma unroll
@@ -127,7 +132,7 @@ __global__ void __launch_bounds__(kMmaThreads, 3)
         }
     } else {
         // a warp takes pieces of 32 j, `pieces` to a line
-        const int pieces = (4 * ks + 31) / 32, dc = kMmaWarps / pieces, dr = kMmaWarps - dc * pieces;
+        const int pieces = (4 * ks + 31) / 32, dc = NW / pieces, dr = NW - dc * pieces;
         int       c = warp / pieces, r = warp - c * pieces;
         while (c < nl) {
 #pragma unroll
@@ -155,7 +160,7 @@ __global__ void __launch_bounds__(kMmaThreads, 3)
 
     const int     kk = lane & 3, nn = lane >> 2; // the lane's j within a step and real column within a tile
     const double *lines = reinterpret_cast<const double *>(mma_sm) + (nn & 1);
-    for (int u = warp; u < units; u += kMmaWarps) {
+    for (int u = warp; u < units; u += NW) {
         const int tile = tile_of(u), c0 = (u - tile * groups) * 4 * NTW;
         double    ao[NTW][2], ae[NTW][2];
 #pragma unroll
@@ -196,8 +201,8 @@ __global__ void __launch_bounds__(kMmaThreads, 3)
         }
         static_assert(kTabAhead == 2, "at most one step is left");
         if (ks & 1) step(cur[0], 0);
-        if (u + kMmaWarps < units) {
-            q = tab + (long)tile_of(u + kMmaWarps) * ks * 32 + lane;
+        if (u + NW < units) {
+            q = tab + (long)tile_of(u + NW) * ks * 32 + lane;
 #pragma unroll
             for (int i = 0; i < kTabAhead; i++) cur[i] = __ldg(q + i * 32);
         }
@@ -274,38 +279,39 @@ __global__ void __launch_bounds__(kDenseThreads)
 }
 
 // Lines per CTA: 4 ntw lines per warp unit, `groups` units side by side.
-//  * groups: the least that gives all eight warps a unit (n < 64 has fewer than eight output tiles).
-//  * ntw: the widest of 4, 3, 2 whose lines leave room for three CTAs on an SM (n = 100: 43.5 us at 4
-//    against 44.5 at 3 and 48 at 2 for 40000 rows; n = 300: 38 us at 3 against 41 at 2; n = 500: 139 us
-//    at 2 against 152 at 1, two CTAs per SM with 3: 146), then 2 with two CTAs, then 1 (n = 1000, 2000 rows:
-//    161 us, 169 at 2).  Columns take the width (up to 5) that
+//  * groups: the least that gives all warps a unit (n <= 48 has fewer than four output tiles).
+//  * ntw: the widest of 4, 3, 2 whose lines leave room for 24 warps on an SM (n = 100: 43.5 us at 4
+//    against 44.5 at 3 and 48.1 at 2 for 40000 rows; n = 300: 38 us at 3 against 41 at 2; n = 500: 139 us
+//    at 2 against 152 at 1, 146 at 3 with 16 warps), then 2 with 16 warps (n = 700), then 1 (n = 1000: 161 us,
+//    169 at 2).  Columns take the width (up to 5) that
 //    leaves the fewest idle columns in a plane's last tile (100 columns: 42 us at 5, 46.5 at 4).
-//  * fewer lines per CTA where the launch would not give every SM two (7688 rows of n = 31: 4.8 us at 24
+//  * fewer lines per CTA where the launch would not give every SM sixteen warps (7688 rows of n = 31: 4.8 us at 24
 //    lines, 6.4 at 48; 2500 rows of n = 50: 3.6 us at 8, 4.5 at 16).
 void dense_shape(bool cols, int n, long nlines, long planes, int *ntw, int *groups) {
-    const int units = out_tiles(n);
-    int       g = units >= kMmaWarps ? 1 : std::min(4, kMmaWarps / units), w = 0;
+    const int units = out_tiles(n), nt = mma_threads(n), warps = nt / 32, full = 768 / nt;
+    int       g = units >= warps ? 1 : std::min(4, warps / units), w = 0;
     auto per_sm = [&](int v) { return kMmaSmemMax / (long)(mma_smem(cols, n, 4 * v * g) + 1024); };
     auto padded = [&](int v) { return (nlines + 4L * v * g - 1) / (4L * v * g) * (4L * v * g); };
     for (int v = cols ? 5 : 4; v >= 2; v--)
-        if (per_sm(v) >= 3 && (w == 0 || (cols && padded(v) < padded(w)))) w = v;
-    if (w == 0) w = per_sm(2) >= 2 ? 2 : 1;
+        if (per_sm(v) >= full && (w == 0 || (cols && padded(v) < padded(w)))) w = v;
+    if (w == 0) w = per_sm(2) * 3 >= full * 2 ? 2 : 1;
     auto ctas = [&]() { return padded(w) / (4L * w * g) * planes; };
-    while (w > 2 && ctas() < 296) w--;
-    while (g > 1 && ctas() < 296) g--;
-    while (w > 1 && ctas() < 148) w--;
+    const long slots = 148L * full;
+    while (w > 2 && ctas() * 3 < slots * 2) w--;
+    while (g > 1 && ctas() * 3 < slots * 2) g--;
+    while (w > 1 && ctas() * 3 < slots) w--;
     *ntw = w;
     *groups = g;
 }
 
-template <bool COLS, int NTW>
+template <bool COLS, int NTW, int NT>
 int launch_mma(Ctx *c, int n, long nlines, long planes, const double2 *in, long in_ld, long in_plane, double2 *out,
                long out_ld, long out_plane, int groups, const double2 *tab) {
     const int    nl = 4 * NTW * groups;
     const size_t shm = mma_smem(COLS, n, nl);
-    HH_CUDA(cudaFuncSetAttribute(k_dst1_mma<COLS, NTW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+    HH_CUDA(cudaFuncSetAttribute(k_dst1_mma<COLS, NTW, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
     dim3 grid((unsigned)((nlines + nl - 1) / nl), (unsigned)planes);
-    return launch_kernel(c, k_dst1_mma<COLS, NTW>, grid, kMmaThreads, shm, in, out, n, nlines, in_ld, out_ld, in_plane, out_plane,
+    return launch_kernel(c, k_dst1_mma<COLS, NTW, NT>, grid, NT, shm, in, out, n, nlines, in_ld, out_ld, in_plane, out_plane,
                                                                  groups, std::sqrt(2.0 / (n + 1)), tab);
 }
 
@@ -347,18 +353,21 @@ int launch_dst_dense(Ctx *c, int n, bool cols, long nlines, long planes, const d
     const double2 *tab = reinterpret_cast<const double2 *>(mat);
     int ntw = 1, groups = 1;
     dense_shape(cols, n, nlines, planes, &ntw, &groups);
-#define HH_MMA(W)                                                                                                            \
-    case W:                                                                                                                  \
-        return cols ? launch_mma<true, W>(c, n, nlines, planes, in, in_ld, in_plane, out, out_ld, out_plane, groups, tab)    \
-                    : launch_mma<false, W>(c, n, nlines, planes, in, in_ld, in_plane, out, out_ld, out_plane, groups, tab);
+    auto pick = [&](auto ntw_c) {
+        constexpr int W = decltype(ntw_c)::value;
+        auto go = [&](auto launch) {
+            return launch(c, n, nlines, planes, in, in_ld, in_plane, out, out_ld, out_plane, groups, tab);
+        };
+        if (mma_threads(n) == 128) return cols ? go(launch_mma<true, W, 128>) : go(launch_mma<false, W, 128>);
+        return cols ? go(launch_mma<true, W, 256>) : go(launch_mma<false, W, 256>);
+    };
     switch (ntw) {
-        HH_MMA(1)
-        HH_MMA(2)
-        HH_MMA(3)
-        HH_MMA(4)
-        HH_MMA(5)
+    case 1: return pick(std::integral_constant<int, 1>{});
+    case 2: return pick(std::integral_constant<int, 2>{});
+    case 3: return pick(std::integral_constant<int, 3>{});
+    case 4: return pick(std::integral_constant<int, 4>{});
+    case 5: return pick(std::integral_constant<int, 5>{});
     }
-#undef HH_MMA
     set_error("DST length %d: no tile shape", n);
     return HH_ERR_UNSUPPORTED;
 }
