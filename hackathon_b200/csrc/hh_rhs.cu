@@ -102,27 +102,33 @@ __device__ __forceinline__ double2 pade_rhs(const PadeJob &J, int c1, int c2, in
 }
 
 // The two sweeps of one segment of `top` <= 8 points; V(m) is v at the segment's point m, W points reached on
-// either side, put(m, value) takes the results.
-template <int W, typename Val, typename Put>
-__device__ __forceinline__ void pade_segment(Val V, int top, const PadeJob &J, Put put) {
+// either side, put(m, value) takes the results in order.
+template <int W, bool FULL, typename Val, typename Put>
+__device__ __forceinline__ void pade_sweeps(Val V, int top, const PadeJob &J, Put put) {
     const double r = J.r;
     double2 B = make_double2(0.0, 0.0), F = B, Bn[kSegP];
 #pragma unroll
     for (int m = kSegP + W - 1; m >= 0; m--) {
         if (m < kSegP) Bn[m] = B;
-        if (m < top + W) B = zaxpy_r(V(m), -r, B);
+        if (FULL || m < top + W) B = zaxpy_r(V(m), -r, B);
     }
 #pragma unroll
     for (int m = -W; m < 0; m++) F = zaxpy_r(V(m), -r, F);
 #pragma unroll
     for (int m = 0; m < kSegP; m++) {
-        if (m < top) {
+        if (FULL || m < top) {
             const double2 vm = V(m);
             const double2 u = zaxpy_r(vm, -r, make_double2(F.x + Bn[m].x, F.y + Bn[m].y));
             put(m, make_double2(fma(u.x, J.scale, u.x * J.scale_lo), fma(u.y, J.scale, u.y * J.scale_lo)));
             F = zaxpy_r(vm, -r, F);
         }
     }
+}
+
+template <int W, typename Val, typename Put>
+__device__ __forceinline__ void pade_segment(Val V, int top, const PadeJob &J, Put put) {
+    if (top == kSegP) pade_sweeps<W, true>(V, top, J, put);
+    else pade_sweeps<W, false>(V, top, J, put);
 }
 
 // One block: the values of f that its span reaches come in with asynchronous copies, v is formed from them
@@ -140,25 +146,31 @@ template <int W> __device__ __forceinline__ void pade_block(const PadeJob &J, un
         const bool in = c < J.n1;
         {
             const double2 *f = J.f + J.f0 - J.fa + (in ? c : 0) * J.f1 + c2 * J.f2;
-            for (int e = e0 + (t >> 5); e <= e1; e += kPadeThreads / 32)
-                pade_async16(sm + (e - e0) * 32 + cc, f + (long)e * J.fa);
+            const long     step = (kPadeThreads / 32) * J.fa;
+            int            e = e0 + (t >> 5);
+            f += e * J.fa;
+            for (double2 *to = sm + t; e <= e1; e += kPadeThreads / 32, f += step, to += kPadeThreads) pade_async16(to, f);
         }
         pade_async_wait();
         __syncthreads();
-        constexpr int NV = (kSpanS + 2 * W + 7) / 8;
-        double2       vv[NV];
+        constexpr int  NV = (kSpanS + 2 * W + 7) / 8;
+        double2        vv[NV];
+        const double2 *at0 = sm + (m0 - W - e0) * 32 + t; // f left of point m0 - W + (t >> 5)
 #pragma unroll
         for (int i = 0; i < NV; i++) {
-            const int r = (t >> 5) + 8 * i;
+            const int r = (t >> 5) + 8 * i, m = m0 - W + r;
             vv[i] = zero;
-            if (in && r < len)
-                vv[i] = pade_rhs<W, FIRST>(J, c, c2, m0 - W + r, [&](int e) { return sm[(e - e0) * 32 + cc]; });
+            if (in && r < len) {
+                const double2 *l = at0 + 256 * i;
+                if (m >= 1 && m <= J.n - 2) vv[i] = pade_diff<FIRST>(l[0], l[32], l[64]); // no end near: the same difference
+                else vv[i] = pade_rhs<W, FIRST>(J, c, c2, m, [&](int e) { return sm[(e - e0) * 32 + cc]; });
+            }
         }
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < NV; i++) {
             const int r = (t >> 5) + 8 * i;
-            if (r < len) sm[r * 32 + cc] = vv[i];
+            if (r < len) sm[t + 256 * i] = vv[i];
         }
         __syncthreads();
         const int i0 = (t >> 5) * kSegP; // the thread's first point within the span
@@ -166,7 +178,10 @@ template <int W> __device__ __forceinline__ void pade_block(const PadeJob &J, un
         const double2 *v = sm + (i0 + W) * 32 + cc;
         double2       *o = J.out + c + c2 * J.o2 + (long)(m0 + i0) * J.oa;
         pade_segment<W>([&](int m) { return v[m * 32]; }, min(kSegP, span - i0), J,
-                        [&](int m, double2 u) { o[m * J.oa] = u; });
+                        [&](int, double2 u) {
+                            *o = u;
+                            o += J.oa;
+                        });
     } else {
         // kRowsX neighbouring rows, kSpanX points: tiles [row][point + point / 8] (the segments of 8 start on
         // different banks)
@@ -187,30 +202,34 @@ template <int W> __device__ __forceinline__ void pade_block(const PadeJob &J, un
         }
         pade_async_wait();
         __syncthreads();
-        constexpr int NV = (kSpanX + 2 * W + 15) / 16;
-        double2       vv[NV];
+        constexpr int  NV = (kSpanX + 2 * W + 15) / 16;
+        double2        vv[NV];
+        const int      p0 = m0 - W - e0 + k; // f left of point m0 - W + k; at(p + 16 i) = at(p) + 18 i
+        const double2 *lo = row + at(p0), *mi = row + at(p0 + 1), *hi = row + at(p0 + 2);
 #pragma unroll
         for (int i = 0; i < NV; i++) {
-            const int e = k + 16 * i;
+            const int e = k + 16 * i, m = m0 - W + e;
             vv[i] = zero;
-            if (in && e < len)
-                vv[i] = pade_rhs<W, FIRST>(J, c1, c2, m0 - W + e, [&](int y) { return row[at(y - e0)]; });
+            if (in && e < len) {
+                if (m >= 1 && m <= J.n - 2) vv[i] = pade_diff<FIRST>(lo[18 * i], mi[18 * i], hi[18 * i]);
+                else vv[i] = pade_rhs<W, FIRST>(J, c1, c2, m, [&](int y) { return row[at(y - e0)]; });
+            }
         }
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < NV; i++) {
             const int e = k + 16 * i;
-            if (e < len) row[at(e)] = vv[i];
+            if (e < len) row[at(k) + 18 * i] = vv[i];
         }
         __syncthreads();
         const int i0 = k * kSegP, top = in ? max(0, min(kSegP, span - i0)) : 0;
         double2   u[kSegP];
-        if (top > 0)
-            pade_segment<W>([&](int m) { return row[at(i0 + W + m)]; }, top, J, [&](int m, double2 x) { u[m] = x; });
+        if (top > 0) // at(8 k + W + m) = 9 k + at(W + m)
+            pade_segment<W>([&](int m) { return row[9 * k + at(W + m)]; }, top, J, [&](int m, double2 x) { u[m] = x; });
         __syncthreads(); // the tile takes the results, for contiguous stores
 #pragma unroll
         for (int m = 0; m < kSegP; m++)
-            if (m < top) row[at(i0 + m)] = u[m];
+            if (m < top) row[9 * k + m] = u[m];
         __syncthreads();
         if (in) {
             double2 *o = J.out + c1 * J.o1 + c2 * J.o2 + m0;
@@ -219,8 +238,10 @@ template <int W> __device__ __forceinline__ void pade_block(const PadeJob &J, un
     }
 }
 
-// Bound by instruction issue and shared memory: a point costs 1.5 to 2 values of v and a segment of 8 points
-// 2 (W + 8) steps of one fused multiply-add per component.  All derivatives of an assembly share one launch.
+// Bound by shared memory (56 % of its wavefronts) and instruction issue: a point costs 1.5 to 2 values of v and a
+// segment of 8 points 2 (W + 8) steps of one fused multiply-add per component.  Points with no end near take the
+// plain difference at constant offsets: 33.7 -> 25.7 million warp instructions at 125^3, assembly and solve of 2D
+// 511^2 51.1 -> 50.0 us, of 3D 125^3 255 -> 253.  All derivatives of an assembly share one launch.
 __global__ void __launch_bounds__(kPadeThreads, 3) k_pade(const __grid_constant__ PadeJobs jobs) {
     extern __shared__ __align__(16) double2 pade_sm[];
     unsigned blk = blockIdx.x;
