@@ -108,8 +108,8 @@ struct SymParams {
 };
 
 // TMA-tile input of the symmetric line solve: one right-hand side of the CTA's CW lines arrives
-// as a tile [rows][CW] in shared memory, brought by tensor copies over a (re/im, line, row,
-// right-hand side) map in boxes of br rows, NBUF right-hand sides ahead.  Thread 0 issues the
+// as a tile [rows][CW] in shared memory, brought by tensor copies over a (double of a
+// row, row, right-hand side) map in boxes of br rows, NBUF right-hand sides ahead.  Thread 0 issues the
 // copies; the outputs are stored from registers as in the per-thread prefetch form.
 template <int SRC, typename MT> struct SymTileBufs {
     static constexpr int value = SRC == 6 && !is_real_v<MT> ? 1 : 2; // complex order 6 spends the space on its pivots
