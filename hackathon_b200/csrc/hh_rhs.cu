@@ -344,15 +344,14 @@ struct Rhs3DArgs {
 // 0), layer nz-1 with the super-diagonal one (ap..dp of nz-1).  fxx on the y and z faces, fyy on the x
 // and z faces and fzz on the x and y faces are zero, as the reference leaves them.
 //
-// A thread marches through kZRun layers of its (i, j) with the layers below, at and above in registers, the
+// A thread marches through RUN layers of its (i, j) with the layers below, at and above in registers, the
 // one after those on its way: each field crosses L2 once instead of three times.
-constexpr int kZRun = 16;
-__global__ void __launch_bounds__(256) k_rhs3d_combine(const __grid_constant__ Rhs3DArgs A) {
+template <int RUN> __global__ void __launch_bounds__(256) k_rhs3d_combine(const __grid_constant__ Rhs3DArgs A) {
     const int i = blockIdx.x * 32 + (threadIdx.x & 31), j = blockIdx.y * 8 + (threadIdx.x >> 5);
     pdl_wait();
     pdl_next();
     if (i >= A.nx || j >= A.ny) return;
-    const int     nx = A.nx, ny = A.ny, nz = A.nz, l0 = blockIdx.z * kZRun, l1 = min(nz, l0 + kZRun);
+    const int     nx = A.nx, ny = A.ny, nz = A.nz, l0 = blockIdx.z * RUN, l1 = min(nz, l0 + RUN);
     const long    Ex = nx + 2, Ey = ny + 2, Exy = Ex * Ey, nxy = (long)nx * ny;
     const double2 zero = make_double2(0.0, 0.0);
     const bool    six = A.order == 6;
@@ -677,8 +676,17 @@ int assemble_rhs3d(Plan *p, const hh_rhs3d_data *d, double2 *rhs) {
         set_error("hh_rhs3d: %d x %d x %d is too large", nx, ny, nz);
         return HH_ERR_UNSUPPORTED;
     }
-    dim3 grid((unsigned)((nx + 31) / 32), (unsigned)((ny + 7) / 8), (unsigned)((nz + kZRun - 1) / kZRun));
-    return launch_kernel(c, k_rhs3d_combine, grid, 256, 0, A);
+    // Layers per block: 16, or 8 or 4 where the blocks are then still all resident at once (two to an SM), so that a
+    // small problem does not march through 16 layers on a part of the chip.  Assembly and solve against 16: 31^3
+    // 47.0 -> 43.0 us, 48^3 54.2 -> 43.5, 63^3 65.5 -> 53.8.
+    // As a kernel argument the run cost 2.5 % at 125^3; 32 layers in one wave were slower (127^3 238 -> 253 us).
+    const long bx = (nx + 31) / 32, by = (ny + 7) / 8;
+    auto       go = [&](auto kernel, int run) {
+        return launch_kernel(c, kernel, dim3((unsigned)bx, (unsigned)by, (unsigned)((nz + run - 1) / run)), 256, 0, A);
+    };
+    if (bx * by * ((nz + 3) / 4) <= 2 * 148) return go(k_rhs3d_combine<4>, 4);
+    if (bx * by * ((nz + 7) / 8) <= 2 * 148) return go(k_rhs3d_combine<8>, 8);
+    return go(k_rhs3d_combine<16>, 16);
 }
 
 } // namespace hh

@@ -224,7 +224,7 @@ def test_rhs2d_segment_and_tile_edges(ctx, oracle, n):
     plan.close()
 
 
-@pytest.mark.parametrize("nx,ny,nz", [(3, 4, 5), (16, 65, 8), (129, 7, 33), (31, 130, 66)])
+@pytest.mark.parametrize("nx,ny,nz", [(3, 4, 5), (16, 65, 8), (129, 7, 33), (31, 130, 66), (97, 96, 40)])
 def test_rhs3d_segment_and_tile_edges(ctx, oracle, nx, ny, nz):
     rng = np.random.default_rng(nx + ny + nz)
     hx, hy, hz = 1.0 / (nx + 1), 0.9 / (ny + 1), 1.1 / (nz + 1)
