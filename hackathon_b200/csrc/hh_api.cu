@@ -59,16 +59,19 @@ int cuda_fail(cudaError_t e, const char *what, const char *file, int line) {
     return e == cudaErrorMemoryAllocation ? HH_ERR_NOMEM : HH_ERR_CUDA;
 }
 
-bool may_start_early(Ctx *c) {
-    const bool fresh = c->fresh;
-    c->fresh = false;
-    if (fresh || c->pool) return false;
+bool capturing(Ctx *c) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return true;
     }
-    return cap == cudaStreamCaptureStatusNone;
+    return cap != cudaStreamCaptureStatusNone;
+}
+
+bool may_start_early(Ctx *c) {
+    const bool fresh = c->fresh;
+    c->fresh = false;
+    return !fresh && !c->pool && !capturing(c);
 }
 
 static int upload(Ctx *c, void *dst, const void *src, size_t bytes) {
@@ -985,12 +988,7 @@ static void acquire_work(Plan &p, int batch, int src_order, double2 **work, long
     const long   pitch = (p.nx + 7) / 8 * 8;
     const size_t bytes = sizeof(double2) * (size_t)pitch * (size_t)p.ny * (size_t)(p.dim == 3 ? p.nz : 1) * (size_t)batch;
     if (bytes < 2 * c->l2_bytes || bytes > kWorkKeep) return;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess) {
-        cudaGetLastError();
-        return;
-    }
-    if (cap != cudaStreamCaptureStatusNone) return;
+    if (capturing(c)) return;
     cudaMemPool_t pool = work_pool_of(c);
     if (!pool) return;
     void *w = nullptr;
@@ -1266,7 +1264,7 @@ extern "C" int hh_solve_source(hh_plan *pl, const double *f, double *u, int batc
 // plan i taking nrhs[i] consecutive fields of f and u.  The transforms do not depend on k, so each
 // direction is one launch over the whole batch; the line solves are one launch with a table of
 // which right-hand sides use which plan's factors (or one launch per plan where the plans do not
-// share a symmetric kernel variant).  table: device memory for that table (nullptr: the context's
+// share a symmetric kernel variant, and in a stream capture whose table would not fit the kernel's arguments).  table: device memory for that table (nullptr: the context's
 // own, grown on demand, which orders the solve behind earlier work on the context's stream).
 int hh::solve_source_multi(Plan *const *plans, const int *nrhs, int nplans, const double2 *f, double2 *u,
                            void *table) {

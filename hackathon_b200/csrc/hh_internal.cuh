@@ -114,6 +114,9 @@ struct Ctx {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Whether the context's stream is in a capture (or may be: its state cannot be read)
+bool capturing(Ctx *c);
+
 // Whether the next launch on the context's stream may start early: not the first after the tables, a plan or
 // the stream changed (its set-up reads them), not on the request loop's contexts (plans are set up on other
 // streams there), not in a stream capture (graphs keep plain kernel dependencies).
@@ -213,7 +216,8 @@ int launch_lines_pack(Ctx *c, const double2 *in, double2 *out, long batch, long 
                       bool unpack);
 // one symmetric line-solve launch over several plans of one shape (plan i: nrhs[i] consecutive
 // fields); table_dev holds line_solve_multi_table_bytes(nplans, total) bytes; HH_ERR_UNSUPPORTED
-// (nothing launched) when the plans do not all take the same symmetric kernel variant
+// (nothing launched) when the plans do not all take the same symmetric kernel variant, or when a table too large
+// for the kernel's arguments would be copied inside a stream capture
 size_t line_solve_multi_table_bytes(int nplans, int total);
 int launch_line_solve_multi(Plan *const *plans, const int *nrhs, int nplans, const double2 *in, double2 *out,
                             int src_order, void *table_dev);

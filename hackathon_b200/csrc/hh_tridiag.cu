@@ -733,8 +733,9 @@ size_t line_solve_multi_table_bytes(int nplans, int total) {
 // One symmetric line-solve launch over the right-hand sides of several plans of one shape: plan i
 // solves nrhs[i] consecutive fields of the batch (plans in order).  Every plan must take the
 // symmetric kernel with the same variant; table_dev (line_solve_multi_table_bytes) receives the
-// plan references and the chunk table in stream order.  Returns HH_ERR_UNSUPPORTED when the plans
-// do not qualify, before launching anything.
+// plan references and the chunk table in stream order, where they do not fit the kernel's arguments.  Returns
+// HH_ERR_UNSUPPORTED when the plans do not qualify, before launching anything; so too for a device table inside a
+// stream capture, which would record the address of the host tables freed on return instead of their contents.
 int launch_line_solve_multi(Plan *const *plans, const int *nrhs, int nplans, const double2 *in, double2 *out,
                             int src_order, void *table_dev) {
     Plan *p0 = plans[0];
@@ -774,6 +775,9 @@ int launch_line_solve_multi(Plan *const *plans, const int *nrhs, int nplans, con
     if (nplans <= SymMulti::kPlans && chunks.size() <= (size_t)SymMulti::kChunks) {
         std::copy(refs.begin(), refs.end(), m.iref);
         std::copy(chunks.begin(), chunks.end(), m.ichunk);
+    } else if (capturing(p0->ctx)) {
+        set_error("multi-plan line solve: %d plans in %zu chunks in a stream capture", nplans, chunks.size());
+        return HH_ERR_UNSUPPORTED;
     } else {
         char *tab = static_cast<char *>(table_dev);
         HH_CUDA(cudaMemcpyAsync(tab, refs.data(), sizeof(SymPlanRef) * refs.size(), cudaMemcpyHostToDevice, p0->ctx->stream));
