@@ -251,6 +251,7 @@ __global__ void k_make_dense(int n, double *mat) {
 // One line per CTA against the full matrix, for the lines too long for k_dst1_mma.  The matrix is
 // symmetric: thread k walks column k, so that a warp reads neighbouring values.
 constexpr int kDenseThreads = 128;
+constexpr int kDenseMaxN = 4096; // the longest line the transforms accept here
 template <bool STRIDED>
 __global__ void __launch_bounds__(kDenseThreads)
     k_dst1_dense(const double2 *__restrict__ in, double2 *__restrict__ out, int n, long in_ld, long out_ld,
@@ -309,7 +310,7 @@ int launch_mma(Ctx *c, int n, long nlines, long planes, const double2 *in, long 
                long out_ld, long out_plane, int groups, const double2 *tab) {
     const int    nl = 4 * NTW * groups;
     const size_t shm = mma_smem(COLS, n, nl);
-    HH_CUDA(cudaFuncSetAttribute(k_dst1_mma<COLS, NTW, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+    HH_TRY(allow_smem(k_dst1_mma<COLS, NTW, NT>, kMmaSmemMax));
     dim3 grid((unsigned)((nlines + nl - 1) / nl), (unsigned)planes);
     return launch_kernel(c, k_dst1_mma<COLS, NTW, NT>, grid, NT, shm, in, out, n, nlines, in_ld, out_ld, in_plane, out_plane,
                                                                  groups, std::sqrt(2.0 / (n + 1)), tab);
@@ -346,7 +347,7 @@ int launch_dst_dense(Ctx *c, int n, bool cols, long nlines, long planes, const d
     if (n > kMmaMaxN) {
         const size_t shm = sizeof(double2) * (size_t)n;
         auto         kern = cols ? k_dst1_dense<true> : k_dst1_dense<false>;
-        HH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+        HH_TRY(allow_smem(kern, sizeof(double2) * kDenseMaxN));
         dim3 grid((unsigned)nlines, (unsigned)planes);
         return launch_kernel(c, kern, grid, kDenseThreads, shm, in, out, n, in_ld, out_ld, in_plane, out_plane, mat);
     }

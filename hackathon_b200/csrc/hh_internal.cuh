@@ -122,6 +122,14 @@ bool capturing(Ctx *c);
 // streams there), not in a stream capture (graphs keep plain kernel dependencies).
 bool may_start_early(Ctx *c);
 
+// Lets `kern` use up to `most` bytes of dynamic shared memory.  The limit belongs to the function and the device, not to
+// the launch: contexts of different threads share it, so every caller of a kernel passes the same `most` (the largest
+// that any size needs); a limit set to each launch's own need would fail a larger launch of another thread.
+template <typename... P> int allow_smem(void (*kern)(P...), size_t most) {
+    HH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    return HH_OK;
+}
+
 template <typename... P, typename... A>
 int launch_kernel(Ctx *c, void (*kern)(P...), dim3 grid, int threads, size_t smem, A &&...args) {
     cudaLaunchConfig_t cfg{};

@@ -809,15 +809,17 @@ static int launch_sym_t(Plan *p, const double2 *in, double2 *out, int batch, con
     sp.pu = p->pade_u;
     double cz = 1.0;
     for (int k = 0; k < 16; k++) sp.cz[k] = cz *= -p->pade_linf;
-    const int io_elems = TIO ? sym_tile_elems(p->rows, CW) * SymTileBufs<SRC, MT>::value : NR * (KS + 2) * NT;
-    const int shm = 128 + (int)(sizeof(double2) * io_elems +
-                                sizeof(MT) * (2 * (LOG + 1) * NT + (SymUIS<SRC, KS, MT>::value ? KS * NT : 0) +
-                                              (SymPCS<SRC, KS, CW, MT>::value ? 5 * NT : 0)) +
-                                (SRC == 6 ? sizeof(double) * 2 * (LOG + 1) * NT : 0));
+    auto smem = [](int rows) {
+        const int io_elems = TIO ? sym_tile_elems(rows, CW) * SymTileBufs<SRC, MT>::value : NR * (KS + 2) * NT;
+        return 128 + (int)(sizeof(double2) * io_elems +
+                           sizeof(MT) * (2 * (LOG + 1) * NT + (SymUIS<SRC, KS, MT>::value ? KS * NT : 0) +
+                                         (SymPCS<SRC, KS, CW, MT>::value ? 5 * NT : 0)) +
+                           (SRC == 6 ? sizeof(double) * 2 * (LOG + 1) * NT : 0));
+    };
+    const int shm = smem(p->rows);
     CUtensorMap in_map{};
     if constexpr (TIO) HH_TRY(encode_line_map(&in_map, in, p, batch, CW, sym_tile_rows_per_box(p->rows)));
-    HH_CUDA(cudaFuncSetAttribute(k_line_solve_sym<SRC, NT, CW, MINB, NR, KS, TIO, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 shm));
+    HH_TRY(allow_smem(k_line_solve_sym<SRC, NT, CW, MINB, NR, KS, TIO, MT>, smem(NT / CW * KS))); // (NT / CW segments a line)
     const long groups = (p->span() + CW - 1) / CW;
     int blocks_per_sm = 0, dev = 0, sms = 148;
     HH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, k_line_solve_sym<SRC, NT, CW, MINB, NR, KS, TIO, MT>, NT,

@@ -532,20 +532,23 @@ static PadeJob pade_job(const double2 *f, double2 *out, const double *bc, int n,
     return J;
 }
 
+static size_t pade_smem(bool xdir, int w) {
+    return sizeof(double2) * (xdir ? (size_t)kRowsX * ((kSpanX + 2 * w + 2) * 9 / 8 + 1) : (size_t)(kSpanS + 2 * w + 2) * 32);
+}
+
 static int launch_pade(Ctx *c, const PadeJobs &jobs) {
     long   blocks = 0;
     size_t shm = 0;
     for (int i = 0; i < jobs.count; i++) {
         const PadeJob &J = jobs.j[i];
         blocks += J.blocks;
-        shm = std::max(shm, sizeof(double2) * (J.xdir ? (size_t)kRowsX * ((kSpanX + 2 * J.w + 2) * 9 / 8 + 1)
-                                                      : (size_t)(kSpanS + 2 * J.w + 2) * 32));
+        shm = std::max(shm, pade_smem(J.xdir, J.w));
     }
     if (blocks > 0x7fffffffL) {
         set_error("right-hand side: grid too large");
         return HH_ERR_UNSUPPORTED;
     }
-    HH_CUDA(cudaFuncSetAttribute(k_pade, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+    HH_TRY(allow_smem(k_pade, std::max(pade_smem(true, kReach4), pade_smem(false, kReach4))));
     return launch_kernel(c, k_pade, dim3((unsigned)blocks), kPadeThreads, shm, jobs);
 }
 
