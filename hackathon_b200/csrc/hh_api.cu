@@ -931,11 +931,13 @@ static int transform_inverse(Plan &p, double2 *in, double2 *out, int batch, bool
 // pass gain nothing (1023^2 x 8: 193 us either way), so the line is at twice the L2.  The arithmetic, and so every
 // bit, is the same.
 //  * The workspace is allocated and freed in stream order from one pool per device, shared by the contexts on it
-//    and destroyed with the last of them, which keeps at most kWorkKeep bytes between solves; a solve that
-//    would need more, or cannot get it, runs in place in the output as smaller ones do.
+//    and destroyed with the last of them, which never holds more than kWorkKeep bytes, however many streams solve
+//    at once; a solve that cannot get its part of them runs in place in the output as smaller ones do.  What the
+//    pool holds between solves goes to another allocation of the process that would fail without it
+//    (the driver releases it: a cudaMalloc of all free memory and half of what was held succeeds).
 //  * In place as well: solves under stream capture (a graph's own allocations would restrict it), the request
 //    loop's (its budget does not know the workspace) and the host-buffer forms (bound by their copies).
-constexpr size_t kWorkKeep = 4ULL << 30;
+constexpr size_t kWorkKeep = 4ULL << 30; // the pool's size, and what it keeps between solves
 struct WorkPool {
     cudaMemPool_t pool = nullptr;
     int           users = 0;
@@ -952,6 +954,7 @@ static cudaMemPool_t work_pool_of(Ctx *c) {
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = c->device;
+        props.maxSize = kWorkKeep;
         uint64_t keep = kWorkKeep;
         int      off = 0; // solves on different streams never wait for each other's workspace
         if (cudaMemPoolCreate(&w.pool, &props) != cudaSuccess ||

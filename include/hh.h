@@ -177,7 +177,13 @@ int  hh_plan_set_rows_variant(hh_plan *plan, int variant);
 int  hh_plan_rows_variant(const hh_plan *plan);
 
 /* Solve A u = rhs for `batch` assembled right-hand sides (the reference's solver(System),
- * 2D_Program/solver_functions/solver.c:14, 3D_Program/solver_functions/solver.c:263). */
+ * 2D_Program/solver_functions/solver.c:14, 3D_Program/solver_functions/solver.c:263).
+ * Memory of the device-buffer solves (this one, hh_solve_source, hh_solve_source_multi): with an odd
+ * row length and fields of twice the L2 up to 4 GB they take a workspace of about the fields' size, in
+ * stream order, from a pool of at most 4 GB per device that the contexts on it share and the last of
+ * them destroys; without room for it, and in a stream capture, they work in sol_dev alone.  What
+ * the pool holds between solves is released to a cudaMalloc of the process that needs it.  The
+ * result does not depend on the workspace. */
 int hh_solve(hh_plan *plan, const double *rhs_dev, double *sol_dev, int batch);
 /* Same with host buffers: host-to-device copy, solve, device-to-host copy on the plan's stream. */
 int hh_solve_host(hh_plan *plan, const double *rhs_host, double *sol_host, int batch);

@@ -132,3 +132,39 @@ def test_padded_workspace_shared_and_given_back():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", _SHARED], cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "shared ok" in r.stdout, r.stdout + r.stderr
+
+
+_MANY = """
+import torch
+import hackathon_b200 as hh
+n, batch, count = 1023, 64, 7
+streams = [torch.cuda.Stream() for _ in range(count)]
+g = torch.Generator(device="cuda").manual_seed(11)
+f = torch.view_as_complex(torch.randn((batch, n, n, 2), dtype=torch.float64, device="cuda", generator=g))
+u = [torch.empty_like(f) for _ in range(count)]
+ctxs = [hh.Context(0, s.cuda_stream) for s in streams]
+plans = [hh.Plan.helmholtz(c, 2, n, 6, 30.0) for c in ctxs]
+for p, c in zip(plans, ctxs):  # each kernel is loaded, no workspace taken yet
+    p.solve_source(f, u[0], 1)
+    c.synchronize()
+free0 = low = torch.cuda.mem_get_info()[0]
+for _ in range(3):
+    for p, y in zip(plans, u):
+        p.solve_source(f, y, batch)
+    low = min(low, torch.cuda.mem_get_info()[0])
+for c in ctxs:
+    c.synchronize()
+torch.cuda.synchronize()
+assert all(torch.equal(y, u[0]) for y in u[1:])
+used = free0 - low
+assert (1 << 30) - (1 << 25) <= used <= (4 << 30) + (1 << 27), used
+print("many ok", used)
+"""
+
+
+def test_padded_workspace_is_bounded_over_streams():
+    """Seven streams solving 1 GB batches at once hold at most the pool's 4 GB between them (and 128 MB for
+    what else the driver may take); those that get no workspace run in place, with the same bits."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _MANY], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "many ok" in r.stdout, r.stdout + r.stderr
