@@ -433,7 +433,7 @@ template <int M> struct WCfg;
 // kernel (2: the next line loads while one is transformed; 1: more warps per SM instead), MINB
 // CTAs per SM the register budget is sized for; CWPC warps per CTA and CNT tiles per warp in the
 // columns kernel (CNT - 1 tiles load while one is transformed); RING: the rows use the CTA-ring
-// kernel with RWPC warps per CTA: 0 never, 1 always, 2 from ring_lines() lines on
+// kernel with RWPC warps per CTA: 0 never, 1 always, 2 as ring_by_lines() says
 template <> struct WCfg<1024> { static constexpr int TL = 32, R = 32, WPC = 2, NBUF = 2, MINB = 3, CWPC = 2, CNT = 2, RWPC = 4, RING = 1; };
 template <> struct WCfg<512>  { static constexpr int TL = 16, R = 32, WPC = 2, NBUF = 2, MINB = 3, CWPC = 2, CNT = 2, RWPC = 4, RING = 2; };
 template <> struct WCfg<256>  { static constexpr int TL = 16, R = 16, WPC = 4, NBUF = 2, MINB = 3, CWPC = 4, CNT = 2, RWPC = 4, RING = 0; };
@@ -1611,21 +1611,27 @@ template <int M, bool LP, bool UPD = false> static int launch_w2(Ctx *c, const D
                                                                         c->err_word);
 }
 
-// The ring's CTAs hold RWPC line groups and stand two on an SM, the per-warp kernel's hold two: with fewer lines
-// than give every SM one ring CTA, the smaller CTAs spread better.  511^2, whole solves, per-warp -> ring:
-// 1 right-hand side (511 lines) 20.6 -> 22.4 us, 2 24.7 -> 28.5, 4 (2044 lines) 35.5 -> 31.9, 32 176.5 -> 162.8;
-// the rows transform of 128: 230 -> 197 us.
-template <int M> static long ring_lines() {
+// The ring takes 2368 lines of 511 at a time (two CTAs of four two-line groups on each of 148 SMs), the per-warp
+// kernel 1776 (three of two).  A pass over as many lines costs the per-warp kernel less, so the ring is the better one
+// where it needs fewer passes, or as many (but not one) with its last hardly begun.  511^2, whole solves of assembled
+// right-hand sides, per-warp -> ring:
+//   1 right-hand side (511 lines) 16.6 -> 19.3 us, 3 (1533) 26.7 -> 31.3, 4 (2044) 33.2 -> 31.1, 5 (2555) 46.0 -> 44.7,
+//   6 (3066) 46.0 -> 47.8, 8 54.7 -> 50.9, 10 (5110) 63.9 -> 66.0, 12 77.2 -> 75.7, 16 99.4 -> 95.8, 32 190 -> 176.5;
+//   1776 lines 35.4 -> 38.8, 1900 41.1 -> 39.6, 2369 55.0 -> 52.7, 2664 42.3 -> 41.5, 3552 48.2 -> 51.5.
+// From 5329 lines on the ring always needs fewer.
+template <int M> static bool ring_by_lines(long lines) {
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         sms = 148;
-    return (long)sms * WCfg<M>::RWPC * WGeom<M>::LPW; // 1184 lines of 511
+    const long ring = 2L * sms * WCfg<M>::RWPC * WGeom<M>::LPW, warp = (long)WCfg<M>::MINB * sms * WCfg<M>::WPC * WGeom<M>::LPW;
+    const long rp = (lines + ring - 1) / ring, wp = (lines + warp - 1) / warp;
+    return rp < wp || (rp == wp && rp > 1 && lines - (rp - 1) * ring < ring / 8);
 }
 
 // rows kernel: a.rows_kernel 1 = the CTA ring, 2 = per-warp buffers, 0 = the length's default
 template <int M, bool LP, bool UPD = false> static int launch_w(Ctx *c, const DstArgs &a) {
     const bool ring = a.rows_kernel ? a.rows_kernel == 1
-                                    : WCfg<M>::RING == 1 || (WCfg<M>::RING == 2 && a.nlines * a.planes >= ring_lines<M>());
+                                    : WCfg<M>::RING == 1 || (WCfg<M>::RING == 2 && ring_by_lines<M>(a.nlines * a.planes));
     return ring ? launch_wr<M, LP, UPD>(c, a) : launch_wp<M, LP, UPD>(c, a);
 }
 
