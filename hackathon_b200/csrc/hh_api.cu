@@ -204,6 +204,7 @@ extern "C" int hh_ctx_inject_wait_expiry(hh_ctx *x) {
     const int one = 1;
     HH_CUDA(cudaMemcpyAsync(x->c.inject_word, &one, sizeof(int), cudaMemcpyHostToDevice, x->c.stream));
     HH_CUDA(cudaStreamSynchronize(x->c.stream));
+    x->c.inject_armed = true;
     return HH_OK;
 }
 

@@ -1589,6 +1589,7 @@ template <int M, bool LP, bool UPD = false> static int launch_wp(Ctx *c, const D
     HH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dst1_w<M, LP, UPD>, 32 * G::WPC, G::SMEM));
     const long groups = (a.nlines * a.planes + G::LPW - 1) / G::LPW;
     const long ctas = std::min<long>((groups + G::WPC - 1) / G::WPC, (long)std::max(1, per_sm) * sms);
+    c->inject_armed = false;
     return launch_kernel(c, k_dst1_w<M, LP, UPD>, dim3((unsigned)ctas), 32 * G::WPC, G::SMEM, a.in, a.out, a.nlines, a.planes, a.in_ld, a.out_ld,
                                                                      a.in_plane, a.out_plane, tw, sn, c->err_word,
                                                                      c->inject_word);
@@ -1628,10 +1629,11 @@ template <int M> static bool ring_by_lines(long lines) {
     return rp < wp || (rp == wp && rp > 1 && lines - (rp - 1) * ring < ring / 8);
 }
 
-// rows kernel: a.rows_kernel 1 = the CTA ring, 2 = per-warp buffers, 0 = the length's default
+// rows kernel: a.rows_kernel 1 = the CTA ring, 2 = per-warp buffers, 0 = the length's default (the per-warp kernel,
+// which the failure injection lives in, also where the rule would take the ring while an injection is armed)
 template <int M, bool LP, bool UPD = false> static int launch_w(Ctx *c, const DstArgs &a) {
     const bool ring = a.rows_kernel ? a.rows_kernel == 1
-                                    : WCfg<M>::RING == 1 || (WCfg<M>::RING == 2 && ring_by_lines<M>(a.nlines * a.planes));
+                                    : WCfg<M>::RING == 1 || (WCfg<M>::RING == 2 && !c->inject_armed && ring_by_lines<M>(a.nlines * a.planes));
     return ring ? launch_wr<M, LP, UPD>(c, a) : launch_wp<M, LP, UPD>(c, a);
 }
 

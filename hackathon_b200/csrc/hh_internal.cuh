@@ -9,6 +9,7 @@
 #include <stdint.h>
 #include <stddef.h>
 
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <string>
@@ -74,6 +75,7 @@ struct Ctx {
     long long                launches = 0;       // kernels launched through this context
     int                     *err_word = nullptr; // set by kernels whose bounded waits expire
     int                     *inject_word = nullptr; // armed by hh_ctx_inject_wait_expiry, taken by one launch
+    std::atomic<bool>        inject_armed{false};   // since it was armed no launch has looked at inject_word
     size_t                   l2_bytes = 0;        // the device's L2 size (3D transform slabs)
     std::string              dev_name;            // the device's model name (tuning-cache key)
     // stage timing (hh_ctx_set_stage_timing)

@@ -559,9 +559,10 @@ extern "C" int hh_server_inject_wait_expiry(hh_server *s) {
     }
     // the dispatcher owns the context's stream: write the word synchronously instead
     const int one = 1;
+    hh::Ctx    *cx = reinterpret_cast<hh::Ctx *>(s->ctx); // Ctx is hh_ctx's first member
     cudaError_t e = cudaSetDevice(s->device);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(reinterpret_cast<hh::Ctx *>(s->ctx)->inject_word, &one, sizeof(int), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(cx->inject_word, &one, sizeof(int), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) cx->inject_armed = true;
     if (e != cudaSuccess) {
         set_error("hh_server_inject_wait_expiry: %s", cudaGetErrorString(e));
         return HH_ERR_CUDA;

@@ -31,6 +31,20 @@ def test_expired_wait_is_reported_and_the_context_recovers(ctx, oracle):
     assert rel_err(dst.cpu().numpy(), oracle.dst1_rows(x)) < 1e-13
 
 
+@pytest.mark.parametrize("n,rows", [(511, 4), (511, 4088), (63, 20000)])
+def test_expired_wait_at_every_row_count(ctx, n, rows):
+    """The rows transforms of n + 1 = 64 .. 512 take the injection whatever number of rows they get (511 has another
+    kernel for many of them)."""
+    x = torch.zeros((rows, n), dtype=torch.complex128, device="cuda")
+    torch.cuda.synchronize()
+    ctx.inject_wait_expiry()
+    ctx.dst1_rows(n, rows, x, x)
+    with pytest.raises(hh.HHError, match="HH_ERR_DEVICE"):
+        ctx.synchronize()
+    ctx.dst1_rows(n, rows, x, x)
+    ctx.synchronize()
+
+
 def test_expired_wait_fails_its_request_in_the_loop(ctx):
     # the loop's plans take the tuning cache's settings; without an entry they keep the length's
     # default rows kernel, which is the one the injection is armed in
