@@ -666,9 +666,12 @@ static int tune_measure(hh_plan *pl, int batch) {
     p.variant = best;
     // the rows transform: the CTA ring or per-warp line buffers (lengths n + 1 = 64 .. 1024), the
     // two-warp line kernel or the Stockham kernel (2048), timed as one forward and one inverse
-    // transform of the batch
+    // transform of the batch.  Where the faster of the two depends on the number of rows, the plan keeps the rule
+    // that goes by it (0): a choice made at this batch would hold for every other.
     const int mx = p.nx + 1;
-    if (rc == HH_OK && mx >= 64 && mx <= 2048 && (mx & (mx - 1)) == 0) {
+    if (rows_kernel_by_lines(p.nx)) {
+        p.rows_kernel = 0;
+    } else if (rc == HH_OK && mx >= 64 && mx <= 2048 && (mx & (mx - 1)) == 0) {
         int   best_rk = p.rows_kernel;
         float best_t = 1e30f;
         for (int rk = 1; rk <= 2 && rc == HH_OK; rk++) {

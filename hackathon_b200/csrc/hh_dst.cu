@@ -1687,6 +1687,8 @@ template <bool IS, bool OS, bool LP = false, bool UPD = false> static int launch
     return launch_dst_dense(c, n, IS, a.nlines, a.planes, a.in, a.in_ld, a.in_plane, a.out, a.out_ld, a.out_plane);
 }
 
+bool rows_kernel_by_lines(int n) { return n + 1 == 512 && WCfg<512>::RING == 2; }
+
 bool rows_update_supported(int n, int rows_kernel) {
     const int m = n + 1;
     return (m >= 64 && m <= 1024 && (m & (m - 1)) == 0) || (m == 2048 && rows_kernel != 2);

@@ -214,6 +214,7 @@ int launch_dst_rows(Ctx *c, int n, long rows, const double2 *in, long in_ld, dou
 // `out` (out <- out - DST(in)), for the lengths rows_update_supported admits (n + 1 = 64 .. 1024,
 // and 2048 unless rows_kernel is 2); HH_ERR_UNSUPPORTED, before any launch, otherwise.
 bool rows_update_supported(int n, int rows_kernel);
+bool rows_kernel_by_lines(int n); // the default rows kernel of length n goes by the number of rows
 int  launch_dst_rows_update(Ctx *c, int n, long rows, const double2 *in, long in_ld, double2 *out, long out_ld,
                             int rows_kernel);
 // kern: 0 = CTA tiles of 8 swizzled columns where the length allows, 1 = per-warp tiles of LPW columns

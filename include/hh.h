@@ -172,7 +172,8 @@ int  hh_plan_dst_variant(const hh_plan *plan);
  * tickets ahead into it), 2 per-warp double buffers, 0 (the default) the length's own choice (the
  * ring at n + 1 = 1024, by the number of rows at 512, else per-warp buffers).  The result does not depend on it.  At n + 1 = 2048: 0 and 1 two warps
  * per line (in a CTA ring), 2 the Stockham kernel of the longer lengths; the two agree to
- * rounding.  hh_plan_tune times both choices for every plan of these lengths. */
+ * rounding.  hh_plan_tune times both choices for the plans of these lengths, but for n + 1 = 512, where it
+ * keeps 0. */
 int  hh_plan_set_rows_variant(hh_plan *plan, int variant);
 int  hh_plan_rows_variant(const hh_plan *plan);
 

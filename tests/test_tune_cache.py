@@ -55,3 +55,20 @@ def test_cache_hit_skips_timing(ctx, tmp_path):
     for p in (a, b, c):
         p.close()
     hh.tune_cache_clear()
+
+
+@pytest.mark.gpu
+def test_tuning_keeps_the_rule_by_rows_at_511(ctx, tmp_path):
+    """At n + 1 = 512 the faster rows kernel depends on the number of rows, so tuning at one batch must not
+    settle it for every other: the plan and the cache entry keep the default."""
+    hh.tune_cache_clear()
+    plan = hh.Plan.helmholtz(ctx, 2, 511, 4, 20.0)
+    plan.rows_variant = 2
+    plan.tune(8)
+    assert plan.rows_variant == 0
+    path = tmp_path / "tune.txt"
+    hh.tune_cache_save(str(path))
+    entry = [x for x in path.read_text().splitlines() if not x.startswith("#")]
+    assert len(entry) == 1 and entry[0].split("\t")[-1] == "0"
+    plan.close()
+    hh.tune_cache_clear()
