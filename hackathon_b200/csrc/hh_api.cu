@@ -628,114 +628,104 @@ extern "C" int hh_plan_variant(const hh_plan *pl) { return pl ? pl->p.variant : 
 static int transform_forward(Plan &p, const double2 *in, double2 *out, int batch, bool lp = false, long ld = 0);
 static int transform_inverse(Plan &p, double2 *in, double2 *out, int batch, bool lp = false, long ld = 0);
 
+static void acquire_work(Plan &p, int batch, int src_order, double2 **work, long *ld);
+static Plan padded_plan(const Plan &p, long ld);
+
 // Times every line-solve variant on `batch` zero right-hand sides (the solve does the same work
-// for any values) and keeps the fastest.  Blocks; must not run inside a stream capture.
+// for any values) and keeps the fastest, then the transforms' kernels; each where a solve of this batch keeps the
+// transformed field (in place or in the padded workspace, whose aligned rows rank the kernels differently: 3D
+// 255^3 x 4 at order 6 the rows kernels are even in place and 2264 against 2213 us a solve padded).
+// Blocks; must not run inside a stream capture.
 static int tune_measure(hh_plan *pl, int batch) {
     Plan &p = pl->p;
     Ctx  *c = p.ctx;
     HH_CUDA(cudaSetDevice(c->device));
-    double2 *buf = nullptr;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    int rc = HH_OK, best = p.variant;
-    float best_ms = 1e30f;
-    const int src = p.src_order;
-    auto run = [&]() -> int {
-        if (cudaMalloc(&buf, sizeof(double2) * (size_t)p.field * batch) != cudaSuccess ||
-            cudaMemsetAsync(buf, 0, sizeof(double2) * (size_t)p.field * batch, c->stream) != cudaSuccess ||
+    const size_t bytes = sizeof(double2) * (size_t)p.field * batch;
+    const int    src = p.src_order;
+    double2     *buf = nullptr;
+    cudaEvent_t  e0 = nullptr, e1 = nullptr;
+    // the time of three passes over the field, after a warm-up
+    auto timed = [&](float *ms, auto pass) -> int {
+        double2 *work = nullptr;
+        long     ld = p.nx;
+        acquire_work(p, batch, src, &work, &ld);
+        auto run = [&]() -> int {
+            if (work) HH_CUDA(cudaMemsetAsync(work, 0, bytes / p.nx * ld, c->stream));
+            for (int r = 0; r < 4; r++) {
+                if (r == 1) HH_CUDA(cudaEventRecord(e0, c->stream));
+                HH_TRY(pass(work ? work : buf, ld));
+            }
+            HH_CUDA(cudaEventRecord(e1, c->stream));
+            HH_CUDA(cudaEventSynchronize(e1));
+            HH_CUDA(cudaEventElapsedTime(ms, e0, e1));
+            return HH_OK;
+        };
+        const int rc = run();
+        if (work) cudaFreeAsync(work, c->stream);
+        return rc;
+    };
+    auto transforms = [&](double2 *w, long ld) -> int { // one forward and one inverse transform of the batch
+        HH_TRY(transform_forward(p, buf, w, batch, false, ld));
+        return transform_inverse(p, w, buf, batch, false, ld);
+    };
+    auto measure = [&]() -> int {
+        if (cudaMalloc(&buf, bytes) != cudaSuccess || cudaMemsetAsync(buf, 0, bytes, c->stream) != cudaSuccess ||
             cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) {
             set_error("hh_plan_tune: %s", cudaGetErrorString(cudaGetLastError()));
             return HH_ERR_CUDA;
         }
-        for (int v = 0; v < solve_variant_count(); v++) {
+        float ms = 0.f, best_ms = 1e30f;
+        int   best = p.variant, rc = HH_OK;
+        for (int v = 0; v < solve_variant_count() && rc == HH_OK; v++) {
             p.variant = v;
-            HH_TRY(launch_line_solve(&p, buf, buf, batch, src)); // warm-up
-            HH_CUDA(cudaEventRecord(e0, c->stream));
-            for (int r = 0; r < 3; r++) HH_TRY(launch_line_solve(&p, buf, buf, batch, src));
-            HH_CUDA(cudaEventRecord(e1, c->stream));
-            HH_CUDA(cudaEventSynchronize(e1));
-            float ms = 0.f;
-            HH_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-            if (ms < best_ms) {
-                best_ms = ms;
-                best = v;
-            }
+            rc = timed(&ms, [&](double2 *w, long ld) -> int {
+                Plan q = ld == p.nx ? p : padded_plan(p, ld);
+                return launch_line_solve(&q, w, w, batch, src);
+            });
+            if (rc == HH_OK && ms < best_ms) best_ms = ms, best = v;
         }
-        return HH_OK;
+        p.variant = best;
+        HH_TRY(rc);
+        // the rows transform: the CTA ring or per-warp line buffers (lengths n + 1 = 64 .. 1024), the
+        // two-warp line kernel or the Stockham kernel (2048).  Where the faster of the two depends on the number
+        // of rows, the plan keeps the rule that goes by it (0): a choice made at this batch would hold for
+        // every other.
+        const int mx = p.nx + 1;
+        if (rows_kernel_by_lines(p.nx)) {
+            p.rows_kernel = 0;
+        } else if (mx >= 64 && mx <= 2048 && (mx & (mx - 1)) == 0) {
+            best = p.rows_kernel, best_ms = 1e30f;
+            for (int rk = 1; rk <= 2 && rc == HH_OK; rk++) {
+                p.rows_kernel = rk;
+                rc = timed(&ms, transforms);
+                if (rc == HH_OK && ms < best_ms) best_ms = ms, best = rk;
+            }
+            p.rows_kernel = best;
+            HH_TRY(rc);
+        }
+        // 3D plans: the columns kernel and the slab of the transform passes, over candidates from a sixteenth of
+        // L2 to the whole batch
+        if (p.dim == 3) {
+            const long planes = (long)p.nz * batch, plane_bytes = 16L * p.nx * p.ny;
+            std::vector<long> cand = {planes};
+            for (long div : {16L, 8L, 4L, 3L, 2L}) {
+                const long sp = std::max(1L, (long)(c->l2_bytes / div) / plane_bytes);
+                if (sp < planes && std::find(cand.begin(), cand.end(), sp) == cand.end()) cand.push_back(sp);
+            }
+            long best_slab = p.slab;
+            best = p.col_kernel, best_ms = 1e30f;
+            for (int trial = 0; trial < 2 * (int)cand.size() && rc == HH_OK; trial++) {
+                p.slab = cand[(size_t)trial / 2];
+                p.col_kernel = trial % 2;
+                rc = timed(&ms, transforms);
+                if (rc == HH_OK && ms < best_ms) best_ms = ms, best = p.col_kernel, best_slab = p.slab;
+            }
+            p.slab = best_slab;
+            p.col_kernel = best;
+        }
+        return rc;
     };
-    rc = run();
-    p.variant = best;
-    // the rows transform: the CTA ring or per-warp line buffers (lengths n + 1 = 64 .. 1024), the
-    // two-warp line kernel or the Stockham kernel (2048), timed as one forward and one inverse
-    // transform of the batch.  Where the faster of the two depends on the number of rows, the plan keeps the rule
-    // that goes by it (0): a choice made at this batch would hold for every other.
-    const int mx = p.nx + 1;
-    if (rows_kernel_by_lines(p.nx)) {
-        p.rows_kernel = 0;
-    } else if (rc == HH_OK && mx >= 64 && mx <= 2048 && (mx & (mx - 1)) == 0) {
-        int   best_rk = p.rows_kernel;
-        float best_t = 1e30f;
-        for (int rk = 1; rk <= 2 && rc == HH_OK; rk++) {
-            p.rows_kernel = rk;
-            auto pass = [&]() -> int {
-                HH_TRY(transform_forward(p, buf, buf, batch));
-                return transform_inverse(p, buf, buf, batch);
-            };
-            if ((rc = pass()) != HH_OK) break;
-            if (cudaEventRecord(e0, c->stream) != cudaSuccess) { rc = HH_ERR_CUDA; break; }
-            for (int r = 0; r < 3 && rc == HH_OK; r++) rc = pass();
-            if (rc != HH_OK) break;
-            float ms = 0.f;
-            if (cudaEventRecord(e1, c->stream) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
-                cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) {
-                rc = HH_ERR_CUDA;
-                break;
-            }
-            if (ms < best_t) {
-                best_t = ms;
-                best_rk = rk;
-            }
-        }
-        p.rows_kernel = best_rk;
-    }
-    // 3D plans: the slab of the transform passes, over candidates from a sixteenth of L2 to the
-    // whole batch, timed as one forward and one inverse transform
-    if (rc == HH_OK && p.dim == 3) {
-        const long planes = (long)p.nz * batch, plane_bytes = 16L * p.nx * p.ny;
-        std::vector<long> cand = {planes};
-        for (long div : {16L, 8L, 4L, 3L, 2L}) {
-            const long sp = std::max(1L, (long)(c->l2_bytes / div) / plane_bytes);
-            if (sp < planes && std::find(cand.begin(), cand.end(), sp) == cand.end()) cand.push_back(sp);
-        }
-        long  best_slab = p.slab;
-        int   best_ck = p.col_kernel;
-        float best_t = 1e30f;
-        for (int trial = 0; trial < 2 * (int)cand.size(); trial++) {
-            const long sp = cand[(size_t)trial / 2];
-            p.slab = sp;
-            p.col_kernel = trial % 2;
-            auto pass = [&]() -> int {
-                HH_TRY(transform_forward(p, buf, buf, batch));
-                return transform_inverse(p, buf, buf, batch);
-            };
-            if ((rc = pass()) != HH_OK) break;
-            if (cudaEventRecord(e0, c->stream) != cudaSuccess) { rc = HH_ERR_CUDA; break; }
-            for (int r = 0; r < 3 && rc == HH_OK; r++) rc = pass();
-            if (rc != HH_OK) break;
-            float ms = 0.f;
-            if (cudaEventRecord(e1, c->stream) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
-                cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) {
-                rc = HH_ERR_CUDA;
-                break;
-            }
-            if (ms < best_t) {
-                best_t = ms;
-                best_slab = sp;
-                best_ck = p.col_kernel;
-            }
-        }
-        p.slab = best_slab;
-        p.col_kernel = best_ck;
-    }
+    int rc = measure();
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     if (buf) {

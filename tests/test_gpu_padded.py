@@ -168,3 +168,28 @@ def test_padded_workspace_is_bounded_over_streams():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", _MANY], cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "many ok" in r.stdout, r.stdout + r.stderr
+
+
+_TUNED = """
+import torch
+import hackathon_b200 as hh
+n, batch = 1023, 17
+torch.zeros(1, device="cuda")
+ctx = hh.Context(0, 1)
+plan = hh.Plan.helmholtz(ctx, 2, n, 6, 30.0)
+plan.tune(8)  # a batch that solves in place: the kernels are loaded, no workspace taken yet
+hh.tune_cache_clear()
+torch.cuda.synchronize()
+free0 = torch.cuda.mem_get_info()[0]
+plan.tune(batch)
+held = free0 - torch.cuda.mem_get_info()[0]
+assert held >= batch * 1024 * n * 16, held
+print("tuned ok")
+"""
+
+
+def test_tuning_times_the_layout_that_solves_use():
+    """Tuning at a batch whose solves take the padded workspace takes it too (the pool keeps it)."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _TUNED], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "tuned ok" in r.stdout, r.stdout + r.stderr
