@@ -1088,16 +1088,18 @@ extern "C" int hh_solve_lines(hh_plan *pl, const double *in, double *out, int ba
     return hh_solve_lines_strided(pl, in, out, batch, fused, pl->p.row_stride, pl->p.field);
 }
 
-// One solve: forward transforms, the line solves given by `lines(plan, field)`, inverse transforms, in the output
-// buffer or (padded) in a workspace.
-template <typename Lines>
-static int solve_passes(Plan &p, const double2 *in, double2 *out, int batch, int src_order, bool may_pad, Lines lines) {
+// One solve: forward transforms, the line solves given by `lines(field, row pitch)`, inverse transforms, in the output
+// buffer or (padded) in a workspace.  `before(row pitch)` runs before anything is queued.
+template <typename Before, typename Lines>
+static int solve_passes(Plan &p, const double2 *in, double2 *out, int batch, int src_order, bool may_pad, Before before,
+                        Lines lines) {
     Ctx     *c = p.ctx;
     double2 *work = nullptr;
     long     ld = p.nx;
     if (may_pad) acquire_work(p, batch, src_order, &work, &ld);
     double2 *w = work ? work : out;
     auto     passes = [&]() -> int {
+        HH_TRY(before(ld));
         HH_TRY(stage_mark(*c, 0));
         HH_TRY(transform_forward(p, in, w, batch, false, ld));
         HH_TRY(stage_mark(*c, 1));
@@ -1117,7 +1119,8 @@ static int solve_passes(Plan &p, const double2 *in, double2 *out, int batch, int
 static int solve_one(hh_plan *pl, const double *in, double *out, int batch, int src_order, bool may_pad) {
     Plan &p = pl->p;
     HH_CUDA(cudaSetDevice(p.ctx->device));
-    return solve_passes(p, (const double2 *)in, (double2 *)out, batch, src_order, may_pad, [&](double2 *w, long ld) -> int {
+    auto nothing = [](long) { return HH_OK; };
+    return solve_passes(p, (const double2 *)in, (double2 *)out, batch, src_order, may_pad, nothing, [&](double2 *w, long ld) -> int {
         if (ld == p.nx) return launch_line_solve(&p, w, w, batch, src_order);
         Plan q = padded_plan(p, ld);
         return launch_line_solve(&q, w, w, batch, src_order);
@@ -1270,26 +1273,13 @@ int hh::solve_source_multi(Plan *const *plans, const int *nrhs, int nplans, cons
     int   total = 0;
     for (int i = 0; i < nplans; i++) total += nrhs[i];
     if (total == 0) return HH_OK;
-    const bool own_table = !table;
     // the padded form needs the positions of lines, which every plan's line solve must know
-    bool may_pad = own_table;
+    bool may_pad = true;
     for (int i = 0; i < nplans; i++)
         may_pad = may_pad && (p0.dim == 2 || (plans[i]->variant >= 2 && sym_solve_supported(plans[i], p0.src_order)));
-    return solve_passes(p0, f, u, total, p0.src_order, may_pad, [&](double2 *w, long ld) -> int {
-        if (own_table) {
-            const size_t need = line_solve_multi_table_bytes(nplans, total);
-            if (c->multi_tab_bytes < need) {
-                HH_CUDA(cudaStreamSynchronize(c->stream));
-                cudaFree(c->multi_tab);
-                c->multi_tab = nullptr;
-                c->multi_tab_bytes = 0;
-                HH_CUDA(cudaMalloc(&c->multi_tab, need));
-                c->multi_tab_bytes = need;
-            }
-            table = c->multi_tab;
-        }
-        std::vector<Plan>   padded;
-        std::vector<Plan *> ps(plans, plans + nplans);
+    std::vector<Plan>   padded;
+    std::vector<Plan *> ps(plans, plans + nplans);
+    auto before = [&](long ld) -> int { // the plans over the field's layout, and the table where they need one
         if (ld != p0.nx) {
             padded.reserve((size_t)nplans);
             for (int i = 0; i < nplans; i++) {
@@ -1297,6 +1287,20 @@ int hh::solve_source_multi(Plan *const *plans, const int *nrhs, int nplans, cons
                 ps[(size_t)i] = &padded[(size_t)i];
             }
         }
+        if (table || nplans < 2 || capturing(c)) return HH_OK;
+        const size_t need = line_solve_multi_table_bytes(ps.data(), nrhs, nplans, p0.src_order);
+        if (c->multi_tab_bytes < need) {
+            HH_CUDA(cudaStreamSynchronize(c->stream));
+            cudaFree(c->multi_tab);
+            c->multi_tab = nullptr;
+            c->multi_tab_bytes = 0;
+            HH_CUDA(cudaMalloc(&c->multi_tab, need));
+            c->multi_tab_bytes = need;
+        }
+        if (need) table = c->multi_tab;
+        return HH_OK;
+    };
+    return solve_passes(p0, f, u, total, p0.src_order, may_pad, before, [&](double2 *w, long) -> int {
         int rc = nplans > 1 ? launch_line_solve_multi(ps.data(), nrhs, nplans, w, w, p0.src_order, table) : HH_ERR_UNSUPPORTED;
         if (rc == HH_ERR_UNSUPPORTED) { // one launch per plan
             rc = HH_OK;

@@ -226,10 +226,10 @@ int launch_line_solve(Plan *p, const double2 *in, double2 *out, int batch, int s
 int launch_lines_pack(Ctx *c, const double2 *in, double2 *out, long batch, long planes, long nlines, int world,
                       bool unpack);
 // one symmetric line-solve launch over several plans of one shape (plan i: nrhs[i] consecutive
-// fields); table_dev holds line_solve_multi_table_bytes(nplans, total) bytes; HH_ERR_UNSUPPORTED
+// fields); table_dev holds line_solve_multi_table_bytes (0: the table fits the kernel's arguments); HH_ERR_UNSUPPORTED
 // (nothing launched) when the plans do not all take the same symmetric kernel variant, or when a table too large
 // for the kernel's arguments would be copied inside a stream capture
-size_t line_solve_multi_table_bytes(int nplans, int total);
+size_t line_solve_multi_table_bytes(Plan *const *plans, const int *nrhs, int nplans, int src_order);
 int launch_line_solve_multi(Plan *const *plans, const int *nrhs, int nplans, const double2 *in, double2 *out,
                             int src_order, void *table_dev);
 // res = A_h u - rhs (FP64, zero Dirichlet ring); norms (optional, zeroed by the caller) receive
@@ -241,7 +241,7 @@ int read_device_error(Ctx *c, int *val);
 long slab_planes(const Plan &p, long planes); // 3D transform slab in planes (the plan's or the default)
 bool sym_solve_supported(const Plan *p, int src_order);
 // the fused-source solve of several plans of one shape in one pass (hh_solve_source_multi);
-// table: device memory of line_solve_multi_table_bytes, or nullptr for the context's own
+// table: device memory of line_solve_multi_table_bytes, or nullptr for the context's own (where one is needed)
 int solve_source_multi(Plan *const *plans, const int *nrhs, int nplans, const double2 *f, double2 *u, void *table);
 // the reference's rhs() on the device for plans of any stencil (hh_rhs2d / hh_rhs3d)
 int assemble_rhs2d(Plan *p, const hh_rhs2d_data *d, double2 *rhs);

@@ -209,10 +209,10 @@ int run_batch(hh_server *s, Batch *b, const std::vector<hh_plan *> &plans, cudaE
         cx->err_word = s->words + si; // the kernels of this batch report into its stream's word
         HH_CUDA(cudaMemsetAsync(cx->err_word, 0, sizeof(int), st));
         if (after) HH_CUDA(cudaStreamWaitEvent(st, after, 0)); // the plan's set-up
-        int total = 0;
-        for (Req *q : b->reqs) total += q->r.nrhs;
-        // the multi-plan chunk table of this batch, from the pool in stream order
-        HH_CUDA(cudaMallocFromPoolAsync(&tab, hh::line_solve_multi_table_bytes((int)ps.size(), total), s->pool, st));
+        // the multi-plan chunk table of this batch, where it needs one, from the pool in stream order
+        const size_t tab_bytes =
+            ps.size() > 1 ? hh::line_solve_multi_table_bytes(ps.data(), b->counts.data(), (int)ps.size(), r0.order) : 0;
+        if (tab_bytes) HH_CUDA(cudaMallocFromPoolAsync(&tab, tab_bytes, s->pool, st));
         if (b->staging == 0) { // straight from the caller's device buffers
             HH_TRY(hh::solve_source_multi(ps.data(), b->counts.data(), (int)ps.size(), (const double2 *)r0.f,
                                           (double2 *)r0.u, tab));
@@ -236,7 +236,7 @@ int run_batch(hh_server *s, Batch *b, const std::vector<hh_plan *> &plans, cudaE
             HH_CUDA(cudaFreeAsync(buf, st));
             buf = nullptr;
         }
-        HH_CUDA(cudaFreeAsync(tab, st));
+        if (tab) HH_CUDA(cudaFreeAsync(tab, st));
         tab = nullptr;
         if (inject) HH_CUDA(cudaMemsetAsync(cx->err_word, 1, 1, st)); // as if a wait had expired
         b->flag = s->flags + si;

@@ -726,31 +726,20 @@ int launch_line_solve_sym(Plan *p, const double2 *in, double2 *out, int batch, i
                         : launch_sym_cplx(p, in, out, batch, src_order, nullptr);
 }
 
-size_t line_solve_multi_table_bytes(int nplans, int total) {
-    return sizeof(SymPlanRef) * (size_t)nplans + sizeof(SymChunk) * (size_t)(total + nplans);
-}
-
-// One symmetric line-solve launch over the right-hand sides of several plans of one shape: plan i
-// solves nrhs[i] consecutive fields of the batch (plans in order).  Every plan must take the
-// symmetric kernel with the same variant; table_dev (line_solve_multi_table_bytes) receives the
-// plan references and the chunk table in stream order, where they do not fit the kernel's arguments.  Returns
-// HH_ERR_UNSUPPORTED when the plans do not qualify, before launching anything; so too for a device table inside a
-// stream capture, which would record the address of the host tables freed on return instead of their contents.
-int launch_line_solve_multi(Plan *const *plans, const int *nrhs, int nplans, const double2 *in, double2 *out,
-                            int src_order, void *table_dev) {
+// The chunks of right-hand sides of a multi-plan launch: the single-plan choice for the whole batch, chunks never
+// crossing a plan boundary.  HH_ERR_UNSUPPORTED when the plans do not all take one symmetric kernel.
+static int multi_chunks(Plan *const *plans, const int *nrhs, int nplans, int src_order, std::vector<SymChunk> *chunks) {
     Plan *p0 = plans[0];
+    int   total = 0;
     for (int i = 0; i < nplans; i++) {
         const Plan *pi = plans[i];
         if (pi->variant < 2 || pi->variant != p0->variant || !sym_solve_supported(pi, src_order)) {
             set_error("multi-plan line solve: plan %d does not take the symmetric kernel variant %d", i, p0->variant);
             return HH_ERR_UNSUPPORTED;
         }
+        total += nrhs[i];
     }
-    int total = 0;
-    for (int i = 0; i < nplans; i++) total += nrhs[i];
     if (total == 0) return HH_OK;
-    // right-hand sides per chunk: the single-plan choice for the whole batch, chunks never
-    // crossing a plan boundary
     const int ks = (p0->variant >= 5) ? 16 : kSeg;
     const int P = sym_segments(p0->rows, ks), CW = 256 / P, nr = (p0->variant == 4 && P > 8) ? 2 : 1;
     const long groups = (p0->span() + CW - 1) / CW;
@@ -758,25 +747,52 @@ int launch_line_solve_multi(Plan *const *plans, const int *nrhs, int nplans, con
     HH_CUDA(cudaGetDevice(&dev));
     HH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int rb = pick_rb(groups, total, (p0->variant == 2 ? 2 : 1) * sms, nr);
+    for (int i = 0, b = 0; i < nplans; b += nrhs[i], i++)
+        for (int b0 = b; b0 < b + nrhs[i]; b0 += rb) chunks->push_back(SymChunk{i, b0, std::min(b + nrhs[i], b0 + rb), 0});
+    if (chunks->size() > 65535) {
+        set_error("multi-plan line solve: %zu chunks", chunks->size());
+        return HH_ERR_UNSUPPORTED;
+    }
+    return HH_OK;
+}
+
+static bool multi_in_arguments(int nplans, size_t chunks) { return nplans <= SymMulti::kPlans && chunks <= (size_t)SymMulti::kChunks; }
+
+static size_t multi_table_bytes(int nplans, size_t chunks) { return sizeof(SymPlanRef) * (size_t)nplans + sizeof(SymChunk) * chunks; }
+
+size_t line_solve_multi_table_bytes(Plan *const *plans, const int *nrhs, int nplans, int src_order) {
+    std::vector<SymChunk> chunks;
+    if (multi_chunks(plans, nrhs, nplans, src_order, &chunks) != HH_OK || multi_in_arguments(nplans, chunks.size())) return 0;
+    return multi_table_bytes(nplans, chunks.size());
+}
+
+// One symmetric line-solve launch over the right-hand sides of several plans of one shape: plan i
+// solves nrhs[i] consecutive fields of the batch (plans in order).  Every plan must take the
+// symmetric kernel with the same variant; table_dev (line_solve_multi_table_bytes, nullptr where that is 0) receives
+// the plan references and the chunk table in stream order, where they do not fit the kernel's arguments.  Returns
+// HH_ERR_UNSUPPORTED when the plans do not qualify, before launching anything; so too for a device table inside a
+// stream capture, which would record the address of the host tables freed on return instead of their contents.
+int launch_line_solve_multi(Plan *const *plans, const int *nrhs, int nplans, const double2 *in, double2 *out,
+                            int src_order, void *table_dev) {
+    Plan *p0 = plans[0];
+    int   total = 0;
+    for (int i = 0; i < nplans; i++) total += nrhs[i];
+    std::vector<SymChunk> chunks;
+    HH_TRY(multi_chunks(plans, nrhs, nplans, src_order, &chunks));
+    if (total == 0) return HH_OK;
     std::vector<SymPlanRef> refs((size_t)nplans);
-    std::vector<SymChunk>   chunks;
-    for (int i = 0, b = 0; i < nplans; b += nrhs[i], i++) {
-        const Plan *pi = plans[i];
+    for (int i = 0; i < nplans; i++) {
+        const Plan  *pi = plans[i];
         const double h2 = pi->h * pi->h;
         refs[(size_t)i] = SymPlanRef{pi->Pv, pi->subt, pi->diagt, make_double2(pi->k2.x * h2 / 20.0, pi->k2.y * h2 / 20.0)};
-        for (int b0 = b; b0 < b + nrhs[i]; b0 += rb) chunks.push_back(SymChunk{i, b0, std::min(b + nrhs[i], b0 + rb), 0});
-    }
-    if (chunks.size() > 65535) {
-        set_error("multi-plan line solve: %zu chunks", chunks.size());
-        return HH_ERR_UNSUPPORTED;
     }
     SymMulti m;
     m.nchunks = (int)chunks.size();
-    if (nplans <= SymMulti::kPlans && chunks.size() <= (size_t)SymMulti::kChunks) {
+    if (multi_in_arguments(nplans, chunks.size())) {
         std::copy(refs.begin(), refs.end(), m.iref);
         std::copy(chunks.begin(), chunks.end(), m.ichunk);
-    } else if (capturing(p0->ctx)) {
-        set_error("multi-plan line solve: %d plans in %zu chunks in a stream capture", nplans, chunks.size());
+    } else if (!table_dev || capturing(p0->ctx)) {
+        set_error("multi-plan line solve: no table for %d plans in %zu chunks", nplans, chunks.size());
         return HH_ERR_UNSUPPORTED;
     } else {
         char *tab = static_cast<char *>(table_dev);

@@ -25,7 +25,7 @@ def _problem(stream, dim, n, order, nplans, counts):
 
 # 16 plans and 64 chunks (of one right-hand side each, at short lines) are the last that fit the arguments
 SHAPES = [(2, 63, 6, 16, [1] * 16), (2, 63, 6, 17, [1] * 17), (2, 255, 4, 40, [2, 1] * 20), (3, 31, 6, 17, [1] * 17),
-          (2, 63, 2, 2, [32, 32]), (2, 63, 2, 2, [33, 32])]
+          (2, 63, 2, 2, [32, 32]), (2, 63, 2, 2, [33, 32]), (2, 255, 4, 17, [16] * 17)]  # (the last: a padded workspace)
 
 
 @pytest.mark.parametrize("dim,n,order,nplans,counts", SHAPES)
@@ -47,5 +47,21 @@ def test_multi_in_a_capture_equals_solo_solves(dim, n, order, nplans, counts):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(u, solo)
+    del graph
+    ctx.close()
+
+
+def test_first_multi_solve_may_be_captured():
+    """Three plans need no device table, so a context's very first multi solve allocates nothing."""
+    stream = torch.cuda.Stream()
+    ctx, plans, f, solo = _problem(stream, 2, 127, 4, 3, [2, 1, 2])
+    u = torch.empty_like(f)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        hh.solve_source_multi(plans, [2, 1, 2], f, u)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(u, solo)
     del graph
     ctx.close()
