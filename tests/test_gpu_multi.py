@@ -1,5 +1,6 @@
 """hh_solve_source_multi past the plans (16) and chunks (64) whose table travels in the kernel's arguments: the
-table is copied to device memory, or, in a stream capture, the line solve goes plan by plan."""
+table is copied to device memory, or, in a stream capture, the line solve goes plan by plan.  The fields of every
+plan are bitwise its own solves."""
 import pytest
 
 import hackathon_b200 as hh
@@ -49,6 +50,44 @@ def test_multi_in_a_capture_equals_solo_solves(dim, n, order, nplans, counts):
         assert torch.equal(u, solo)
     del graph
     ctx.close()
+
+
+@pytest.mark.parametrize("dim,n,order,nplans,counts", SHAPES)
+def test_multi_equals_solo_solves(dim, n, order, nplans, counts):
+    """One call and one line-solve launch (the table in the arguments or in device memory), the solo solves' bits."""
+    ctx, plans, f, solo = _problem(torch.cuda.Stream(), dim, n, order, nplans, counts)
+    u = torch.full_like(f, float("nan"))
+    torch.cuda.synchronize()
+    before = ctx.launches
+    hh.solve_source_multi(plans, counts, f, u)
+    ctx.synchronize()
+    assert ctx.launches - before == (3 if dim == 2 else 5)
+    assert torch.equal(u, solo)
+    ctx.close()
+
+
+def test_request_loop_merges_more_plans_than_the_arguments_hold(ctx):
+    """Sixty requests of one shape, each at its own k, queued while the loop sets up: it merges batches of more than
+    16 plans, and every request gets its solo solve."""
+    hh.tune_cache_clear()
+    n = 63
+    ks = [1.0 + 0.6 * i for i in range(60)]
+    g = torch.Generator(device="cuda").manual_seed(8)
+    f = torch.view_as_complex(torch.randn((60, n, n, 2), dtype=torch.float64, device="cuda", generator=g))
+    u = torch.empty_like(f)
+    torch.cuda.synchronize()
+    srv = hh.Server(0, hbm_budget=4 << 30, streams=2)
+    ids = [srv.submit(2, n, 6, k, 1, f[i], u[i], on_device=True) for i, k in enumerate(ks)]
+    infos = [srv.wait(i) for i in ids]
+    srv.close()
+    assert max(i["batch_rhs"] for i in infos) > 16
+    for i, k in enumerate(ks):
+        plan = hh.Plan.helmholtz(ctx, 2, n, 6, k)
+        solo = torch.empty_like(f[i])
+        plan.solve_source(f[i], solo, 1)
+        ctx.synchronize()
+        assert torch.equal(u[i], solo)
+        plan.close()
 
 
 def test_first_multi_solve_may_be_captured():
