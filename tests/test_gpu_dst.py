@@ -253,3 +253,33 @@ def test_dst_any_length_tensor_core_tiles(ctx, n, rows, ncols, planes):
     o = _host(t)
     assert rel_err(o[..., :ncols], want(x[..., :ncols].transpose(0, 2, 1)).transpose(0, 2, 1)) < 1e-13
     assert np.array_equal(o[..., ncols], x[..., ncols])
+
+
+@pytest.mark.parametrize("n", [1000, 1201, 1500, 2399, 2400, 2401, 4000, 4094])
+@pytest.mark.parametrize("rows,ncols,planes", [(1, 1, 1), (37, 33, 2)])
+def test_dst_long_lengths_without_an_fft_kernel(ctx, n, rows, ncols, planes):
+    """The longest lines of the tensor-core products (one tile of four lines takes 225 KB at 2400) and the dense
+    kernel past them, rows and columns, in place and pitched, against numpy's FFT of the odd extension.  Sums of
+    at most n products of values of order 1: n eps."""
+    rng = np.random.default_rng(n + rows)
+    tol = n * 2.0 ** -52
+
+    def want(x):
+        z = np.zeros(x.shape[:-1] + (1,))
+        y = np.fft.fft(np.concatenate([z, x, z, -x[..., ::-1]], axis=-1), axis=-1)[..., 1:n + 1]
+        return y * 0.5j * np.sqrt(2.0 / (n + 1))
+
+    x = rng.standard_normal((rows, n + 3)) + 1j * rng.standard_normal((rows, n + 3))
+    t, o = _dev(x), torch.full((rows, n + 1), float("nan"), dtype=torch.complex128, device="cuda")
+    ctx.dst1_rows(n, rows, t, o, in_ld=n + 3, out_ld=n + 1)
+    ctx.dst1_rows(n, rows, t, t, in_ld=n + 3, out_ld=n + 3)
+    ctx.synchronize()
+    got, ref = _host(t), want(x[:, :n])
+    assert rel_err(got[:, :n], ref) < tol and np.array_equal(got[:, n:], x[:, n:])
+    assert np.array_equal(_host(o)[:, :n], got[:, :n]) and np.isnan(_host(o)[:, n]).all()
+    x = rng.standard_normal((planes, n, ncols + 2)) + 1j * rng.standard_normal((planes, n, ncols + 2))
+    t = _dev(x)
+    ctx.dst1_cols(n, ncols, planes, t, ncols + 2, n * (ncols + 2), t)
+    ctx.synchronize()
+    got, ref = _host(t), want(x[..., :ncols].transpose(0, 2, 1)).transpose(0, 2, 1)
+    assert rel_err(got[..., :ncols], ref) < tol and np.array_equal(got[..., ncols:], x[..., ncols:])
