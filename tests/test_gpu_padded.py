@@ -193,3 +193,48 @@ def test_tuning_times_the_layout_that_solves_use():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", _TUNED], cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "tuned ok" in r.stdout, r.stdout + r.stderr
+
+
+_WHICH = """
+import sys
+import torch
+import hackathon_b200 as hh
+torch.zeros(1, device="cuda")
+cases = [(3, 255, 6, 30.0, 1, 6, 1), (3, 255, 4, 30.0, 1, 2, 1), (3, 255, 6, 9 + 2j, 1, 5, 1), (3, 125, 6, 20.0, 9, 6, 1),
+         (3, 125, 2, 20.0, 9, 2, 1), (3, 125, 2, 20.0, 9, 0, 0), (2, 2047, 6, 100.0, 4, 6, 1), (2, 1023, 4, 50.0, 17, 3, 1),
+         (2, 1023, 6, 50 + 5j, 17, 6, 1), (2, 701, 6, 50.0, 35, 1, 1), (2, 1023, 4, 50.0, 12, 3, 0), (2, 500, 4, 20.0, 80, 6, 0)]
+for dim, n, order, k, batch, variant, padded in cases:
+    ctx = hh.Context(0, 1)
+    plan = hh.Plan.helmholtz(ctx, dim, n, order, k)
+    plan.variant = variant
+    f = torch.view_as_complex(torch.randn((batch,) + (n,) * dim + (2,), dtype=torch.float64, device="cuda"))
+    u, w = torch.empty_like(f), torch.empty_like(f)
+    for b in range(batch):  # one field at a time stays in place, but for one that is itself past the line
+        plan.solve_source(f[b], w[b], 1)
+    ctx.synchronize()
+    ctx.close()  # a workspace of these goes with the context
+    ctx = hh.Context(0, 1)
+    plan = hh.Plan.helmholtz(ctx, dim, n, order, k)
+    plan.variant = variant
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    plan.solve_source(f, u, batch)
+    ctx.synchronize()
+    held = free0 - torch.cuda.mem_get_info()[0]
+    size = batch * ((n + 7) // 8 * 8) * n ** (dim - 1) * 16
+    assert (held >= size) if padded else (held < size // 4), (dim, n, order, batch, variant, held, size)
+    assert torch.equal(u, w), (dim, n, order, batch, variant)
+    ctx.close()
+    del f, u, w
+    torch.cuda.empty_cache()
+print("which ok")
+"""
+
+
+def test_which_solves_take_the_workspace():
+    """What the pool holds after a solve says whether it was padded: the shapes above, the same shapes where the line
+    solve does not know the positions (3D, variant 0), below the size and with even rows; and for the batches whose
+    single fields stay in place, the padded bits against those."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _WHICH], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "which ok" in r.stdout, r.stdout + r.stderr

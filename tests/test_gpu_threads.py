@@ -40,7 +40,7 @@ static void *work(void *p) {
     d2.f_ext = d3.f_ext = d;
     d2.k_ext = d3.k2_ext = k;
     if (!ok) { j->bad = -1; printf("%s %d: %s\n", j->what, n, hh_last_error()); return NULL; }
-    for (int i = 0; i < 2000; i++) {
+    for (int i = 0; i < (n > 2400 ? 300 : 2000); i++) {
         int rc = three ? hh_rhs3d(pl, &d3, r) : rhs ? hh_rhs2d(pl, &d2, r) : tile ? hh_solve_source(pl, d, d, 1) : hh_dst1_rows(c, n, 1, d, n, d, n);
         if (rc != HH_OK && j->bad++ == 0) printf("%s %d: %s\n", j->what, n, hh_last_error());
         if (i % 128 == 127) hh_ctx_synchronize(c);
