@@ -68,7 +68,8 @@ inline size_t mma_smem(bool cols, int n, int nl) {
 // COLS: line c of a plane is column c (element j at c + j ld); otherwise row c (element j at c ld + j).
 // What is not a product counts here: at n = 100 a warp's one unit is 208 of its instructions, and with plain
 // indexing in the three phases it ran 1262, now 776 (40000 rows 49 -> 43.5 us, 8000 rows of n = 500 160 -> 139,
-// 61504 of n = 31 23 -> 17.5, 100 columns x 400 planes 46 -> 42); so the addresses of a phase advance by constants, nothing is computed per thread that the launch can pass, and the first table steps of a unit are on
+// 61504 of n = 31 23 -> 17.5, 100 columns x 400 planes 46 -> 42); so the addresses of a phase advance by
+// constants, nothing is computed per thread that the launch can pass, and the first table steps of a unit are on
 // their way before its lines are.
 template <bool COLS, int NTW, int NT>
 __global__ void __launch_bounds__(NT, 768 / NT)
@@ -288,12 +289,13 @@ __global__ void __launch_bounds__(kDenseThreads)
 //    leaves the fewest idle columns in a plane's last tile (100 columns: 42 us at 5, 46.5 at 4).
 //  * fewer lines per CTA where the launch would not give every SM sixteen warps (7688 rows of n = 31: 4.8 us at 24
 //    lines, 6.4 at 48; 2500 rows of n = 50: 3.6 us at 8, 4.5 at 16).
+constexpr int kRowsMaxNtw = 4, kColsMaxNtw = 5;
 void dense_shape(bool cols, int n, long nlines, long planes, int *ntw, int *groups) {
     const int units = out_tiles(n), nt = mma_threads(n), warps = nt / 32, full = 768 / nt;
     int       g = units >= warps ? 1 : std::min(4, warps / units), w = 0;
     auto per_sm = [&](int v) { return kMmaSmemMax / (long)(mma_smem(cols, n, 4 * v * g) + 1024); };
     auto padded = [&](int v) { return (nlines + 4L * v * g - 1) / (4L * v * g) * (4L * v * g); };
-    for (int v = cols ? 5 : 4; v >= 2; v--)
+    for (int v = cols ? kColsMaxNtw : kRowsMaxNtw; v >= 2; v--)
         if (per_sm(v) >= full && (w == 0 || (cols && padded(v) < padded(w)))) w = v;
     if (w == 0) w = per_sm(2) * 3 >= full * 2 ? 2 : 1;
     auto ctas = [&]() { return padded(w) / (4L * w * g) * planes; };
@@ -359,8 +361,11 @@ int launch_dst_dense(Ctx *c, int n, bool cols, long nlines, long planes, const d
         auto go = [&](auto launch) {
             return launch(c, n, nlines, planes, in, in_ld, in_plane, out, out_ld, out_plane, groups, tab);
         };
-        if (mma_threads(n) == 128) return cols ? go(launch_mma<true, W, 128>) : go(launch_mma<false, W, 128>);
-        return cols ? go(launch_mma<true, W, 256>) : go(launch_mma<false, W, 256>);
+        const bool    small = mma_threads(n) == 128;
+        if (cols) return small ? go(launch_mma<true, W, 128>) : go(launch_mma<true, W, 256>);
+        if constexpr (W <= kRowsMaxNtw) return small ? go(launch_mma<false, W, 128>) : go(launch_mma<false, W, 256>);
+        set_error("DST length %d: no tile shape", n);
+        return (int)HH_ERR_UNSUPPORTED;
     };
     switch (ntw) {
     case 1: return pick(std::integral_constant<int, 1>{});

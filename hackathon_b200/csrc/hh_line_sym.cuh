@@ -73,6 +73,12 @@ template <int SRC, int KS, int CW, typename MT> struct SymPCS {
     static constexpr bool value = SymUIS<SRC, KS, MT>::value && (CW == 4 || CW >= 16);
 };
 
+// Order 6 with 8-row segments scans its Pade sweeps: tables of the stage multipliers, [LOG + 1][NT] each way
+// (16-row segments take their entering value from the neighbour and have none).
+template <int SRC, int KS> struct SymTT {
+    static constexpr int value = SRC == 6 && KS < 16 ? 1 : 0;
+};
+
 // Intra-warp inclusive scan of B over the segments of each line in the warp, with the stage
 // multipliers tab[j * NT] (the thread's own map product at stage j).  FWD composes left to right.
 template <int CW, bool FWD>
@@ -166,7 +172,7 @@ __device__ __forceinline__ void sym_chunk(const double2 *__restrict__ in, double
         else return ui[k];
     };
     constexpr bool PCS = SymPCS<SRC, KS, CW, MT>::value;
-    const MT *pcs = reinterpret_cast<const MT *>(ttB + (ilog2_t<32 / CW>() + 1) * NT);
+    const MT *pcs = reinterpret_cast<const MT *>(ttB + SymTT<SRC, KS>::value * (ilog2_t<32 / CW>() + 1) * NT);
     auto PC = [&](int j) -> MT { return lds_keep(pcs + j * NT + t); };
     const MT tau_in = PCS ? MT{} : cmul(s, ui_in); // L_0 = s / P of row r0 - 1
     const MT rs = PCS ? MT{} : (KEEP_L ? s : crcp(s));
@@ -594,8 +600,8 @@ __global__ void __launch_bounds__(NT, MINB)
     MT *tabB = tabF + (LOG + 1) * NT;                   // [LOG + 1][NT]
     constexpr bool UIS = SymUIS<SRC, KS, MT>::value;
     MT *uis = tabB + (LOG + 1) * NT;               // [KS][NT] tau_k (UIS)
-    double  *ttF = reinterpret_cast<double *>(uis + (UIS ? KS * NT : 0)); // [LOG + 1][NT] (order 6)
-    double  *ttB = ttF + (LOG + 1) * NT;
+    double  *ttF = reinterpret_cast<double *>(uis + (UIS ? KS * NT : 0)); // [LOG + 1][NT] (SymTT)
+    double  *ttB = ttF + SymTT<SRC, KS>::value * (LOG + 1) * NT;
     (void)HALO;
 
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
@@ -713,7 +719,7 @@ __global__ void __launch_bounds__(NT, MINB)
         }
         c2 = sp.h2 * b6;
         if constexpr (SymPCS<SRC, KS, CW, MT>::value) {
-            double2 *pcs = reinterpret_cast<double2 *>(ttB + (LOG + 1) * NT);
+            double2 *pcs = reinterpret_cast<double2 *>(ttB + SymTT<SRC, KS>::value * (LOG + 1) * NT);
             pcs[t] = cmul(s, ui_in);
             pcs[NT + t] = crcp(s);
             pcs[2 * NT + t] = c1;
@@ -734,7 +740,7 @@ __global__ void __launch_bounds__(NT, MINB)
             sm.pl[t] = t < 9 ? sp.pl[t] : (t == 9 ? sp.linf : 0.0);
             sm.pu[t] = t < 9 ? sp.pu[t] : (t == 9 ? sp.uinf : 0.0);
         }
-        if constexpr (KS < 16) { // (16-row segments need no Pade scan)
+        if constexpr (SymTT<SRC, KS>::value) {
             __syncthreads();
             double af = 1.0, ab = 1.0;
 #pragma unroll
@@ -814,7 +820,7 @@ static int launch_sym_t(Plan *p, const double2 *in, double2 *out, int batch, con
         return 128 + (int)(sizeof(double2) * io_elems +
                            sizeof(MT) * (2 * (LOG + 1) * NT + (SymUIS<SRC, KS, MT>::value ? KS * NT : 0) +
                                          (SymPCS<SRC, KS, CW, MT>::value ? 5 * NT : 0)) +
-                           (SRC == 6 ? sizeof(double) * 2 * (LOG + 1) * NT : 0));
+                           sizeof(double) * 2 * SymTT<SRC, KS>::value * (LOG + 1) * NT);
     };
     const int shm = smem(p->rows);
     CUtensorMap in_map{};
