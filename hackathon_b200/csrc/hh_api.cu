@@ -939,6 +939,14 @@ struct WorkPool {
 static std::mutex              g_work_mu;
 static std::map<int, WorkPool> g_work;
 
+// While it lives, the thread may call what a capture on another stream forbids by default (making a pool, taking or giving back memory):
+// without it a solve that takes a workspace invalidates that capture.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 static cudaMemPool_t work_pool_of(Ctx *c) {
     if (c->work_pool) return c->work_pool;
     std::lock_guard<std::mutex> g(g_work_mu);
@@ -986,6 +994,7 @@ static void acquire_work(Plan &p, int batch, int src_order, double2 **work, long
     const size_t bytes = sizeof(double2) * (size_t)pitch * (size_t)p.ny * (size_t)(p.dim == 3 ? p.nz : 1) * (size_t)batch;
     if (bytes < 2 * c->l2_bytes || bytes > kWorkKeep) return;
     if (capturing(c)) return;
+    RelaxedCapture relaxed;
     cudaMemPool_t pool = work_pool_of(c);
     if (!pool) return;
     void *w = nullptr;
@@ -1110,6 +1119,7 @@ static int solve_passes(Plan &p, const double2 *in, double2 *out, int batch, int
     };
     int rc = passes();
     if (work) {
+        RelaxedCapture    relaxed;
         const cudaError_t e = cudaFreeAsync(work, c->stream);
         if (rc == HH_OK && e != cudaSuccess) rc = cuda_fail(e, "cudaFreeAsync", __FILE__, __LINE__);
     }

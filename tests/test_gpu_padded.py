@@ -238,3 +238,40 @@ def test_which_solves_take_the_workspace():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", _WHICH], cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "which ok" in r.stdout, r.stdout + r.stderr
+
+
+_BESIDE = """
+import sys
+import torch
+import hackathon_b200 as hh
+n, batch = 1023, 17
+a, b = torch.cuda.Stream(), torch.cuda.Stream()
+ctx = hh.Context(0, b.cuda_stream)
+plan = hh.Plan.helmholtz(ctx, 2, n, 6, 30.0)
+f = torch.view_as_complex(torch.randn((batch, n, n, 2), dtype=torch.float64, device="cuda"))
+u, w, x = torch.empty_like(f), torch.empty_like(f), torch.zeros(16, device="cuda")
+for i in range(batch):  # in place: no workspace yet
+    plan.solve_source(f[i], w[i], 1)
+ctx.synchronize()
+free0 = torch.cuda.mem_get_info()[0]
+for again in range(2):  # the first padded solve makes the pool, the second finds it
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=a, capture_error_mode=sys.argv[1]):
+        x.add_(1)
+        plan.solve_source(f, u, batch)
+        x.add_(1)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(u, w) and x[0].item() == 2 * (again + 1)
+    u.zero_()
+assert free0 - torch.cuda.mem_get_info()[0] >= batch * 1024 * n * 16
+print("beside ok")
+"""
+
+
+@pytest.mark.parametrize("mode", ["global", "thread_local"])
+def test_padded_solve_beside_a_capture_on_another_stream(mode):
+    """A solve that makes the workspace pool, or takes from it, leaves another stream's capture valid."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _BESIDE, mode], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "beside ok" in r.stdout, r.stdout + r.stderr
