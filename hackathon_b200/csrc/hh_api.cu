@@ -1297,8 +1297,9 @@ int hh::solve_source_multi(Plan *const *plans, const int *nrhs, int nplans, cons
                 ps[(size_t)i] = &padded[(size_t)i];
             }
         }
-        if (table || nplans < 2 || capturing(c)) return HH_OK;
+        if (table || nplans < 2) return HH_OK;
         const size_t need = line_solve_multi_table_bytes(ps.data(), nrhs, nplans, p0.src_order);
+        if (need == 0 || capturing(c)) return HH_OK;
         if (c->multi_tab_bytes < need) {
             HH_CUDA(cudaStreamSynchronize(c->stream));
             cudaFree(c->multi_tab);
@@ -1307,7 +1308,7 @@ int hh::solve_source_multi(Plan *const *plans, const int *nrhs, int nplans, cons
             HH_CUDA(cudaMalloc(&c->multi_tab, need));
             c->multi_tab_bytes = need;
         }
-        if (need) table = c->multi_tab;
+        table = c->multi_tab;
         return HH_OK;
     };
     return solve_passes(p0, f, u, total, p0.src_order, may_pad, before, [&](double2 *w, long) -> int {

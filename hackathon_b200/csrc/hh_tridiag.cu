@@ -761,6 +761,9 @@ static bool multi_in_arguments(int nplans, size_t chunks) { return nplans <= Sym
 static size_t multi_table_bytes(int nplans, size_t chunks) { return sizeof(SymPlanRef) * (size_t)nplans + sizeof(SymChunk) * chunks; }
 
 size_t line_solve_multi_table_bytes(Plan *const *plans, const int *nrhs, int nplans, int src_order) {
+    long total = 0; // (a chunk holds at least one right-hand side: small batches need no look at the chunks)
+    for (int i = 0; i < nplans; i++) total += nrhs[i];
+    if (multi_in_arguments(nplans, (size_t)total)) return 0;
     std::vector<SymChunk> chunks;
     if (multi_chunks(plans, nrhs, nplans, src_order, &chunks) != HH_OK || multi_in_arguments(nplans, chunks.size())) return 0;
     return multi_table_bytes(nplans, chunks.size());
