@@ -442,7 +442,8 @@ __global__ void __launch_bounds__(NT, MINB)
 // way) read 4 complex values a row and sweep through L1 and bounded the solve.  MT = double: every table is
 // real (real k), so the multipliers are, and the products lose their zero halves.
 //   y_r = f_r - L_r y_{r-1},  x_r = (1/P_r) y_r - tau_r x_{r+1},  tau_r = super_r / P_r
-// (3D 125^3, real k: 60 -> 40 us; 2D 511^2, complex k: 16.4 -> 11.8 us.)
+// (line solve of 3D 125^3, real k: 60 -> 40 us; whole solves with complex k: 2D 511^2 32.8 -> 20.4 us, 2047^2 353
+// -> 296.)
 template <typename MT> __device__ __forceinline__ MT row_coef(const double2 *__restrict__ tab, int rows, int r, double m0,
                                                               double m1, double m2) {
     if constexpr (is_real_v<MT>) {
@@ -454,7 +455,9 @@ template <typename MT> __device__ __forceinline__ MT row_coef(const double2 *__r
     }
 }
 
-template <int NT, int MINB, typename MT>
+// SMT: the L_r and tau_r of a thread's rows but the first lie in shared memory, one column per thread, as complex
+// ones of 512 threads do not fit their 128 registers.
+template <int NT, int MINB, typename MT, bool SMT>
 __global__ void __launch_bounds__(NT, MINB)
     k_line_solve_rows(const double2 *__restrict__ in, double2 *__restrict__ out, int lines, int rows, int prow,
                       long row_stride, long field, int batch, int rb, int CW, const double2 *__restrict__ Pv,
@@ -462,7 +465,9 @@ __global__ void __launch_bounds__(NT, MINB)
                       const double2 *__restrict__ supt, const double *__restrict__ mu) {
     constexpr int NW = NT / 32;
     __shared__ ScanSmem<NW> sm;
-    extern __shared__ double2 pre[]; // [kSeg][NT] prefetch of the next right-hand side
+    extern __shared__ double2 pre[]; // [kSeg][NT] prefetch of the next right-hand side, then (SMT) [kSeg - 1][NT] of
+                                     // the L_r and [kSeg - 1][NT] of the tau_r past the first
+    [[maybe_unused]] MT *Ls = reinterpret_cast<MT *>(pre + kSeg * NT) + threadIdx.x, *ts = Ls + (kSeg - 1) * NT;
     Lane L;
     L.lane = threadIdx.x & 31;
     L.w = threadIdx.x >> 5;
@@ -480,7 +485,16 @@ __global__ void __launch_bounds__(NT, MINB)
 
     // ---- factors of this thread's rows, kept for the whole chunk.  Rows past the end of a line are neutral
     // (zero data, zero reciprocal pivots), so the sweeps run without per-row conditions.
-    MT Lr[kSeg], ui[kSeg], tau[kSeg];
+    constexpr int NR = SMT ? 1 : kSeg; // of L_r and tau_r in registers
+    MT Lr[NR], ui[kSeg], tau[NR];
+    auto Lm = [&](int u) -> MT {
+        if constexpr (SMT) return u == 0 ? Lr[0] : lds_keep(Ls + (u - 1) * NT);
+        else return Lr[u];
+    };
+    auto tm = [&](int u) -> MT {
+        if constexpr (SMT) return u == 0 ? tau[0] : lds_keep(ts + (u - 1) * NT);
+        else return tau[u];
+    };
     MT Af = coef_of<MT>(make_double2(1.0, 0.0)), Ab = Af;
     {
         MT uprev = (live && r0 > 0 && r0 < rows) ? coef_of<MT>(Pv[(long)L.s * lines + q]) : MT{}; // 1/P of row r0-1
@@ -488,19 +502,25 @@ __global__ void __launch_bounds__(NT, MINB)
 #pragma unroll
         for (int u = 0; u < kSeg; u++) {
             const int r = r0 + u;
-            Lr[u] = MT{};
+            MT        l{}, tu{};
             ui[u] = MT{};
-            tau[u] = MT{};
             if (live && r < rows) {
                 const MT dia = row_coef<MT>(diagt, prow, r, m0, m1, m2);
                 if (r == 0) ui[u] = first_pivot(dia);
-                else ui[u] = factor_step(row_coef<MT>(subt, prow, r, m0, m1, m2), dia, sp, uprev, Lr[u]);
+                else ui[u] = factor_step(row_coef<MT>(subt, prow, r, m0, m1, m2), dia, sp, uprev, l);
                 sp = row_coef<MT>(supt, prow, r, m0, m1, m2);
-                tau[u] = cmul(sp, ui[u]);
+                tu = cmul(sp, ui[u]);
             }
             uprev = ui[u];
-            Af = cmul(Af, mneg(Lr[u]));
-            Ab = cmul(Ab, mneg(tau[u]));
+            Af = cmul(Af, mneg(l));
+            Ab = cmul(Ab, mneg(tu));
+            if (u < NR) {
+                Lr[u < NR ? u : 0] = l;
+                tau[u < NR ? u : 0] = tu;
+            } else {
+                Ls[(u - 1) * NT] = l;
+                ts[(u - 1) * NT] = tu;
+            }
         }
     }
     const double2 Afc = coef_full(Af), Abc = coef_full(Ab); // (the scans compose complex maps)
@@ -529,22 +549,22 @@ __global__ void __launch_bounds__(NT, MINB)
         if (b + 1 < b_end) prefetch(b + 1);
         double2 yh = zero;
 #pragma unroll
-        for (int u = 0; u < kSeg; u++) yh = zfms(v[u], Lr[u], yh);
+        for (int u = 0; u < kSeg; u++) yh = zfms(v[u], Lm(u), yh);
         double2 y = scan_forward(Afc, yh, L, sm, par);
         par ^= 1;
 #pragma unroll
         for (int u = 0; u < kSeg; u++) {
-            y = zfms(v[u], Lr[u], y);
+            y = zfms(v[u], Lm(u), y);
             v[u] = cmul(ui[u], y);
         }
         double2 xh = zero;
 #pragma unroll
-        for (int u = kSeg - 1; u >= 0; u--) xh = zfms(v[u], tau[u], xh);
+        for (int u = kSeg - 1; u >= 0; u--) xh = zfms(v[u], tm(u), xh);
         double2 x = scan_backward(Abc, xh, L, sm, par);
         par ^= 1;
 #pragma unroll
         for (int u = kSeg - 1; u >= 0; u--) {
-            x = zfms(v[u], tau[u], x);
+            x = zfms(v[u], tm(u), x);
             v[u] = x;
         }
         double2 *dst = out + (long)b * field + off0;
@@ -592,16 +612,16 @@ static int rows_chunk(long groups, int batch, int minb) {
     return rb;
 }
 
-template <int NT, int MINB, typename MT>
+template <int NT, int MINB, typename MT, bool SMT = false>
 static int launch_solve_rows(Plan *p, const double2 *in, double2 *out, int batch) {
     int CW, P;
     HH_TRY(solve_geometry(p->rows, NT, &CW, &P));
-    const int shm = (int)(sizeof(double2) * kSeg * NT);
-    HH_CUDA(cudaFuncSetAttribute(k_line_solve_rows<NT, MINB, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
+    const int shm = (int)(sizeof(double2) * kSeg * NT + (SMT ? sizeof(MT) * 2 * (kSeg - 1) * NT : 0));
+    HH_CUDA(cudaFuncSetAttribute(k_line_solve_rows<NT, MINB, MT, SMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
     const long groups = (p->lines + CW - 1) / CW;
     const int  rb = rows_chunk(groups, batch, MINB);
     dim3 grid((unsigned)groups, (unsigned)((batch + rb - 1) / rb));
-    return launch_kernel(p->ctx, k_line_solve_rows<NT, MINB, MT>, grid, NT, (size_t)shm, in, out, p->lines, p->rows, p->prow,
+    return launch_kernel(p->ctx, k_line_solve_rows<NT, MINB, MT, SMT>, grid, NT, (size_t)shm, in, out, p->lines, p->rows, p->prow,
                          p->row_stride, p->field, batch, rb, CW, p->Pv, p->subt, p->diagt, p->rowc, p->mu);
 }
 
@@ -644,16 +664,31 @@ static int launch_solve_const(Plan *p, const double2 *in, double2 *out, int batc
     return launch_solve_v<512, 1>(p, in, out, batch, src);
 }
 
-// Per-row coefficients: variant 1 takes 256 threads; variant 0 512 with real coefficients, and 256 where 512
-// would leave SMs without a line group or where complex ones would not fit 128 registers.  Lines past 2048
-// rows only fit 512.
+// Per-row coefficients: variant 1 takes 256 threads, and variant 0 whichever of the two forms is the faster:
+//  * 256 threads have less to set up and half the lines in a CTA (half as wide row pieces): real ones stand two on an
+//    SM, complex ones keep their multipliers in 201 registers;
+//  * 512 threads (complex ones with multipliers in shared memory) win where their CTAs fill half the SMs and the
+//    row pieces of 256 would be narrow (real ones of up to 256 rows, about even, take them where they fill all SMs).
+// Whole solves, 256 -> 512 threads, one right-hand side but where noted: real, 1023 lines of 127 rows 18.2 -> 21.0 us,
+// of 511 32.4 -> 32.0, of 1023 77 -> 54.6, 255 of 2047 74 -> 44; complex, 1023 of 127 18.2 -> 21.1, 511 of 255
+// 15.5 -> 17.5 (two right-hand sides 21.4 -> 20.2), 511 of 511 23.1 -> 20.3, 2047 of 2047 510 -> 294, 63 of 1023 16.4
+// -> 21.2.  Lines past 2048 rows only fit 512; complex ones of few lines then keep their multipliers in (spilled)
+// registers: 31 lines of 4095 64.9 us with shared memory, 50.8 so, 127 lines 74.1 and 76.7.
 static int launch_solve_rows_any(Plan *p, const double2 *in, double2 *out, int batch) {
     int CW, P;
     HH_TRY(solve_geometry(p->rows, 512, &CW, &P));
-    const bool small = p->rows <= 256 * kSeg && (p->variant == 1 || !p->real_rows || (p->lines + CW - 1) / CW < 148);
+    const long groups = (p->lines + CW - 1) / CW, ctas = groups * batch;
+    const bool few = p->lines <= 64;
+    bool       wide = p->rows > 256 * kSeg;
+    if (!wide && p->variant != 1) {
+        if (p->real_rows) wide = p->rows > 512 ? ctas >= 64 : p->rows > 256 ? ctas > 64 : groups >= 148;
+        else wide = p->rows > 128 && !few && ctas >= 64;
+    }
     if (p->real_rows)
-        return small ? launch_solve_rows<256, 2, double>(p, in, out, batch) : launch_solve_rows<512, 1, double>(p, in, out, batch);
-    return small ? launch_solve_rows<256, 1, double2>(p, in, out, batch) : launch_solve_rows<512, 1, double2>(p, in, out, batch);
+        return wide ? launch_solve_rows<512, 1, double>(p, in, out, batch) : launch_solve_rows<256, 2, double>(p, in, out, batch);
+    if (!wide) return launch_solve_rows<256, 1, double2>(p, in, out, batch);
+    return few && p->rows > 256 * kSeg ? launch_solve_rows<512, 1, double2>(p, in, out, batch)
+                                       : launch_solve_rows<512, 1, double2, true>(p, in, out, batch);
 }
 
 int launch_line_solve_sym(Plan *p, const double2 *in, double2 *out, int batch, int src_order);
