@@ -929,7 +929,9 @@ static int transform_inverse(Plan &p, double2 *in, double2 *out, int batch, bool
 //    at once; a solve that cannot get its part of them runs in place in the output as smaller ones do.  What the
 //    pool holds between solves goes to another allocation of the process that would fail without it
 //    (the driver releases it: a cudaMalloc of all free memory and half of what was held succeeds).
-//  * In place as well: solves under stream capture (a graph's own allocations would restrict it), the request
+//  * In place as well: 2D line solves of single lines, whose 16-byte pieces an even pitch does not help and a pitch of
+//    2^k values slows (2047^2 x 8 with 8-row segments 1055 -> 1071 us, 4095^2 x 3 2075 -> 2121);
+//  * and solves under stream capture (a graph's own allocations would restrict it), the request
 //    loop's (its budget does not know the workspace) and the host-buffer forms (bound by their copies).
 constexpr size_t kWorkKeep = 4ULL << 30; // the pool's size, and what it keeps between solves
 struct WorkPool {
@@ -993,6 +995,7 @@ static void acquire_work(Plan &p, int batch, int src_order, double2 **work, long
     const long   pitch = (p.nx + 7) / 8 * 8;
     const size_t bytes = sizeof(double2) * (size_t)pitch * (size_t)p.ny * (size_t)(p.dim == 3 ? p.nz : 1) * (size_t)batch;
     if (bytes < 2 * c->l2_bytes || bytes > kWorkKeep) return;
+    if (p.dim == 2 && line_group(&p, batch, src_order) < 2) return;
     if (capturing(c)) return;
     RelaxedCapture relaxed;
     cudaMemPool_t pool = work_pool_of(c);

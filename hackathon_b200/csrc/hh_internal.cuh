@@ -240,6 +240,7 @@ int launch_axpy(Ctx *c, double2 *u, const double2 *v, double s, long n); // u +=
 int read_device_error(Ctx *c, int *val);
 long slab_planes(const Plan &p, long planes); // 3D transform slab in planes (the plan's or the default)
 bool sym_solve_supported(const Plan *p, int src_order);
+int  line_group(const Plan *p, int batch, int src_order);
 // the fused-source solve of several plans of one shape in one pass (hh_solve_source_multi);
 // table: device memory of line_solve_multi_table_bytes, or nullptr for the context's own (where one is needed)
 int solve_source_multi(Plan *const *plans, const int *nrhs, int nplans, const double2 *f, double2 *u, void *table);

@@ -674,21 +674,30 @@ static int launch_solve_const(Plan *p, const double2 *in, double2 *out, int batc
 // 15.5 -> 17.5 (two right-hand sides 21.4 -> 20.2), 511 of 511 23.1 -> 20.3, 2047 of 2047 510 -> 294, 63 of 1023 16.4
 // -> 21.2.  Lines past 2048 rows only fit 512; complex ones of few lines then keep their multipliers in (spilled)
 // registers: 31 lines of 4095 64.9 us with shared memory, 50.8 so, 127 lines 74.1 and 76.7.
-static int launch_solve_rows_any(Plan *p, const double2 *in, double2 *out, int batch) {
+static bool rows_wide(const Plan *p, int batch) {
     int CW, P;
-    HH_TRY(solve_geometry(p->rows, 512, &CW, &P));
+    if (p->rows > 256 * kSeg || solve_geometry(p->rows, 512, &CW, &P) != HH_OK) return true; // (past 4096 rows: refused)
+    if (p->variant == 1) return false;
     const long groups = (p->lines + CW - 1) / CW, ctas = groups * batch;
-    const bool few = p->lines <= 64;
-    bool       wide = p->rows > 256 * kSeg;
-    if (!wide && p->variant != 1) {
-        if (p->real_rows) wide = p->rows > 512 ? ctas >= 64 : p->rows > 256 ? ctas > 64 : groups >= 148;
-        else wide = p->rows > 128 && !few && ctas >= 64;
-    }
+    if (p->real_rows) return p->rows > 512 ? ctas >= 64 : p->rows > 256 ? ctas > 64 : groups >= 148;
+    return p->rows > 128 && p->lines > 64 && ctas >= 64;
+}
+
+static int launch_solve_rows_any(Plan *p, const double2 *in, double2 *out, int batch) {
+    const bool wide = rows_wide(p, batch);
     if (p->real_rows)
         return wide ? launch_solve_rows<512, 1, double>(p, in, out, batch) : launch_solve_rows<256, 2, double>(p, in, out, batch);
     if (!wide) return launch_solve_rows<256, 1, double2>(p, in, out, batch);
-    return few && p->rows > 256 * kSeg ? launch_solve_rows<512, 1, double2>(p, in, out, batch)
-                                       : launch_solve_rows<512, 1, double2, true>(p, in, out, batch);
+    return p->lines <= 64 && p->rows > 256 * kSeg ? launch_solve_rows<512, 1, double2>(p, in, out, batch)
+                                                  : launch_solve_rows<512, 1, double2, true>(p, in, out, batch);
+}
+
+// The lines a CTA of the plan's line solve takes, the width of its row pieces in values
+int line_group(const Plan *p, int batch, int src_order) {
+    if (p->variant >= 2 && sym_solve_supported(p, src_order)) return 256 / sym_segments(p->rows, p->variant >= 5 ? 16 : kSeg);
+    int       CW = 1, P;
+    const int nt = p->const_rows ? (p->variant == 1 ? 256 : 512) : rows_wide(p, batch) ? 512 : 256;
+    return solve_geometry(p->rows, nt, &CW, &P) == HH_OK ? CW : 1;
 }
 
 int launch_line_solve_sym(Plan *p, const double2 *in, double2 *out, int batch, int src_order);

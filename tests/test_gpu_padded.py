@@ -202,7 +202,8 @@ import hackathon_b200 as hh
 torch.zeros(1, device="cuda")
 cases = [(3, 255, 6, 30.0, 1, 6, 1), (3, 255, 4, 30.0, 1, 2, 1), (3, 255, 6, 9 + 2j, 1, 5, 1), (3, 125, 6, 20.0, 9, 6, 1),
          (3, 125, 2, 20.0, 9, 2, 1), (3, 125, 2, 20.0, 9, 0, 0), (2, 2047, 6, 100.0, 4, 6, 1), (2, 1023, 4, 50.0, 17, 3, 1),
-         (2, 1023, 6, 50 + 5j, 17, 6, 1), (2, 701, 6, 50.0, 35, 1, 1), (2, 1023, 4, 50.0, 12, 3, 0), (2, 500, 4, 20.0, 80, 6, 0)]
+         (2, 1023, 6, 50 + 5j, 17, 6, 1), (2, 701, 6, 50.0, 35, 1, 1), (2, 1023, 4, 50.0, 12, 3, 0), (2, 500, 4, 20.0, 80, 6, 0),
+         (2, 2047, 4, 50.0, 5, 3, 0), (2, 2047, 4, 50.0, 5, 5, 1), (2, 4095, 4, 50 + 1j, 1, 5, 0)]
 for dim, n, order, k, batch, variant, padded in cases:
     ctx = hh.Context(0, 1)
     plan = hh.Plan.helmholtz(ctx, dim, n, order, k)
@@ -233,7 +234,7 @@ print("which ok")
 
 def test_which_solves_take_the_workspace():
     """What the pool holds after a solve says whether it was padded: the shapes above, the same shapes where the line
-    solve does not know the positions (3D, variant 0), below the size and with even rows; and for the batches whose
+    solve does not know the positions (3D, variant 0), below the size, with even rows and with line solves of single lines; and for the batches whose
     single fields stay in place, the padded bits against those."""
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", _WHICH], cwd=root, capture_output=True, text=True, timeout=300)
