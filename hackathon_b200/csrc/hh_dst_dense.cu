@@ -250,8 +250,12 @@ __global__ void k_make_dense(int n, double *mat) {
 }
 
 // One line per CTA against the full matrix, for the lines too long for k_dst1_mma.  The matrix is
-// symmetric: thread k walks column k, so that a warp reads neighbouring values.
-constexpr int kDenseThreads = 128;
+// symmetric: thread k walks column k, so that a warp reads neighbouring values.  Every CTA streams the whole matrix
+// through L2, and what bounds it is the latency of those loads, so the CTA is as large as can be and each thread has
+// 16 of them in flight (30 rows of n = 4000: one dot product per thread along a row, 128 threads 12.4 ms; along a column
+// 15.4, so 2.4; 30 columns 11.4, 20.6 and 2.4).
+constexpr int kDenseThreads = 1024;
+constexpr int kDenseAhead = 16;  // matrix values a thread has in flight
 constexpr int kDenseMaxN = 4096; // the longest line the transforms accept here
 template <bool STRIDED>
 __global__ void __launch_bounds__(kDenseThreads)
@@ -268,9 +272,21 @@ __global__ void __launch_bounds__(kDenseThreads)
     __syncthreads();
     const double coef = sqrt(2.0 / (n + 1));
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        double sr = 0.0, si = 0.0;
-        for (int m = 0; m < n; m++) {
-            const double s = __ldg(mat + (long)m * n + k);
+        double        sr = 0.0, si = 0.0;
+        const double *col = mat + k;
+        int           m = 0;
+        for (; m + kDenseAhead <= n; m += kDenseAhead, col += (long)kDenseAhead * n) {
+            double s[kDenseAhead];
+#pragma unroll
+            for (int i = 0; i < kDenseAhead; i++) s[i] = __ldg(col + (long)i * n);
+#pragma unroll
+            for (int i = 0; i < kDenseAhead; i++) {
+                sr = fma(s[i], x[m + i].x, sr);
+                si = fma(s[i], x[m + i].y, si);
+            }
+        }
+        for (; m < n; m++, col += n) {
+            const double s = __ldg(col);
             sr = fma(s, x[m].x, sr);
             si = fma(s, x[m].y, si);
         }
