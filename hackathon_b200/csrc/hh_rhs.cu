@@ -29,6 +29,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 namespace hh {
@@ -346,8 +347,9 @@ struct Rhs3DArgs {
 //
 // A thread marches through RUN layers of its (i, j) with the layers below, at and above in registers, the
 // one after those on its way: each field crosses L2 once instead of three times.
-template <int RUN> __global__ void __launch_bounds__(256) k_rhs3d_combine(const __grid_constant__ Rhs3DArgs A) {
-    const int i = blockIdx.x * 32 + (threadIdx.x & 31), j = blockIdx.y * 8 + (threadIdx.x >> 5);
+// A block is 2^LW points wide in x, 256 / 2^LW in y.
+template <int RUN, int LW> __global__ void __launch_bounds__(256) k_rhs3d_combine(const __grid_constant__ Rhs3DArgs A) {
+    const int i = (blockIdx.x << LW) + (threadIdx.x & ((1 << LW) - 1)), j = (blockIdx.y << (8 - LW)) + (threadIdx.x >> LW);
     pdl_wait();
     pdl_next();
     if (i >= A.nx || j >= A.ny) return;
@@ -683,13 +685,21 @@ int assemble_rhs3d(Plan *p, const hh_rhs3d_data *d, double2 *rhs) {
     // small problem does not march through 16 layers on a part of the chip.  Assembly and solve against 16: 31^3
     // 47.0 -> 43.0 us, 48^3 54.2 -> 43.5, 63^3 65.5 -> 53.8.
     // As a kernel argument the run cost 2.5 % at 125^3; 32 layers in one wave were slower (127^3 238 -> 253 us).
-    const long bx = (nx + 31) / 32, by = (ny + 7) / 8;
-    auto       go = [&](auto kernel, int run) {
-        return launch_kernel(c, kernel, dim3((unsigned)bx, (unsigned)by, (unsigned)((nz + run - 1) / run)), 256, 0, A);
+    // Blocks 32 points wide, or 16 or 8 where nx is no more, whose lanes would idle: 8 x 300 x 300 at order 4 19.4 -> 8.2
+    // us, 5 x 200 x 300 13.6 -> 6.3.
+    auto width = [&](auto lw_c) {
+        constexpr int LW = decltype(lw_c)::value;
+        const long    bx = (nx + (1 << LW) - 1) >> LW, by = (ny + (256 >> LW) - 1) / (256 >> LW);
+        auto          go = [&](auto kernel, int run) {
+            return launch_kernel(c, kernel, dim3((unsigned)bx, (unsigned)by, (unsigned)((nz + run - 1) / run)), 256, 0, A);
+        };
+        if (bx * by * ((nz + 3) / 4) <= 2 * 148) return go(k_rhs3d_combine<4, LW>, 4);
+        if (bx * by * ((nz + 7) / 8) <= 2 * 148) return go(k_rhs3d_combine<8, LW>, 8);
+        return go(k_rhs3d_combine<16, LW>, 16);
     };
-    if (bx * by * ((nz + 3) / 4) <= 2 * 148) return go(k_rhs3d_combine<4>, 4);
-    if (bx * by * ((nz + 7) / 8) <= 2 * 148) return go(k_rhs3d_combine<8>, 8);
-    return go(k_rhs3d_combine<16>, 16);
+    if (nx <= 8) return width(std::integral_constant<int, 3>{});
+    if (nx <= 16) return width(std::integral_constant<int, 4>{});
+    return width(std::integral_constant<int, 5>{});
 }
 
 } // namespace hh
