@@ -920,10 +920,10 @@ static int transform_inverse(Plan &p, double2 *in, double2 *out, int batch, bool
 // ---- padded workspace.  Where nx is odd (n = 2^k - 1, the common case) every other row of a field starts in the
 // middle of a 32-byte sector, so the 32- to 128-byte row pieces that the columns transform and the line
 // solve move end in partial sectors and straddle 128-byte lines.  A large solve therefore keeps its transformed
-// field in a workspace with rows of a multiple of 8 values: 3D 255^3 x 4, columns transform 526 -> 426 us, whole solve
-// 2.18 -> 1.99 ms; 2D 2047^2 x 16 1.63 -> 1.56 ms, 1023^2 x 64 1.29 -> 1.26 ms.  Fields that stay in L2 from pass to
-// pass gain nothing (1023^2 x 8: 193 us either way), so the line is at twice the L2.  The arithmetic, and so every
-// bit, is the same.
+// field in a workspace with rows of a multiple of 8 values.  Whole solves in place and padded in turn, under the power
+// cap: 3D 255^3 x 4 order 4 2153 -> 2073 us (its columns transform alone, at full clock, 526 -> 426), 2D 1023^2 x 40
+// 821 -> 783, 2047^2 x 8 812 -> 770, at order 6 845 -> 812.  Fields that stay in L2 from pass to pass gain nothing
+// (1023^2 x 8: 193 us either way), so the line is at twice the L2.  The arithmetic, and so every bit, is the same.
 //  * The workspace is allocated and freed in stream order from one pool per device, shared by the contexts on it
 //    and destroyed with the last of them, which never holds more than kWorkKeep bytes, however many streams solve
 //    at once; a solve that cannot get its part of them runs in place in the output as smaller ones do.  What the
@@ -941,8 +941,8 @@ struct WorkPool {
 static std::mutex              g_work_mu;
 static std::map<int, WorkPool> g_work;
 
-// While it lives, the thread may call what a capture on another stream forbids by default (making a pool, taking or giving back memory):
-// without it a solve that takes a workspace invalidates that capture.
+// While it lives, the thread may call what a capture on another stream forbids by default (making a pool, taking or
+// giving back memory): without it a solve that takes a workspace invalidates that capture.
 struct RelaxedCapture {
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }

@@ -20,9 +20,11 @@
 //     (T^-1 v)_i = (v_i - r (F_{i-1} + B_{i+1})) / sqrt(d^2 - 4),  F_i = v_i - r F_{i-1},  B_i = v_i - r B_{i+1},
 // r = (d - sqrt(d^2 - 4)) / 2.  F and B forget their start by r per point (0.101 at d = 10, 0.268 at d = 4), so a
 // thread forms them for its 8 points from W points outside (r^W < 1.3e-17), independently of every other.
-// Arithmetic follows the reference's expression order (complex throughout: where the reference's
-// 3D rhs.c:149 keeps its partial sums in real doubles, here they stay complex; the two agree for
-// real data, which is what the reference's own problems have).
+// So the derivatives are the reference's to rounding, not its recurrence step by step, and what one point contributes
+// beyond its W neighbours, under 1.3e-17 of its value, is left out.  The combination has the reference's terms in
+// their order, with reciprocals of the spacings formed once in place of divisions, complex throughout (where
+// the reference's 3D rhs.c:149 keeps its partial sums in real doubles; the two agree for real data, which is what
+// the reference's own problems have).
 #include "hh_internal.cuh"
 
 #include <math.h>

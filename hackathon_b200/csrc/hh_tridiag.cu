@@ -579,7 +579,7 @@ struct SolveVariant {
     int nt, minb;
 };
 static const SolveVariant kVariants[] = {{512, 1}, {256, 2}};
-constexpr int kNumVariants = 2; // plus variants 2..5: k_line_solve_sym where the plan allows it
+constexpr int kNumVariants = 2; // plus variants 2..6: k_line_solve_sym where the plan allows it
 
 // segments per line: a power of two >= NT/32 (so at most 32 lines share a warp)
 static int solve_geometry(int rows, int nt, int *CW, int *P) {

@@ -243,8 +243,9 @@ int hh_residual(hh_plan *plan, const double *sol_dev, const double *rhs_dev, dou
  * evaluates through its user callbacks comes as sampled arrays, x fastest, complex unless noted;
  * a NULL boundary array means identically zero.  rhs_dev receives nx*ny (nx*ny*nz) values, the
  * input of hh_solve on the same plan.  The plan's stencil rows give the Dirichlet corrections.
- * Arithmetic follows the reference's expression order (complex throughout; the reference's 3D
- * rhs.c:149 keeps its partial sums in real doubles, which agrees for real data). */
+ * The terms are the reference's in its order, complex throughout (the reference's 3D rhs.c:149 keeps
+ * its partial sums in real doubles, which agrees for real data); spacings enter as reciprocals, and
+ * the Pade derivatives agree with its recurrences to rounding. */
 typedef struct {
     int           order;        /* 2, 4 or 6                                                    */
     double        hx, hy;       /* grid spacings                                                */
